@@ -639,7 +639,9 @@ void launch_pass(const State& s, const Plan& plan, const Pass& p) {
     return;
   }
   if (s.precision == KETGPU_C128) {
-    launch_fused_simt<double>(s, p, static_cast<const char*>(plan.d_mat64) + plan.off64[p.mat_index]);
+    const void* mat = static_cast<const char*>(plan.d_mat64) + plan.off64[p.mat_index];
+    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, mat);
+    else launch_fused_simt<double>(s, p, mat);
   } else if (p.tensor) {
     launch_fused_tc(s, p, static_cast<const char*>(plan.d_tc) + plan.offtc[p.mat_index],
                     p.norm_out ? plan.d_norm + 2 : nullptr);

@@ -179,6 +179,10 @@ void upload_plan_matrices(Plan& plan, int device);
 // norm_partials: null, or kNormBlocks doubles that receive the per-CTA sums
 // of |out|^2 (zero beyond the grid).
 void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials = nullptr);
+// complex128 dense blocks (fused_f64.cu): mat_t = the FP64 matrix,
+// transposed ([c][r], re/im).
+bool f64_supported(int n, int k);
+void launch_fused_f64(const State& s, const Pass& p, const void* mat_t);
 // Host only: the producer and epilogue forms a tensor-core launch of pass p
 // on an n-qubit state takes (tma_dims = tensor-map dimensions, 0 for the
 // cp.async producers; direct = register-to-HBM stores), given the tensor-map

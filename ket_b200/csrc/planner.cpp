@@ -585,6 +585,13 @@ void emit_fused(Plan& plan, int n, const ketgpu_op* ops, const Block& b, const P
       if (std::find(qs.begin(), qs.end(), q) == qs.end()) qs.push_back(q);
     std::sort(qs.begin(), qs.end());
   }
+  // complex128: a 2-qubit block likewise runs as a 3-qubit one (the FP64
+  // matrix instructions work on 16 rows of the block's real embedding).
+  if (opt.precision == KETGPU_C128 && qs.size() == 2 && f64_supported(n, 3)) {
+    for (int q = n - 1; q >= 0 && qs.size() < 3; --q)
+      if (std::find(qs.begin(), qs.end(), q) == qs.end()) qs.push_back(q);
+    std::sort(qs.begin(), qs.end());
+  }
   const int k = (int)qs.size();
   Pass p;
   p.first_op = b.gates.front();

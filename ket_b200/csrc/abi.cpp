@@ -52,6 +52,47 @@ DeviceGuard::~DeviceGuard() {
   if (cudaGetDevice(&cur) == cudaSuccess && cur != prev && prev >= 0) cudaSetDevice(prev);
 }
 
+namespace {
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[64] = {nullptr};
+
+// The scratch pool of a device (which must be current), made on first use.
+cudaMemPool_t scratch_pool(int device) {
+  if (device < 0 || device >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pools[device]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    KB_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = kPoolKeep;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) cudaMemPoolDestroy(pool);
+    KB_CUDA(e);
+    g_pools[device] = pool;
+  }
+  return g_pools[device];
+}
+}  // namespace
+
+StreamScratch::StreamScratch(size_t bytes, int device, cudaStream_t stream) : st(stream) {
+  cudaMemPool_t pool = scratch_pool(device);
+  if (pool) KB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream));
+  else KB_CUDA(cudaMallocAsync(&p, bytes ? bytes : 8, stream));
+}
+
+StreamScratch::~StreamScratch() {
+  if (p) cudaFreeAsync(p, st);
+}
+
+void release_pools() {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  for (cudaMemPool_t pool : g_pools)
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
 Plan::~Plan() {
   if (device >= 0) {
     int prev = -1;
@@ -473,8 +514,9 @@ State* create_state(int n, int precision) {
   const size_t bytes = (size_t)st->dim() * st->amp_bytes();
   size_t free_b = 0, total_b = 0;
   KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (bytes > free_b) {  // give back ketgpu_run's kept state first
+  if (bytes > free_b) {  // give back ketgpu_run's kept state and the scratch pools first
     release_run_state();
+    release_pools();
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   }
   if (bytes > free_b)
@@ -714,7 +756,10 @@ KB_API int ketgpu_run_last_profile(double* out6) {
 }
 
 KB_API int ketgpu_release_cache(void) {
-  return guard([&] { release_run_state(); });
+  return guard([&] {
+    release_run_state();
+    release_pools();
+  });
 }
 
 KB_API int ketgpu_norm(const ketgpu_state* s, double* out) {

@@ -38,6 +38,21 @@ struct DeviceGuard {
   ~DeviceGuard();
 };
 
+// Device scratch of one call, stream-ordered, from the library's own pool on
+// the device.  The pool keeps up to kPoolKeep bytes between calls (taking them
+// back from the driver at each synchronisation cost 0.1 ms and more a call);
+// release_pools gives them back.
+constexpr uint64_t kPoolKeep = uint64_t{64} << 20;
+struct StreamScratch {
+  void* p = nullptr;
+  cudaStream_t st;
+  StreamScratch(size_t bytes, int device, cudaStream_t stream);
+  ~StreamScratch();
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+};
+void release_pools();
+
 // ---- state -----------------------------------------------------------------
 struct State {
   int n = 0;
@@ -173,7 +188,7 @@ void pass_features(int n, int precision, const std::vector<const ketgpu_op*>& ga
 bool learned_model_attached();
 void learned_predict(const std::vector<float>& rows, std::vector<float>& us);
 
-// ---- kernel launchers (gates.cu / fused_tc.cu / reduce.cu) -----------------
+// ---- kernel launchers (gates.cu / fused_*.cu / reduce.cu) ------------------
 void launch_pass(const State& s, const Plan& plan, const Pass& p);
 void upload_plan_matrices(Plan& plan, int device);
 // norm_partials: null, or kNormBlocks doubles that receive the per-CTA sums
@@ -219,6 +234,7 @@ void rescale_state(const State& s, const double* target, const double* current);
 double reduce_norm(const State& s);
 cplx reduce_inner(const State& a, const State& b);
 void compare_states(const State& a, const State& b, double out[5]);
+// Expectations of Pauli strings (expval.cu); phase[t] = number of Y's mod 4.
 void expval_terms(const State& s, const std::vector<uint64_t>& flip,
                   const std::vector<uint64_t>& sign, const std::vector<int>& phase,
                   double* out);

@@ -1,14 +1,10 @@
-// reduce.cu -- FP64 reductions over the state: norm, inner product, batched
-// Pauli-string expectations, and the fixed-tree Born-rule sampler.
+// reduce.cu -- FP64 reductions over the state: norm, inner product and the
+// fixed-tree Born-rule sampler (Pauli expectations are in expval.cu).
 //
 // Replaces
-//   ket::expval(State, pauli)        src/observable.cpp:18-83
-//   ket::expval(State, PauliSum)     src/observable.cpp:85-91
 //   ket::measure(State, rng)         src/measurement.cpp:12-21
-// The reference runs one serial pass per Pauli term and one O(2^n) scan per
-// shot.  Here every term of a sum shares one launch (each term re-reads the
-// state through XOR-permuted but coalesced loads), and sampling builds one
-// FP64 CDF tree per state and answers all shots with a short descent each.
+// The reference runs one O(2^n) scan per shot.  Sampling here builds one FP64
+// CDF tree per state and answers all shots with a short descent each.
 // All sums are deterministic: fixed per-thread order, fixed warp/block trees,
 // block partials reduced in index order by a second kernel.
 #include <cuda_runtime.h>
@@ -140,66 +136,6 @@ __global__ void finish_partials(const double* __restrict__ part, int count, int 
     for (int i = threadIdx.x; i < count; i += blockDim.x) acc += part[(size_t)i * width + w];
     const double r = block_sum(acc, sh);
     if (threadIdx.x == 0) out[w] = r;
-  }
-}
-
-// Batched Pauli terms.  Term t: flip f, sign mask s, phase i^q.  Contribution
-// of x: Re(i^q (-1)^popcount(x&s) psi[x] conj(psi[x^f])).  blockIdx.y picks
-// a batch of up to kTermBatch terms.
-constexpr int kTermBatch = 8;
-constexpr int kXPerThread = 4;
-
-struct TermArgs {
-  uint64_t flip[kTermBatch];
-  uint64_t sign[kTermBatch];
-  int q[kTermBatch];
-  int count;
-};
-
-template <typename T>
-__global__ void __launch_bounds__(kRThreads)
-    expval_partial(const T* __restrict__ s, uint64_t dim, const uint64_t* __restrict__ flips,
-                   const uint64_t* __restrict__ signs, const int* __restrict__ qs, int n_terms,
-                   double* __restrict__ part /* [term][block] */) {
-  __shared__ double sh[32];
-  const int t0 = blockIdx.y * kTermBatch;
-  const uint64_t chunk = (uint64_t)kRThreads * kXPerThread;
-  const uint64_t nblk = (dim + chunk - 1) / chunk;
-  double acc[kTermBatch];
-#pragma unroll
-  for (int t = 0; t < kTermBatch; ++t) acc[t] = 0;
-  for (uint64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    T a[kXPerThread];
-    uint64_t xs[kXPerThread];
-#pragma unroll
-    for (int e = 0; e < kXPerThread; ++e) {
-      xs[e] = blk * chunk + threadIdx.x + (uint64_t)e * kRThreads;
-      if (xs[e] < dim) a[e] = s[xs[e]];
-    }
-#pragma unroll
-    for (int t = 0; t < kTermBatch; ++t) {
-      if (t0 + t >= n_terms) break;
-      const uint64_t f = flips[t0 + t], sg = signs[t0 + t];
-      const int q = qs[t0 + t];
-#pragma unroll
-      for (int e = 0; e < kXPerThread; ++e) {
-        if (xs[e] >= dim) continue;
-        const T b = s[xs[e] ^ f];
-        const double ar = AmpT<T>::re(a[e]), ai = AmpT<T>::im(a[e]);
-        const double br = AmpT<T>::re(b), bi = AmpT<T>::im(b);
-        const double zr = ar * br + ai * bi;
-        const double zi = ai * br - ar * bi;
-        double v = (q == 0) ? zr : (q == 1) ? -zi : (q == 2) ? -zr : zi;
-        if (__popcll(xs[e] & sg) & 1) v = -v;
-        acc[t] += v;
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kTermBatch; ++t) {
-    if (t0 + t >= n_terms) break;
-    const double r = block_sum(acc[t], sh);
-    if (threadIdx.x == 0) part[(size_t)(t0 + t) * gridDim.x + blockIdx.x] = r;
   }
 }
 
@@ -344,20 +280,6 @@ int grid_for(uint64_t work, int per_block) {
   return (int)g;
 }
 
-// Scratch owned by the call (stream-ordered).
-struct Scratch {
-  void* p = nullptr;
-  cudaStream_t st;
-  Scratch(size_t bytes, cudaStream_t s) : st(s) { KB_CUDA(cudaMallocAsync(&p, bytes ? bytes : 8, s)); }
-  ~Scratch() {
-    if (p) cudaFreeAsync(p, st);
-  }
-  template <typename T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
 template <typename T>
 __global__ void rescale_kernel(T* __restrict__ s, uint64_t dim, const double* __restrict__ target,
                                const double* __restrict__ current) {
@@ -431,8 +353,8 @@ void rescale_state(const State& st, const double* target, const double* current)
 
 double reduce_norm(const State& st) {
   const int blocks = grid_for(st.dim(), kRThreads * 8);
-  Scratch part(sizeof(double) * (blocks + 1), st.stream);
-  double* d = part.as<double>();
+  StreamScratch part(sizeof(double) * (blocks + 1), st.device, st.stream);
+  double* d = static_cast<double*>(part.p);
   if (st.precision == KETGPU_C64)
     norm_partial<float2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), st.dim(), d);
   else
@@ -448,8 +370,8 @@ double reduce_norm(const State& st) {
 
 cplx reduce_inner(const State& a, const State& b) {
   const int blocks = grid_for(a.dim(), kRThreads * 8);
-  Scratch part(sizeof(double) * 2 * (blocks + 1), a.stream);
-  double* d = part.as<double>();
+  StreamScratch part(sizeof(double) * 2 * (blocks + 1), a.device, a.stream);
+  double* d = static_cast<double*>(part.p);
   if (b.stream != a.stream) KB_CUDA(cudaStreamSynchronize(b.stream));
   if (a.precision == KETGPU_C64)
     inner_partial<float2><<<blocks, kRThreads, 0, a.stream>>>(static_cast<const float2*>(a.amps),
@@ -468,8 +390,8 @@ cplx reduce_inner(const State& a, const State& b) {
 
 void compare_states(const State& a, const State& b, double out[5]) {
   const int blocks = grid_for(a.dim(), kRThreads * 8);
-  Scratch part(sizeof(double) * 5 * blocks, a.stream);
-  double* d = part.as<double>();
+  StreamScratch part(sizeof(double) * 5 * blocks, a.device, a.stream);
+  double* d = static_cast<double*>(part.p);
   KB_CUDA(cudaStreamSynchronize(b.stream));
   const bool a64 = a.precision == KETGPU_C64, b64 = b.precision == KETGPU_C64;
   if (a64 && b64)
@@ -496,43 +418,6 @@ void compare_states(const State& a, const State& b, double out[5]) {
   }
 }
 
-void expval_terms(const State& st, const std::vector<uint64_t>& flip, const std::vector<uint64_t>& sign,
-                  const std::vector<int>& phase, double* out) {
-  const int T = (int)flip.size();
-  if (T == 0) return;
-  const int bx = grid_for(st.dim(), kRThreads * kXPerThread);
-  const int by = (T + kTermBatch - 1) / kTermBatch;
-  const size_t meta = sizeof(uint64_t) * 2 * T + sizeof(int) * T;
-  const size_t parts = sizeof(double) * ((size_t)T * bx + T);
-  Scratch sc(meta + parts + 64, st.stream);
-  char* base = sc.as<char>();
-  uint64_t* d_flip = reinterpret_cast<uint64_t*>(base);
-  uint64_t* d_sign = d_flip + T;
-  int* d_q = reinterpret_cast<int*>(d_sign + T);
-  double* d_part = reinterpret_cast<double*>(base + ((meta + 15) / 16) * 16);
-  std::vector<char> host(meta);
-  std::memcpy(host.data(), flip.data(), sizeof(uint64_t) * T);
-  std::memcpy(host.data() + sizeof(uint64_t) * T, sign.data(), sizeof(uint64_t) * T);
-  std::memcpy(host.data() + sizeof(uint64_t) * 2 * T, phase.data(), sizeof(int) * T);
-  KB_CUDA(cudaMemcpyAsync(base, host.data(), meta, cudaMemcpyHostToDevice, st.stream));
-  dim3 grid(bx, by);
-  if (st.precision == KETGPU_C64)
-    expval_partial<float2><<<grid, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), st.dim(),
-                                                              d_flip, d_sign, d_q, T, d_part);
-  else
-    expval_partial<double2><<<grid, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), st.dim(),
-                                                               d_flip, d_sign, d_q, T, d_part);
-  count_launch();
-  double* d_out = d_part + (size_t)T * bx;
-  for (int t = 0; t < T; ++t) {
-    finish_partials<<<1, kRThreads, 0, st.stream>>>(d_part + (size_t)t * bx, bx, 1, d_out + t);
-    count_launch();
-  }
-  KB_CUDA(cudaGetLastError());
-  KB_CUDA(cudaMemcpyAsync(out, d_out, sizeof(double) * T, cudaMemcpyDeviceToHost, st.stream));
-  KB_CUDA(cudaStreamSynchronize(st.stream));
-}
-
 std::atomic<uint64_t> g_tree_builds{0};
 
 uint64_t sample_tree_builds() { return g_tree_builds.load(); }
@@ -555,9 +440,9 @@ void sample_tree(const State& st, const double* u, uint64_t count, uint64_t* out
     st.tree_doubles = total;
   }
   const size_t ubytes = sizeof(double) * count, obytes = sizeof(uint64_t) * count;
-  Scratch sc(ubytes + obytes + 64, st.stream);
+  StreamScratch sc(ubytes + obytes + 64, st.device, st.stream);
   double* buf = st.tree;
-  double* d_u = sc.as<double>();
+  double* d_u = static_cast<double*>(sc.p);
   uint64_t* d_out = reinterpret_cast<uint64_t*>(d_u + count);
   KB_CUDA(cudaMemcpyAsync(d_u, u, ubytes, cudaMemcpyHostToDevice, st.stream));
   const bool build = total && st.tree_version != st.version;

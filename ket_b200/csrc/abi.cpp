@@ -474,7 +474,8 @@ void execute(const Plan& plan, State& s) {
   need(plan.n == s.n, "plan and state have different qubit counts");
   need(plan.precision == s.precision, "plan and state have different precisions");
   upload_plan_matrices(const_cast<Plan&>(plan), s.device);
-  for (const Pass& p : plan.passes) launch_pass(s, plan, p);
+  PassRunner run(s, plan);
+  for (const Pass& p : plan.passes) run.launch(p);
 }
 
 void check_tc_flag() {
@@ -590,6 +591,7 @@ KB_API int ketgpu_state_info(const ketgpu_state* s, int32_t* n, int32_t* precisi
 KB_API void* ketgpu_state_device_ptr(const ketgpu_state* s) {
   if (!s) return nullptr;
   as_state(s)->touch();
+  as_state(s)->exposed = true;
   return as_state(s)->amps;
 }
 
@@ -880,9 +882,10 @@ KB_API int ketgpu_plan_execute_timed(const ketgpu_plan* p, ketgpu_state* s, floa
     const size_t np = plan.passes.size();
     std::vector<cudaEvent_t> ev(np + 1);
     for (auto& e : ev) KB_CUDA(cudaEventCreate(&e));
+    PassRunner run(st, plan);
     KB_CUDA(cudaEventRecord(ev[0], st.stream));
     for (size_t i = 0; i < np; ++i) {
-      launch_pass(st, plan, plan.passes[i]);
+      run.launch(plan.passes[i]);
       KB_CUDA(cudaEventRecord(ev[i + 1], st.stream));
     }
     KB_CUDA(cudaEventSynchronize(ev[np]));

@@ -207,11 +207,11 @@ __global__ void __launch_bounds__(kDiagThreads)
 
 }  // namespace
 
-void launch_diag(const State& s, const Pass& p, const void* data) {
+void launch_diag(const State& s, const Pass& p, const void* data, uint64_t active) {
   (void)p;
   const int n = s.n;
   const int L = std::min(n, kDiagLowBits);
-  const uint64_t n_chunks = uint64_t{1} << (n - L);
+  const uint64_t n_chunks = uint64_t{1} << (std::max(active_bits(active), L) - L);
   const unsigned grid = (unsigned)std::min<uint64_t>(n_chunks, 148ull * 4);
   const size_t table = (size_t{1} << L) * s.amp_bytes();
   const double* prm = reinterpret_cast<const double*>(static_cast<const unsigned char*>(data) + table);

@@ -279,12 +279,14 @@ void launch_k(const State& st, const F64Geom& g, const double2* mat_t) {
 // A k-qubit complex128 block needs whole 8-group column blocks.
 bool f64_supported(int n, int k) { return k >= 3 && k <= 6 && n >= k + 3; }
 
-void launch_fused_f64(const State& st, const Pass& p, const void* mat_t) {
+void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_t active) {
   F64Geom g{};
   g.k = p.k;
   // 1024-amplitude tiles, fewer amplitudes where that leaves teams without a
   // tile: 2^11 tiles or more, down to one column block
-  g.tb = std::clamp(st.n - 11, p.k + 3, kMaxTileBits);
+  uint64_t span = active;  // index bits of the amplitudes the launch covers
+  for (int b = 0; b < p.k; ++b) span |= uint64_t{1} << p.qubits[b];
+  g.tb = std::clamp(__builtin_popcountll(span) - 11, p.k + 3, kMaxTileBits);
   uint64_t tmask = 0;
   for (int b = 0; b < p.k; ++b) {
     tmask |= uint64_t{1} << p.qubits[b];
@@ -297,16 +299,18 @@ void launch_fused_f64(const State& st, const Pass& p, const void* mat_t) {
       tile_mask |= uint64_t{1} << q;
       --extra;
     }
-  for (int q = 0; q < st.n; ++q)
+  span |= tile_mask;
+  for (int q = 0; q < st.n; ++q) {
     if ((tile_mask >> q) & 1) {
       g.tile_pos[j] = q;
       g.is_target[j] = (int)((tmask >> q) & 1);
       if (!g.is_target[j]) g.gpos[gb++] = q;
       ++j;
-      g.ins[g.nins++] = (unsigned char)q;
     }
+    if (((tile_mask | ~span) >> q) & 1) g.ins[g.nins++] = (unsigned char)q;
+  }
   g.q0_group = g.gpos[0] == 0;
-  g.n_tiles = st.dim() >> g.tb;
+  g.n_tiles = uint64_t{1} << (__builtin_popcountll(span) - g.tb);
   const double2* m = static_cast<const double2*>(mat_t);
   switch (p.k) {
     case 3: launch_k<3>(st, g, m); break;

@@ -97,8 +97,8 @@ struct TcGeom {
   int tile_pos[16];   // tile qubits, ascending
   int is_target[16];
   int m_low;          // tile qubits 0..m_low-1 form the low run
-  int nh;             // tile qubits above the low run
-  int hpos[16];
+  int nh;             // positions above the low run that are zero in a tile
+  unsigned char hpos[40];  // base, ascending: tile qubits and inactive ones
   int direct;         // the epilogue stores from registers (see launch_fused_tc)
   // Tensor-copy producer (tma_dims > 0, see launch_tc): dimension i of the
   // tensor map starts at qubit tma_start[i]; a tile's coordinate in it is
@@ -932,7 +932,7 @@ bool tma_wanted(const TcGeom& g, const Pass& p, int tb) {
 // the tile index decomposition, each combination's offset and the
 // cp.async-form direct-store rule.
 template <int KQ>
-void tile_geometry(int n, const Pass& p, TcGeom& g) {
+void tile_geometry(int n, const Pass& p, uint64_t active, TcGeom& g) {
   using Cfg = TcCfg<KQ>;
   g = TcGeom{};
   uint64_t tmask = 0;
@@ -973,8 +973,11 @@ void tile_geometry(int n, const Pass& p, TcGeom& g) {
     g.cdep[c] = d;
   }
   g.nh = 0;
-  for (int i = g.m_low; i < Cfg::TB; ++i) g.hpos[g.nh++] = g.tile_pos[i];
-  g.n_tiles = (uint64_t{1} << n) >> Cfg::TB;
+  // tile bases range over the active qubits outside the tile
+  const uint64_t span = (active & ((uint64_t{1} << n) - 1)) | tiles_mask;
+  for (int q = g.m_low; q < n; ++q)
+    if (((tiles_mask | ~span) >> q) & 1) g.hpos[g.nh++] = (unsigned char)q;
+  g.n_tiles = uint64_t{1} << (__builtin_popcountll(span) - Cfg::TB);
   constexpr int CPT = Cfg::TILE / 2 / 128;
   static_assert(CPT <= 32, "chunk tables");
   for (int i = 0; i < CPT; ++i) {
@@ -1042,10 +1045,10 @@ int encode_half_tiles(const State* st, const Pass& p, TcGeom& g, CUtensorMap* ma
 }
 
 template <int KQ>
-void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials) {
+void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, uint64_t active) {
   using Cfg = TcCfg<KQ>;
   TcGeom g;
-  tile_geometry<KQ>(st.n, p, g);
+  tile_geometry<KQ>(st.n, p, active, g);
   g.norm_out = norm_partials;
   if (norm_partials)  // entries past the grid stay zero for the in-order sum
     KB_CUDA(cudaMemsetAsync(norm_partials, 0, sizeof(double) * kNormBlocks, st.stream));
@@ -1179,19 +1182,19 @@ void build_tc_image(const std::vector<cplx>& mat, int k, std::vector<uint32_t>& 
   std::memcpy(lo + img, &sbw, 4);
 }
 
-void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials) {
-  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials);
-  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials);
-  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials);
+void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active) {
+  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials, active);
+  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials, active);
+  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials, active);
   else fail(KETGPU_ERR_LOGIC, "tensor-core block supports k = 4, 5 or 6");
 }
 
 void tc_form(int n, const Pass& p, int* tma_dims, int* direct) {
   if (p.k < 4 || p.k > 6) fail(KETGPU_ERR_LOGIC, "tensor-core block supports k = 4, 5 or 6");
   TcGeom g;
-  if (p.k == 5) tile_geometry<5>(n, p, g);
-  else if (p.k == 6) tile_geometry<6>(n, p, g);
-  else tile_geometry<4>(n, p, g);
+  if (p.k == 5) tile_geometry<5>(n, p, ~uint64_t{0}, g);
+  else if (p.k == 6) tile_geometry<6>(n, p, ~uint64_t{0}, g);
+  else tile_geometry<4>(n, p, ~uint64_t{0}, g);
   int start[16], tq[16];
   const int nd = p.k == 6 ? encode_half_tiles(nullptr, p, g, nullptr)
                  : tma_wanted(g, p, p.k + kGroupBits) ? tile_runs(g, p.k + kGroupBits, start, tq)

@@ -14,6 +14,7 @@
 // positions, so only the amplitudes a gate changes are read and written.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "internal.h"
@@ -341,12 +342,12 @@ int sm_count(int device) {
 }
 
 template <typename R>
-void launch_pair(const State& st, const Pass& p) {
+void launch_pair(const State& st, const Pass& p, uint64_t active) {
   using T = typename C2<R>::T;
   PairGeom g{};
   g.nfixed = p.nfixed;
   for (int j = 0; j < 3; ++j) g.fixed[j] = p.fixed[j];
-  g.count = st.dim() >> p.nfixed;
+  g.count = (uint64_t{1} << active_bits(active)) >> p.nfixed;
   g.p0 = p.p0;
   g.p1 = p.p1;
   T* s = static_cast<T*>(st.amps);
@@ -407,7 +408,7 @@ void launch_pair(const State& st, const Pass& p) {
 }
 
 template <typename R>
-void launch_fused_simt(const State& st, const Pass& p, const void* mat_t) {
+void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, uint64_t active) {
   using T = typename C2<R>::T;
   FusedGeom g{};
   g.n = st.n;
@@ -430,7 +431,9 @@ void launch_fused_simt(const State& st, const Pass& p, const void* mat_t) {
       g.is_target[j] = (int)((tmask >> q) & 1);
       ++j;
     }
-  g.n_tiles = st.dim() >> g.tb;
+  // the tiles whose base lies below the highest active qubit
+  const uint64_t below = (uint64_t{1} << active_bits(active)) - 1;
+  g.n_tiles = uint64_t{1} << __builtin_popcountll(below & ~tiles_mask);
   const int dim = 1 << p.k;
   const size_t smem = sizeof(T) * ((size_t)dim * dim + ((size_t)1 << g.tb));
   static bool attr_set[2] = {false, false};
@@ -551,9 +554,9 @@ void run_device_data(const std::vector<Pass>& gates, int precision, std::vector<
   else append_run_gates<double>(gates, out);
 }
 
-void launch_run(const State& st, const Pass& p, const void* data) {
+void launch_run(const State& st, const Pass& p, const void* data, uint64_t active) {
   const int bits = st.n < kRunBits ? st.n : kRunBits;
-  const uint64_t n_chunks = st.dim() >> bits;
+  const uint64_t n_chunks = uint64_t{1} << (std::max(active_bits(active), bits) - bits);
   static int sms[64] = {0};
   if (!sms[st.device]) sms[st.device] = sm_count(st.device);
   uint64_t grid = (uint64_t)sms[st.device] * 8;
@@ -593,6 +596,8 @@ __global__ void store_one_kernel(double* p) { *p = 1.0; }
 void set_ground(const State& s) {
   s.touch();
   s.ground_version = s.version;
+  s.active = 0;
+  s.active_version = s.version;
   KB_CUDA(cudaMemsetAsync(s.amps, 0, s.dim() * s.amp_bytes(), s.stream));
   if (s.precision == KETGPU_C64)
     set_one_kernel<float><<<1, 1, 0, s.stream>>>(static_cast<float2*>(s.amps));
@@ -602,16 +607,43 @@ void set_ground(const State& s) {
   KB_CUDA(cudaGetLastError());
 }
 
-void launch_pass(const State& s, const Plan& plan, const Pass& p) {
+PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false) {
+  const uint64_t all = s.dim() - 1;
+  if (plan.finite && s.version == s.active_version && s.active != all) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+      if (!s.exposed) {
+        active_ = s.active;
+        keep_ = true;
+      } else if (s.version == s.ground_version && is_ground(s)) {
+        active_ = 0;
+      }
+    }
+  }
+  active_ &= all;
+}
+
+PassRunner::~PassRunner() {
+  if (keep_) {
+    s_.active = active_;
+    s_.active_version = s_.version;
+  }
+}
+
+void PassRunner::launch(const Pass& p) {
+  const State& s = s_;
+  const Plan& plan = plan_;
   const bool ground = s.version == s.ground_version;
   s.touch();
+  const uint64_t dim = uint64_t{1} << active_bits(active_);
   if (p.kind == PassKind::NormCapture) {
     if (ground) {  // |0...0>: the squared norm is 1, no pass over the state
       store_one_kernel<<<1, 1, 0, s.stream>>>(plan.d_norm);
       count_launch();
       KB_CUDA(cudaGetLastError());
     } else {
-      norm_to_device(s, plan.d_norm + 2, plan.d_norm);
+      norm_to_device(s, dim, plan.d_norm + 2, plan.d_norm);
     }
     return;
   }
@@ -619,34 +651,43 @@ void launch_pass(const State& s, const Plan& plan, const Pass& p) {
     if (p.norm_out)  // the block before summed |out|^2 per CTA into the partials
       norm_from_partials(s, plan.d_norm + 2, plan.d_norm + 1);
     else
-      norm_to_device(s, plan.d_norm + 2, plan.d_norm + 1);
-    rescale_state(s, plan.d_norm, plan.d_norm + 1);
+      norm_to_device(s, dim, plan.d_norm + 2, plan.d_norm + 1);
+    rescale_state(s, dim, plan.d_norm, plan.d_norm + 1);
     return;
   }
   if (p.kind == PassKind::Diagonal) {
-    launch_diag(s, p, static_cast<const char*>(plan.d_diag) + plan.offdiag[p.diag_index]);
+    launch_diag(s, p, static_cast<const char*>(plan.d_diag) + plan.offdiag[p.diag_index], active_);
     return;
   }
+  if (p.kind == PassKind::Phase) {
+    if ((p.p0 & ~active_) == 0) {  // else it acts on zeros only
+      if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
+      else launch_pair<double>(s, p, active_);
+    }
+    return;
+  }
+  if (p.kind == PassKind::Pair) {
+    if ((p.p0 & ~active_) && (p.p1 & ~active_)) return;  // exchanges zeros
+    active_ |= p.p0 | p.p1;
+    if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
+    else launch_pair<double>(s, p, active_);
+    return;
+  }
+  for (int gi : p.gates)
+    for (int j = 0; j < gate_arity(plan.ops[gi].type); ++j) active_ |= uint64_t{1} << plan.ops[gi].q[j];
   if (p.kind == PassKind::SharedRun) {
-    launch_run(s, p, static_cast<const char*>(plan.d_runs) + plan.offrun[p.run_index]);
-    return;
-  }
-  if (p.kind != PassKind::Fused) {
-    if (s.precision == KETGPU_C64)
-      launch_pair<float>(s, p);
-    else
-      launch_pair<double>(s, p);
+    launch_run(s, p, static_cast<const char*>(plan.d_runs) + plan.offrun[p.run_index], active_);
     return;
   }
   if (s.precision == KETGPU_C128) {
     const void* mat = static_cast<const char*>(plan.d_mat64) + plan.off64[p.mat_index];
-    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, mat);
-    else launch_fused_simt<double>(s, p, mat);
+    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, mat, active_);
+    else launch_fused_simt<double>(s, p, mat, active_);
   } else if (p.tensor) {
     launch_fused_tc(s, p, static_cast<const char*>(plan.d_tc) + plan.offtc[p.mat_index],
-                    p.norm_out ? plan.d_norm + 2 : nullptr);
+                    p.norm_out ? plan.d_norm + 2 : nullptr, active_);
   } else {
-    launch_fused_simt<float>(s, p, static_cast<const char*>(plan.d_mat32) + plan.off32[p.mat_index]);
+    launch_fused_simt<float>(s, p, static_cast<const char*>(plan.d_mat32) + plan.off32[p.mat_index], active_);
   }
 }
 

@@ -623,6 +623,50 @@ void emit_fused(Plan& plan, int n, const ketgpu_op* ops, const Block& b, const P
   plan.passes.push_back(p);
 }
 
+// Orders the passes, under every dependency (passes that share a qubit keep
+// their order), so that qubits become active late: of the passes that can go
+// next, the one that leaves the fewest qubits active, the earliest on ties.
+// A run from |0...0> touches 2^active amplitudes a pass (PassRunner).  Once
+// all qubits are active the rest keep their order.
+void order_passes(Plan& plan, const ketgpu_op* ops, int n) {
+  const size_t P = plan.passes.size();
+  std::vector<uint64_t> touch(P, 0), grow(P, 0);
+  for (size_t i = 0; i < P; ++i) {
+    for (int gi : plan.passes[i].gates) {
+      touch[i] |= qubit_mask(ops[gi]);
+      if (!is_diagonal_gate(ops[gi].type)) grow[i] |= qubit_mask(ops[gi]);
+    }
+  }
+  const uint64_t all = n >= 64 ? ~uint64_t{0} : ((uint64_t{1} << n) - 1);
+  uint64_t active = 0;
+  std::vector<size_t> rest(P), order;
+  std::iota(rest.begin(), rest.end(), size_t{0});
+  while (!rest.empty() && active != all) {
+    uint64_t blocked = 0;
+    size_t best = 0;
+    int best_count = 65;
+    for (size_t r = 0; r < rest.size() && blocked != all; ++r) {
+      const size_t i = rest[r];
+      if (!(touch[i] & blocked)) {
+        const int c = __builtin_popcountll(active | grow[i]);
+        if (c < best_count) {
+          best_count = c;
+          best = r;
+        }
+      }
+      blocked |= touch[i];
+    }
+    active |= grow[rest[best]];
+    order.push_back(rest[best]);
+    rest.erase(rest.begin() + (std::ptrdiff_t)best);
+  }
+  order.insert(order.end(), rest.begin(), rest.end());
+  std::vector<Pass> sorted;
+  sorted.reserve(P);
+  for (size_t i : order) sorted.push_back(std::move(plan.passes[i]));
+  plan.passes = std::move(sorted);
+}
+
 }  // namespace
 
 // 48 features: scale (n, bytes), pass kind, block geometry (k, span, low /
@@ -874,6 +918,10 @@ void build_plan(Plan& plan, int n, const ketgpu_op* ops, uint64_t nops, const Pl
   flush();
   t_matrix_jobs = nullptr;
   compute_matrices(plan, ops, jobs);
+  if (opt.fusion == KETGPU_FUSE_GREEDY || opt.fusion == KETGPU_FUSE_LEARNED) order_passes(plan, ops, n);
+  for (uint64_t i = 0; i < nops && plan.finite; ++i)
+    if (is_unitary(ops[i].type))
+      for (double v : ops[i].p) plan.finite = plan.finite && std::isfinite(v);
   bool any_tensor = false;
   for (const Pass& p : plan.passes) any_tensor |= p.tensor;
   if ((opt.renormalize == 0 && any_tensor) || (opt.renormalize > 0 && !plan.passes.empty())) {

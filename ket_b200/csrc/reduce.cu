@@ -322,12 +322,12 @@ __global__ void rescale_kernel(T* __restrict__ s, uint64_t dim, const double* __
 
 }  // namespace
 
-void norm_to_device(const State& st, double* partials, double* out) {
+void norm_to_device(const State& st, uint64_t dim, double* partials, double* out) {
   if (st.precision == KETGPU_C64)
-    norm_partial<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), st.dim(),
+    norm_partial<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), dim,
                                                                    partials);
   else
-    norm_partial<double2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), st.dim(),
+    norm_partial<double2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), dim,
                                                                     partials);
   finish_partials<<<1, kRThreads, 0, st.stream>>>(partials, kNormBlocks, 1, out);
   count_launch(2);
@@ -340,15 +340,46 @@ void norm_from_partials(const State& st, const double* partials, double* out) {
   KB_CUDA(cudaGetLastError());
 }
 
-void rescale_state(const State& st, const double* target, const double* current) {
+void rescale_state(const State& st, uint64_t dim, const double* target, const double* current) {
   if (st.precision == KETGPU_C64)
-    rescale_kernel<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<float2*>(st.amps), st.dim(),
+    rescale_kernel<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<float2*>(st.amps), dim,
                                                                      target, current);
   else
-    rescale_kernel<double2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<double2*>(st.amps), st.dim(),
+    rescale_kernel<double2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<double2*>(st.amps), dim,
                                                                       target, current);
   count_launch();
   KB_CUDA(cudaGetLastError());
+}
+
+namespace {
+// Bit patterns other than those of |0...0> (a negative zero counts).
+__global__ void not_ground(const uint64_t* __restrict__ w, uint64_t words, uint64_t first, unsigned* flag) {
+  bool bad = false;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(w);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words / 2; i += stride) {
+    const ulonglong2 v = w2[i];
+    bad |= (i == 0 ? v.x != first : v.x != 0) || v.y != 0;
+  }
+  if ((words & 1) && blockIdx.x == 0 && threadIdx.x == 0) bad |= words == 1 ? w[0] != first : w[words - 1] != 0;
+  if (bad) *flag = 1u;
+}
+}  // namespace
+
+bool is_ground(const State& st) {
+  StreamScratch sc(sizeof(unsigned), st.device, st.stream);
+  unsigned* d = static_cast<unsigned*>(sc.p);
+  KB_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned), st.stream));
+  const bool c64 = st.precision == KETGPU_C64;
+  const uint64_t words = st.dim() * (c64 ? 1 : 2);
+  not_ground<<<grid_for(words, kRThreads * 16), kRThreads, 0, st.stream>>>(
+      static_cast<const uint64_t*>(st.amps), words, c64 ? 0x3f800000ull : 0x3ff0000000000000ull, d);
+  count_launch();
+  KB_CUDA(cudaGetLastError());
+  unsigned h = 1;
+  KB_CUDA(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st.stream));
+  KB_CUDA(cudaStreamSynchronize(st.stream));
+  return h == 0;
 }
 
 double reduce_norm(const State& st) {

@@ -93,19 +93,30 @@ void release_pools() {
     if (pool) cudaMemPoolTrimTo(pool, 0);
 }
 
+DeviceBlock::DeviceBlock(size_t bytes, int device, cudaStream_t stream) {
+  cudaMemPool_t pool = scratch_pool(device);
+  if (pool) KB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream));
+  else KB_CUDA(cudaMallocAsync(&p, bytes ? bytes : 8, stream));
+}
+
+DeviceBlock& DeviceBlock::operator=(DeviceBlock&& o) noexcept {
+  std::swap(p, o.p);
+  return *this;
+}
+
+// The free is not ordered after any stream's work (the owner saw to that).
+DeviceBlock::~DeviceBlock() {
+  if (p) cudaFree(p);
+}
+
 Plan::~Plan() {
-  if (device >= 0) {
-    int prev = -1;
-    cudaGetDevice(&prev);
-    cudaSetDevice(device);
-    if (d_mat64) cudaFree(d_mat64);
-    if (d_mat32) cudaFree(d_mat32);
-    if (d_tc) cudaFree(d_tc);
-    if (d_norm) cudaFree(d_norm);
-    if (d_diag) cudaFree(d_diag);
-    if (d_runs) cudaFree(d_runs);
-    if (prev >= 0) cudaSetDevice(prev);
-  }
+  if (!block.p) return;
+  int prev = -1;
+  cudaGetDevice(&prev);
+  cudaSetDevice(device);
+  if (!idle) cudaDeviceSynchronize();
+  block = DeviceBlock();
+  if (prev >= 0) cudaSetDevice(prev);
 }
 
 void pauli_masks(int n, const char* pauli, uint64_t& flip, uint64_t& sign, int& q) {
@@ -129,138 +140,6 @@ void pauli_masks(int n, const char* pauli, uint64_t& flip, uint64_t& sign, int& 
     }
   }
   q = num_y % 4;
-}
-
-void upload_plan_copies(Plan& plan, int device);
-
-// Device copies of a plan's tables, once per plan and device.  They go up
-// with cudaMemcpy from pageable host vectors, which may return before the
-// data lands; the kernels that read them run on the states' non-blocking
-// streams, which do not wait for the legacy stream the copies use, so the
-// copies are waited for here.
-void upload_plan_matrices(Plan& plan, int device) {
-  if (plan.device == device) return;
-  upload_plan_copies(plan, device);
-  KB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-}
-
-void upload_plan_copies(Plan& plan, int device) {
-  if (plan.device >= 0) fail(KETGPU_ERR_INVALID, "plan was prepared for another device");
-  plan.device = device;
-  for (const Pass& p : plan.passes)
-    if (p.kind == PassKind::NormCapture && !plan.d_norm)
-      KB_CUDA(cudaMalloc(&plan.d_norm, sizeof(double) * (2 + kNormBlocks)));
-  if (!plan.diags.empty()) {
-    std::vector<unsigned char> all, one;
-    plan.offdiag.assign(plan.diags.size(), 0);
-    for (size_t i = 0; i < plan.diags.size(); ++i) {
-      diag_device_data(plan.diags[i], plan.n, plan.precision, one);
-      plan.offdiag[i] = all.size();
-      all.insert(all.end(), one.begin(), one.end());
-      while (all.size() % 256) all.push_back(0);
-    }
-    KB_CUDA(cudaMalloc(&plan.d_diag, all.size()));
-    KB_CUDA(cudaMemcpy(plan.d_diag, all.data(), all.size(), cudaMemcpyHostToDevice));
-  }
-  if (!plan.runs.empty()) {
-    std::vector<unsigned char> all, one;
-    plan.offrun.assign(plan.runs.size(), 0);
-    for (size_t i = 0; i < plan.runs.size(); ++i) {
-      run_device_data(plan.runs[i], plan.precision, one);
-      plan.offrun[i] = all.size();
-      all.insert(all.end(), one.begin(), one.end());
-      while (all.size() % 256) all.push_back(0);
-    }
-    KB_CUDA(cudaMalloc(&plan.d_runs, all.size()));
-    KB_CUDA(cudaMemcpy(plan.d_runs, all.data(), all.size(), cudaMemcpyHostToDevice));
-  }
-  if (plan.matrices.empty()) return;
-  std::vector<double> h64;
-  std::vector<float> h32;
-  std::vector<uint32_t> htc;
-  std::vector<size_t> tc_jobs;
-  size_t tc_words = 0;
-  plan.off64.assign(plan.matrices.size(), 0);
-  plan.off32.assign(plan.matrices.size(), 0);
-  plan.offtc.assign(plan.matrices.size(), 0);
-  // matrix index -> whether its pass is on the tensor cores
-  std::vector<int> kof(plan.matrices.size(), 0);
-  std::vector<char> tensor(plan.matrices.size(), 0);
-  for (const Pass& p : plan.passes)
-    if (p.kind == PassKind::Fused) {
-      kof[p.mat_index] = p.k;
-      tensor[p.mat_index] = p.tensor;
-    }
-  for (size_t i = 0; i < plan.matrices.size(); ++i) {
-    const std::vector<cplx>& m = plan.matrices[i];
-    const int dim = 1 << kof[i];
-    if (plan.precision == KETGPU_C128) {
-      plan.off64[i] = h64.size() * sizeof(double);
-      for (int c = 0; c < dim; ++c)
-        for (int r = 0; r < dim; ++r) {
-          h64.push_back(m[(size_t)r * dim + c].real());
-          h64.push_back(m[(size_t)r * dim + c].imag());
-        }
-      while (h64.size() % 2) h64.push_back(0);
-    } else if (tensor[i]) {
-      // place now, build below on host threads
-      plan.offtc[i] = tc_words * sizeof(uint32_t);
-      tc_jobs.push_back(i);
-      tc_words += (tc_image_bytes(kof[i]) / 4 + 63) / 64 * 64;  // 256-byte alignment
-    } else {
-      plan.off32[i] = h32.size() * sizeof(float);
-      for (int c = 0; c < dim; ++c)
-        for (int r = 0; r < dim; ++r) {
-          h32.push_back((float)m[(size_t)r * dim + c].real());
-          h32.push_back((float)m[(size_t)r * dim + c].imag());
-        }
-      while (h32.size() % 4) h32.push_back(0);
-    }
-  }
-  if (!h64.empty()) {
-    KB_CUDA(cudaMalloc(&plan.d_mat64, h64.size() * sizeof(double)));
-    KB_CUDA(cudaMemcpy(plan.d_mat64, h64.data(), h64.size() * sizeof(double), cudaMemcpyHostToDevice));
-  }
-  if (!h32.empty()) {
-    KB_CUDA(cudaMalloc(&plan.d_mat32, h32.size() * sizeof(float)));
-    KB_CUDA(cudaMemcpy(plan.d_mat32, h32.data(), h32.size() * sizeof(float), cudaMemcpyHostToDevice));
-  }
-  if (!tc_jobs.empty()) {
-    // tensor-core B images (fp16 splits of every entry) on host threads,
-    // each written at its place in htc
-    htc.assign(tc_words, 0u);
-    auto build = [&](size_t i) {
-      std::vector<uint32_t> img;
-      build_tc_image(plan.matrices[i], kof[i], img);
-      std::memcpy(htc.data() + plan.offtc[i] / sizeof(uint32_t), img.data(), img.size() * sizeof(uint32_t));
-    };
-    const unsigned nt = tc_jobs.size() < 4 ? 1u
-                        : std::min<unsigned>(16u, std::max(1u, std::thread::hardware_concurrency()));
-    if (nt <= 1) {
-      for (size_t i : tc_jobs) build(i);
-    } else {
-      std::atomic<size_t> next{0};
-      std::exception_ptr err;
-      std::atomic<bool> failed{false};
-      std::vector<std::thread> th;
-      for (unsigned t = 0; t < nt; ++t)
-        th.emplace_back([&] {
-          for (size_t j; (j = next.fetch_add(1)) < tc_jobs.size();) {
-            try {
-              build(tc_jobs[j]);
-            } catch (...) {
-              if (!failed.exchange(true)) err = std::current_exception();
-            }
-          }
-        });
-      for (auto& x : th) x.join();
-      if (err) std::rethrow_exception(err);
-    }
-  }
-  if (!htc.empty()) {
-    KB_CUDA(cudaMalloc(&plan.d_tc, htc.size() * sizeof(uint32_t)));
-    KB_CUDA(cudaMemcpy(plan.d_tc, htc.data(), htc.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  }
 }
 
 int tc_error_flag(bool reset);
@@ -470,10 +349,10 @@ void upload(State& s, uint64_t first, uint64_t count, const double* in) {
   }
 }
 
-void execute(const Plan& plan, State& s) {
+void execute(const Plan& plan, State& s, bool one_stream = false) {
   need(plan.n == s.n, "plan and state have different qubit counts");
   need(plan.precision == s.precision, "plan and state have different precisions");
-  upload_plan_matrices(const_cast<Plan&>(plan), s.device);
+  upload_plan_tables(const_cast<Plan&>(plan), s.device, s.stream, one_stream);
   PassRunner run(s, plan);
   for (const Pass& p : plan.passes) run.launch(p);
 }
@@ -698,8 +577,9 @@ KB_API int ketgpu_apply(ketgpu_state* s, const ketgpu_op* ops, uint64_t n_ops, c
     Plan plan;
     build_plan(plan, st.n, ops, n_ops, o);
     DeviceGuard g(st.device);
-    execute(plan, st);
+    execute(plan, st, true);
     KB_CUDA(cudaStreamSynchronize(st.stream));
+    plan.idle = true;
     check_tc_flag();
   });
 }
@@ -735,8 +615,9 @@ KB_API int ketgpu_run(int32_t n, const ketgpu_op* ops, uint64_t n_ops, const ket
     }
     const double state_ms = ms_since(t1);
     const auto t2 = std::chrono::steady_clock::now();
-    execute(plan, *st);
+    execute(plan, *st, true);
     KB_CUDA(cudaStreamSynchronize(st->stream));
+    plan.idle = true;
     const double exec_ms = ms_since(t2);
     const auto t3 = std::chrono::steady_clock::now();
     DownloadTimes dt;
@@ -878,7 +759,7 @@ KB_API int ketgpu_plan_execute_timed(const ketgpu_plan* p, ketgpu_state* s, floa
     State& st = *as_state(s);
     need(plan.n == st.n && plan.precision == st.precision, "plan and state do not match");
     DeviceGuard g(st.device);
-    upload_plan_matrices(const_cast<Plan&>(plan), st.device);
+    upload_plan_tables(const_cast<Plan&>(plan), st.device, st.stream, false);
     const size_t np = plan.passes.size();
     std::vector<cudaEvent_t> ev(np + 1);
     for (auto& e : ev) KB_CUDA(cudaEventCreate(&e));
@@ -975,7 +856,7 @@ KB_API int ketgpu_plan_pass_matrix(const ketgpu_plan* p, uint64_t index, double*
     if (index >= plan.passes.size()) fail(KETGPU_ERR_OUT_OF_RANGE, "pass index out of range");
     const Pass& ps = plan.passes[index];
     if (ps.kind != PassKind::Fused) fail(KETGPU_ERR_INVALID, "pass is not a dense block");
-    const std::vector<cplx>& m = plan.matrices[ps.mat_index];
+    const std::vector<cplx> m = block_matrix(plan.ops.data(), ps.gates, ps.qubits, ps.k);
     *count = 2 * m.size();
     const uint64_t nd = std::min<uint64_t>(capacity, 2 * m.size());
     for (uint64_t i = 0; i < nd; ++i) out[i] = (i & 1) ? m[i / 2].imag() : m[i / 2].real();

@@ -11,8 +11,8 @@
 //   phi(x) = c0 + sum_i a_i x_i + sum_{i<j} b_ij x_i x_j.
 //
 // The kernel splits x into L = min(n, 12) low bits and n - L high bits.  The
-// pair terms inside the low bits are one table of 2^L phases, built on the
-// host in FP64.  A CTA handles 2^L consecutive amplitudes, whose high bits h
+// pair terms inside the low bits are one table of 2^L phases, formed in FP64
+// with the plan's other tables (tables.cu).  A CTA handles 2^L consecutive amplitudes, whose high bits h
 // are fixed.  For that chunk, the linear coefficients of the low bits
 // (a_i + sum_j b_ij h_j) and the constant phi(h) fold into two 64-entry tables,
 // built in FP64 with sincos.  Each amplitude then costs three complex products
@@ -70,40 +70,18 @@ void add_diagonal_gate(const ketgpu_op& op, DiagPoly& poly, int n) {
   }
 }
 
-// Device layout: table[2^L] (state precision, re/im), then FP64
-// [c0, a[n], blh[L][H], bhh[H][H]] with H = n - L, blh[i][j] = b(i, L+j),
+// Device layout: table[2^L] (state precision, re/im; built by tables.cu), then
+// FP64 [c0, a[n], blh[L][H], bhh[H][H]] with H = n - L, blh[i][j] = b(i, L+j),
 // bhh[j][k] = b(L+j, L+k) for j < k.
-void diag_device_data(const DiagPoly& poly, int n, int precision, std::vector<unsigned char>& out) {
+void diag_coefficients(const DiagPoly& poly, int n, std::vector<double>& prm) {
   const int L = std::min(n, kDiagLowBits), H = n - L;
-  const size_t CH = size_t{1} << L;
-  std::vector<double> q(CH, 0.0);
-  for (size_t x = 1; x < CH; ++x) {
-    const int top = 63 - __builtin_clzll(x);
-    double v = q[x ^ (size_t{1} << top)];
-    for (int i = 0; i < top; ++i)
-      if ((x >> i) & 1) v += poly.b[(size_t)i * n + top];
-    q[x] = v;
-  }
-  const size_t amp = precision == KETGPU_C64 ? 8 : 16;
-  std::vector<double> prm;
+  prm.clear();
   prm.push_back(poly.c0);
   for (int i = 0; i < n; ++i) prm.push_back(poly.a[i]);
   for (int i = 0; i < L; ++i)
     for (int j = 0; j < H; ++j) prm.push_back(poly.b[(size_t)i * n + L + j]);
   for (int j = 0; j < H; ++j)
     for (int k = 0; k < H; ++k) prm.push_back(k > j ? poly.b[(size_t)(L + j) * n + L + k] : 0.0);
-  out.assign(CH * amp + prm.size() * sizeof(double), 0);
-  for (size_t x = 0; x < CH; ++x) {
-    const double c = std::cos(q[x]), s = std::sin(q[x]);
-    if (precision == KETGPU_C64) {
-      const float v[2] = {(float)c, (float)s};
-      std::memcpy(&out[x * amp], v, sizeof v);
-    } else {
-      const double v[2] = {c, s};
-      std::memcpy(&out[x * amp], v, sizeof v);
-    }
-  }
-  std::memcpy(&out[CH * amp], prm.data(), prm.size() * sizeof(double));
 }
 
 namespace {

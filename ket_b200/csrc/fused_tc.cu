@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "tc_layout.cuh"
 
 namespace kb {
 
@@ -156,14 +157,6 @@ __host__ __device__ __forceinline__ uint32_t sw128_offset(int row, int kk, int r
   const int kb = kk >> 5;             // 32 fp32 per 128-byte atom row
   const int chunk = (kk & 31) >> 2;   // 16-byte chunk in the row
   return (uint32_t)(kb * rows * 128 + row * 128 + ((chunk ^ (row & 7)) << 4) + ((kk & 3) << 2));
-}
-
-// Byte offset of fp16 element (row, kk) of a K-major SW128 image with `rows`
-// rows (the B images).
-__host__ __device__ __forceinline__ uint32_t sw128_offset_h(int row, int kk, int rows) {
-  const int kb = kk >> 6;             // 64 fp16 per 128-byte atom row
-  const int chunk = (kk & 63) >> 3;   // 16-byte chunk in the row
-  return (uint32_t)(kb * rows * 128 + row * 128 + ((chunk ^ (row & 7)) << 4) + ((kk & 7) << 1));
 }
 
 // Offsets of tile amplitude e (address order: bit j of e <-> qubit

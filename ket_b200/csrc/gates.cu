@@ -637,6 +637,7 @@ void PassRunner::launch(const Pass& p) {
   const bool ground = s.version == s.ground_version;
   s.touch();
   const uint64_t dim = uint64_t{1} << active_bits(active_);
+  const void* table = static_cast<const char*>(plan.block.p) + p.table;
   if (p.kind == PassKind::NormCapture) {
     if (ground) {  // |0...0>: the squared norm is 1, no pass over the state
       store_one_kernel<<<1, 1, 0, s.stream>>>(plan.d_norm);
@@ -656,7 +657,7 @@ void PassRunner::launch(const Pass& p) {
     return;
   }
   if (p.kind == PassKind::Diagonal) {
-    launch_diag(s, p, static_cast<const char*>(plan.d_diag) + plan.offdiag[p.diag_index], active_);
+    launch_diag(s, p, table, active_);
     return;
   }
   if (p.kind == PassKind::Phase) {
@@ -676,18 +677,16 @@ void PassRunner::launch(const Pass& p) {
   for (int gi : p.gates)
     for (int j = 0; j < gate_arity(plan.ops[gi].type); ++j) active_ |= uint64_t{1} << plan.ops[gi].q[j];
   if (p.kind == PassKind::SharedRun) {
-    launch_run(s, p, static_cast<const char*>(plan.d_runs) + plan.offrun[p.run_index], active_);
+    launch_run(s, p, table, active_);
     return;
   }
   if (s.precision == KETGPU_C128) {
-    const void* mat = static_cast<const char*>(plan.d_mat64) + plan.off64[p.mat_index];
-    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, mat, active_);
-    else launch_fused_simt<double>(s, p, mat, active_);
+    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, table, active_);
+    else launch_fused_simt<double>(s, p, table, active_);
   } else if (p.tensor) {
-    launch_fused_tc(s, p, static_cast<const char*>(plan.d_tc) + plan.offtc[p.mat_index],
-                    p.norm_out ? plan.d_norm + 2 : nullptr, active_);
+    launch_fused_tc(s, p, table, p.norm_out ? plan.d_norm + 2 : nullptr, active_);
   } else {
-    launch_fused_simt<float>(s, p, static_cast<const char*>(plan.d_mat32) + plan.off32[p.mat_index], active_);
+    launch_fused_simt<float>(s, p, table, active_);
   }
 }
 

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <complex>
 #include <cstdint>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -52,6 +53,16 @@ struct StreamScratch {
   StreamScratch& operator=(const StreamScratch&) = delete;
 };
 void release_pools();
+// Device memory from the same pool that outlives the call that made it.  Its
+// owner frees it when nothing on the device uses it any more.
+struct DeviceBlock {
+  void* p = nullptr;
+  DeviceBlock() = default;
+  DeviceBlock(size_t bytes, int device, cudaStream_t stream);
+  DeviceBlock(DeviceBlock&& o) noexcept : p(o.p) { o.p = nullptr; }
+  DeviceBlock& operator=(DeviceBlock&& o) noexcept;
+  ~DeviceBlock();
+};
 
 // ---- state -----------------------------------------------------------------
 struct State {
@@ -115,7 +126,7 @@ struct Pass {
   // Fused
   int k = 0;
   int qubits[6] = {0, 0, 0, 0, 0, 0};  // sorted ascending; matrix bit b <-> qubits[b]
-  size_t mat_index = 0;                // into Plan::matrices
+  size_t table = 0;                    // Fused, Diagonal, SharedRun: its table's offset in Plan::block
   bool tensor = false;                 // tcgen05 path
   // tcgen05 block directly before the plan's NormRestore: it also writes
   // per-CTA FP64 sums of |out|^2 into the plan's norm partials, and the
@@ -145,19 +156,16 @@ struct Plan {
   std::vector<ketgpu_op> ops;  // the circuit the plan was built from
   bool finite = true;          // every gate parameter is a finite number
   std::vector<Pass> passes;
-  std::vector<std::vector<cplx>> matrices;  // FP64 block matrices (host)
-  // device copies, built lazily per device: FP64 (c128 SIMT), FP32 (c64 SIMT),
-  // tcgen05 B operands (hi/lo fp16 images in the shared-memory layout)
-  void* d_mat64 = nullptr;
-  void* d_mat32 = nullptr;
-  void* d_tc = nullptr;
-  double* d_norm = nullptr;  // [captured, current, block partials...]
-  std::vector<DiagPoly> diags;  // Diagonal passes (host)
-  void* d_diag = nullptr;       // per Diagonal pass: low-bit table + coefficients
+  std::vector<DiagPoly> diags;          // Diagonal passes (host)
   std::vector<std::vector<Pass>> runs;  // SharedRun passes: each gate lowered (host)
-  void* d_runs = nullptr;               // their device gate records
-  std::vector<size_t> off64, off32, offtc, offdiag, offrun;
+  // Device tables (tables.cu), made at the first execution: block matrices
+  // (transposed FP64 or FP32) or tensor-core operands, diagonal tables with
+  // their coefficients, gate records of shared-memory runs.
+  DeviceBlock block;
+  double* d_norm = nullptr;  // [captured, current, block partials...]
   int device = -1;
+  bool idle = false;  // nothing that reads the tables is in flight
+  std::mutex mu;      // guards the tables' making
   ketgpu_plan_stats stats{};
   ~Plan();
 };
@@ -173,9 +181,10 @@ void single_matrix(int type, const double* p, cplx m[4]);
 Pass lower_gate(const ketgpu_op& op);
 // Per-gate cost in state passes (fraction of the state each pass moves).
 double gate_traffic_fraction(const ketgpu_op& op);
-// Dense block matrix of a gate list restricted to `qubits` (bit b <-> qubits[b]).
-std::vector<cplx> block_matrix(const std::vector<const ketgpu_op*>& gates,
-                               const int* qubits, int k);
+// The gates ops[gates[i]] lowered onto the bits of a block (bit b <-> qubits[b]).
+std::vector<Pass> lower_block(const ketgpu_op* ops, const std::vector<int>& gates, const int* qubits, int k);
+// Their dense matrix, on the host.
+std::vector<cplx> block_matrix(const ketgpu_op* ops, const std::vector<int>& gates, const int* qubits, int k);
 
 // ---- planner ---------------------------------------------------------------
 struct PlanOptions {
@@ -227,7 +236,8 @@ class PassRunner {
 // Whether every amplitude but amps[0] is zero and amps[0] is 1 (one read;
 // synchronises).
 bool is_ground(const State& s);
-void upload_plan_matrices(Plan& plan, int device);
+// one_stream: the plan runs on `stream` only (the tables are not waited for).
+void upload_plan_tables(Plan& plan, int device, cudaStream_t stream, bool one_stream);
 // norm_partials: null, or kNormBlocks doubles that receive the per-CTA sums
 // of |out|^2 (zero beyond the grid).  active (here and below): the index bits
 // that can be set in a nonzero amplitude, the pass's qubits included.
@@ -242,12 +252,13 @@ void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, uint64_t
 // encoder of the driver.
 void tc_form(int n, const Pass& p, int* tma_dims, int* direct);
 // Diagonal pass: device data = table (2^L complex, state precision) then FP64
-// coefficients, laid out by diag_device_data (diag.cu).
+// coefficients.
 void launch_diag(const State& s, const Pass& p, const void* data, uint64_t active);
 // SharedRun pass: device gate records laid out by run_device_data (gates.cu).
 void launch_run(const State& s, const Pass& p, const void* data, uint64_t active);
 void run_device_data(const std::vector<Pass>& gates, int precision, std::vector<unsigned char>& out);
-void diag_device_data(const DiagPoly& poly, int n, int precision, std::vector<unsigned char>& out);
+// The coefficients the diagonal kernel reads after its table (diag.cu).
+void diag_coefficients(const DiagPoly& poly, int n, std::vector<double>& out);
 bool is_diagonal_gate(int type);
 // Add one diagonal gate's phase terms to a polynomial.
 void add_diagonal_gate(const ketgpu_op& op, DiagPoly& poly, int n);

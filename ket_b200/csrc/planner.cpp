@@ -195,21 +195,26 @@ void apply_small(const Pass& p, cplx* v, int nloc) {
 
 }  // namespace
 
-std::vector<cplx> block_matrix(const std::vector<const ketgpu_op*>& gates, const int* qubits, int k) {
-  const int dim = 1 << k;
+std::vector<Pass> lower_block(const ketgpu_op* ops, const std::vector<int>& gates, const int* qubits, int k) {
   std::vector<Pass> local;
   local.reserve(gates.size());
-  for (const ketgpu_op* g : gates) {
-    ketgpu_op o = *g;
+  for (int gi : gates) {
+    ketgpu_op o = ops[gi];
     for (int j = 0; j < gate_arity(o.type); ++j) {
       int li = -1;
       for (int b = 0; b < k; ++b)
         if (qubits[b] == o.q[j]) li = b;
-      if (li < 0) fail(KETGPU_ERR_LOGIC, "block_matrix: gate outside block");
+      if (li < 0) fail(KETGPU_ERR_LOGIC, "lower_block: gate outside block");
       o.q[j] = li;
     }
     local.push_back(lower_gate(o));
   }
+  return local;
+}
+
+std::vector<cplx> block_matrix(const ketgpu_op* ops, const std::vector<int>& gates, const int* qubits, int k) {
+  const int dim = 1 << k;
+  const std::vector<Pass> local = lower_block(ops, gates, qubits, k);
   std::vector<cplx> mat((size_t)dim * dim);
   std::vector<cplx> col(dim);
   for (int c = 0; c < dim; ++c) {
@@ -531,49 +536,7 @@ void emit_diagonal(Plan& plan, int n, const ketgpu_op* ops, const Block& b) {
   plan.passes.push_back(p);
 }
 
-// Block matrices of the plan being built on this thread: emit_fused records
-// each one as a job and build_plan computes them all at the end, in
-// parallel (at k = 6 they are most of the planning time).
-struct MatrixJob {
-  size_t index;
-  std::vector<int> gates;
-  std::vector<int> qubits;
-};
-thread_local std::vector<MatrixJob>* t_matrix_jobs = nullptr;
-
-void compute_matrices(Plan& plan, const ketgpu_op* ops, const std::vector<MatrixJob>& jobs) {
-  auto work = [&](const MatrixJob& jb) {
-    std::vector<const ketgpu_op*> gs;
-    for (int gi : jb.gates) gs.push_back(&ops[gi]);
-    plan.matrices[jb.index] = block_matrix(gs, jb.qubits.data(), (int)jb.qubits.size());
-  };
-  const unsigned nt = jobs.size() < 16 ? 1u
-                      : std::min<unsigned>(16u, std::max(1u, std::thread::hardware_concurrency()));
-  if (nt <= 1) {
-    for (const MatrixJob& jb : jobs) work(jb);
-    return;
-  }
-  std::atomic<size_t> next{0};
-  std::exception_ptr err;
-  std::atomic<bool> failed{false};
-  std::vector<std::thread> th;
-  for (unsigned t = 0; t < nt; ++t)
-    th.emplace_back([&] {
-      for (size_t i; (i = next.fetch_add(1)) < jobs.size();) {
-        try {
-          work(jobs[i]);
-        } catch (...) {
-          if (!failed.exchange(true)) err = std::current_exception();
-        }
-      }
-    });
-  for (auto& x : th) x.join();
-  if (err) std::rethrow_exception(err);
-}
-
 void emit_fused(Plan& plan, int n, const ketgpu_op* ops, const Block& b, const PlanOptions& opt) {
-  std::vector<const ketgpu_op*> gs;
-  for (int gi : b.gates) gs.push_back(&ops[gi]);
   std::vector<int> qs = b.qubits;
   std::sort(qs.begin(), qs.end());
   // complex64 on the tensor cores: a 2- or 3-qubit block is padded to 4
@@ -598,7 +561,7 @@ void emit_fused(Plan& plan, int n, const ketgpu_op* ops, const Block& b, const P
   p.n_gates = (int)b.gates.size();
   p.gates = b.gates;
   if (k == 1) {  // one 2x2 through the streaming pair kernel
-    const std::vector<cplx> mat = block_matrix(gs, qs.data(), k);
+    const std::vector<cplx> mat = block_matrix(ops, b.gates, qs.data(), k);
     p.kind = PassKind::Pair;
     p.mode = kPairGeneral;
     p.nfixed = 1;
@@ -613,13 +576,6 @@ void emit_fused(Plan& plan, int n, const ketgpu_op* ops, const Block& b, const P
   p.k = k;
   for (int j = 0; j < k; ++j) p.qubits[j] = qs[j];
   p.tensor = block_on_tensor_cores(n, k, opt);
-  p.mat_index = plan.matrices.size();
-  if (t_matrix_jobs) {
-    plan.matrices.emplace_back();
-    t_matrix_jobs->push_back({p.mat_index, b.gates, qs});
-  } else {
-    plan.matrices.push_back(block_matrix(gs, qs.data(), k));
-  }
   plan.passes.push_back(p);
 }
 
@@ -738,12 +694,6 @@ void build_plan(Plan& plan, int n, const ketgpu_op* ops, uint64_t nops, const Pl
   plan.precision = opt.precision;
   plan.ops.assign(ops, ops + nops);
   plan.passes.clear();
-  plan.matrices.clear();
-  std::vector<MatrixJob> jobs;
-  struct JobScope {
-    explicit JobScope(std::vector<MatrixJob>* j) { t_matrix_jobs = j; }
-    ~JobScope() { t_matrix_jobs = nullptr; }
-  } job_scope(&jobs);
   uint64_t n_gates = 0;
   double predicted = 0;
   const size_t amp = opt.precision == KETGPU_C64 ? 8 : 16;
@@ -916,8 +866,6 @@ void build_plan(Plan& plan, int n, const ketgpu_op* ops, uint64_t nops, const Pl
     }
   }
   flush();
-  t_matrix_jobs = nullptr;
-  compute_matrices(plan, ops, jobs);
   if (opt.fusion == KETGPU_FUSE_GREEDY || opt.fusion == KETGPU_FUSE_LEARNED) order_passes(plan, ops, n);
   for (uint64_t i = 0; i < nops && plan.finite; ++i)
     if (is_unitary(ops[i].type))

@@ -11,6 +11,7 @@ blocks (``append``) are kept as nodes and flattened with ket's wire remap
 from __future__ import annotations
 
 import enum
+import struct
 from typing import List, Sequence
 
 import numpy as np
@@ -49,6 +50,11 @@ class GateType(enum.IntEnum):
     Composite = 26
     Probe = 27
 
+
+# one ketgpu_op (OP_DTYPE): six 32-bit integers, three doubles
+_pack_op = struct.Struct("<6i3d").pack
+_NO_QUBITS = ((0, 0, 0), (0, 0), (0,), ())
+_NO_PARAMS = ((0.0, 0.0, 0.0), (0.0, 0.0), (0.0,), ())
 
 CLIFFORD = {GateType.H, GateType.X, GateType.Y, GateType.Z, GateType.S, GateType.Sdg,
             GateType.CX, GateType.CY, GateType.CZ, GateType.Swap,
@@ -202,23 +208,20 @@ class Circuit:
         return out
 
     def to_ops(self) -> np.ndarray:
-        gates = self.flat_gates()
-        ops = np.zeros(len(gates), dtype=OP_DTYPE)
-        for i, g in enumerate(gates):
-            ops[i]["type"] = int(g.type)
-            if g.type in (GateType.Barrier, GateType.Probe):
-                ops[i]["nq"] = 0
-            elif g.type == GateType.Measure:
-                ops[i]["nq"] = 1
-                ops[i]["q"][0] = g.qubits[0]
-                ops[i]["q"][1] = g.clbit
+        gates = self._gates
+        if any(g.type is GateType.Composite for g in gates):
+            gates = self.flat_gates()
+        out = bytearray()
+        for g in gates:
+            t = g.type
+            if t is GateType.Barrier or t is GateType.Probe:
+                out += _pack_op(t, 0, 0, 0, 0, 0, 0.0, 0.0, 0.0)
+            elif t is GateType.Measure:
+                out += _pack_op(t, 1, g.qubits[0], g.clbit, 0, 0, 0.0, 0.0, 0.0)
             else:
-                ops[i]["nq"] = len(g.qubits)
-                for j, q in enumerate(g.qubits):
-                    ops[i]["q"][j] = q
-                for j, p in enumerate(g.params):
-                    ops[i]["p"][j] = p
-        return ops
+                q, p = g.qubits, g.params
+                out += _pack_op(t, len(q), *q, *_NO_QUBITS[len(q)], 0, *p, *_NO_PARAMS[len(p)])
+        return np.frombuffer(out, dtype=OP_DTYPE)
 
     def is_clifford(self) -> bool:
         """backend.cpp:16-47: only H X Y Z S Sdg CX CY CZ Swap (+ structural)."""

@@ -212,6 +212,15 @@ __attribute__((target("avx512f"))) void widen_avx512(const float* src, double* d
   _mm_sfence();
 }
 
+// Copy with non-temporal stores, for the same reason.
+__attribute__((target("avx512f"))) void copy_avx512(const char* src, char* dst, uint64_t n) {
+  uint64_t i = std::min<uint64_t>(n, (64 - (reinterpret_cast<uintptr_t>(dst) & 63)) & 63);
+  std::memcpy(dst, src, i);
+  for (; i + 64 <= n; i += 64) _mm512_stream_si512(reinterpret_cast<__m512i*>(dst + i), _mm512_loadu_si512(src + i));
+  std::memcpy(dst + i, src + i, n - i);
+  _mm_sfence();
+}
+
 void widen_scalar(const float* src, double* dst, uint64_t n) {
   for (uint64_t i = 0; i < n; ++i) dst[i] = (double)src[i];
 }
@@ -221,9 +230,9 @@ bool have_avx512() {
   return v;
 }
 
-// Pinned staging for complex64 downloads, kept for the life of the process:
-// a ring of down_ring() buffers of down_chunk() amplitudes (default 4 x 16 MB),
-// all but one of them in flight.  One download at a time uses it.  At 30
+// Pinned staging for downloads, kept for the life of the process: a ring of
+// down_ring() buffers of down_chunk() bytes (default 4 x 16 MB), all but one
+// of them in flight.  One download at a time uses it.  complex64 at 30
 // qubits 4 x 16 MB matched the raw copy (157-160 ms against 162 ms to pinned
 // memory); 3 x 32 MB took 181-188 ms and 4 x 8 MB 213-243 ms, the widening
 // no longer hidden behind the copy.  KETGPU_DOWN_CHUNK_MB and
@@ -235,7 +244,7 @@ uint64_t env_u64(const char* name, uint64_t def, uint64_t lo, uint64_t hi) {
   return v < lo ? lo : (v > hi ? hi : v);
 }
 uint64_t down_chunk() {
-  static const uint64_t v = env_u64("KETGPU_DOWN_CHUNK_MB", 16, 1, 256) * (uint64_t{1} << 20) / 8;
+  static const uint64_t v = env_u64("KETGPU_DOWN_CHUNK_MB", 16, 1, 256) * (uint64_t{1} << 20);
   return v;
 }
 int down_ring() {
@@ -249,7 +258,7 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
-// Where a complex64 download spends the calling thread's time: waiting for
+// Where a staged download spends the calling thread's time: waiting for
 // device-to-host copies, and widening its share of each chunk.
 struct DownloadTimes {
   double copy_wait_ms = 0.0, widen_ms = 0.0;
@@ -258,44 +267,104 @@ struct DownloadTimes {
 // Phase times of the calling thread's last ketgpu_run (ketgpu_run_last_profile).
 thread_local double t_run_profile[6] = {0, 0, 0, 0, 0, 0};
 
-void download(const State& s, uint64_t first, uint64_t count, double* out, DownloadTimes* times = nullptr) {
-  if (s.precision == KETGPU_C128) {
-    KB_CUDA(cudaMemcpyAsync(out, static_cast<const double2*>(s.amps) + first, count * 16,
-                            cudaMemcpyDeviceToHost, s.stream));
+// Below this a copy goes straight to the caller's (pageable) buffer.
+constexpr uint64_t kDirectBytes = uint64_t{4} << 20;
+// Piece of a download that fits the staging buffers as a whole.
+constexpr uint64_t kPieceBytes = uint64_t{1} << 20;
+
+// Amplitudes [first, first + count) into a host buffer, in the state's format
+// or (widen: complex64 only) as complex128.  Large buffers go through pinned
+// staging and are written by several threads: most of the time of a copy
+// into fresh pageable memory is its page faults (32 MB: 7.4 ms in one call).
+void download(const State& s, uint64_t first, uint64_t count, void* out, bool widen, DownloadTimes* times = nullptr) {
+  const uint64_t amp = s.amp_bytes(), total = count * amp;
+  const char* src = static_cast<const char*>(s.amps) + first * amp;
+  if (!count) return;
+  if (!widen && total < kDirectBytes) {
+    KB_CUDA(cudaMemcpyAsync(out, src, total, cudaMemcpyDeviceToHost, s.stream));
     KB_CUDA(cudaStreamSynchronize(s.stream));
     return;
   }
   std::lock_guard<std::mutex> lock(g_stage_mu);
   const uint64_t chunk = down_chunk();
   const int ring = down_ring();
-  if (!g_stage) KB_CUDA(cudaMallocHost(&g_stage, ring * chunk * 8));
-  std::vector<float2*> buf(ring);
-  for (int b = 0; b < ring; ++b) buf[b] = static_cast<float2*>(g_stage) + b * chunk;
+  if (!g_stage) KB_CUDA(cudaMallocHost(&g_stage, ring * chunk));
+  char* stage = static_cast<char*>(g_stage);
+  const bool fast = have_avx512();
+  // staged bytes [at, at + len) of the range, at `from`, into the caller's buffer
+  auto emit = [&](const char* from, uint64_t at, uint64_t len) {
+    if (widen)
+      (fast ? widen_avx512 : widen_scalar)(reinterpret_cast<const float*>(from), static_cast<double*>(out) + at / 4,
+                                           len / 4);
+    else if (fast)
+      copy_avx512(from, static_cast<char*>(out) + at, len);
+    else
+      std::memcpy(static_cast<char*>(out) + at, from, len);
+  };
+  if (total < kDirectBytes) {
+    KB_CUDA(cudaMemcpyAsync(stage, src, total, cudaMemcpyDeviceToHost, s.stream));
+    KB_CUDA(cudaStreamSynchronize(s.stream));
+    emit(stage, 0, total);
+    return;
+  }
+  const unsigned hw = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+  cudaError_t err = cudaSuccess;  // no throw while the workers run
+  std::vector<std::thread> th;
+  if (total <= ring * chunk) {
+    // every piece in flight at once, each handed to whichever worker is next
+    // when it has landed
+    const uint64_t pieces = (total + kPieceBytes - 1) / kPieceBytes;
+    std::vector<cudaEvent_t> ev(pieces);
+    for (auto& e : ev) KB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    std::atomic<uint64_t> landed{0}, taken{0};
+    auto work = [&] {
+      for (uint64_t c; (c = taken.fetch_add(1)) < pieces;) {
+        while (landed.load(std::memory_order_acquire) <= c) _mm_pause();
+        emit(stage + c * kPieceBytes, c * kPieceBytes, std::min(kPieceBytes, total - c * kPieceBytes));
+      }
+    };
+    for (uint64_t c = 0; c < pieces && err == cudaSuccess; ++c) {
+      const uint64_t at = c * kPieceBytes, len = std::min(kPieceBytes, total - at);
+      err = cudaMemcpyAsync(stage + at, src + at, len, cudaMemcpyDeviceToHost, s.stream);
+      if (err == cudaSuccess) err = cudaEventRecord(ev[c], s.stream);
+    }
+    if (err == cudaSuccess) {
+      for (unsigned t = 1; t < std::min<uint64_t>(hw, pieces); ++t) th.emplace_back(work);
+      const auto w0 = std::chrono::steady_clock::now();
+      for (uint64_t c = 0; c < pieces; ++c) {
+        if (err == cudaSuccess) err = cudaEventSynchronize(ev[c]);
+        landed.store(c + 1, std::memory_order_release);
+      }
+      if (times) times->copy_wait_ms += ms_since(w0);
+      const auto s0 = std::chrono::steady_clock::now();
+      work();
+      for (auto& x : th) x.join();
+      if (times) times->widen_ms += ms_since(s0);
+    }
+    for (auto& e : ev) cudaEventDestroy(e);
+    check_cuda(err, "download");
+    return;
+  }
   std::vector<cudaEvent_t> ev(ring);
   for (auto& e : ev) KB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  const uint64_t nchunks = (count + chunk - 1) / chunk;
-  cudaError_t err = cudaSuccess;  // no throw while the workers run
+  const uint64_t nchunks = (total + chunk - 1) / chunk;
   auto issue = [&](uint64_t c) {
-    const uint64_t lo = c * chunk, len = std::min(chunk, count - lo);
-    cudaError_t e = cudaMemcpyAsync(buf[c % ring], static_cast<const float2*>(s.amps) + first + lo, len * 8,
-                                    cudaMemcpyDeviceToHost, s.stream);
+    const uint64_t lo = c * chunk, len = std::min(chunk, total - lo);
+    cudaError_t e = cudaMemcpyAsync(stage + (c % ring) * chunk, src + lo, len, cudaMemcpyDeviceToHost, s.stream);
     if (e == cudaSuccess) e = cudaEventRecord(ev[c % ring], s.stream);
     if (e != cudaSuccess && err == cudaSuccess) err = e;
   };
-  // Chunk c is widened by every worker while chunks c+1 .. c+ring-1 are in
-  // flight.  The workers start once per download and step through the
+  // Chunk c is written out by every worker while chunks c+1 .. c+ring-1 are
+  // in flight.  The workers start once per download and step through the
   // chunks between two barriers; the calling thread is worker 0 and also
   // issues the copies.
-  const unsigned nt = count < (uint64_t{1} << 20) ? 1u
-                                                  : std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-  const bool wide = have_avx512();
+  const unsigned nt = hw;
   auto slice = [&](unsigned t, uint64_t c) {
-    const uint64_t lo = c * chunk, len = std::min(chunk, count - lo);
-    // in floats, rounded to 16 floats (64 bytes of output) per worker
-    const uint64_t nf = 2 * len, per = ((nf + nt - 1) / nt + 15) / 16 * 16;
-    const uint64_t a = std::min(nf, t * per), b = std::min(nf, a + per);
-    if (b > a)
-      (wide ? widen_avx512 : widen_scalar)(reinterpret_cast<const float*>(buf[c % ring]) + a, out + 2 * lo + a, b - a);
+    const uint64_t lo = c * chunk, len = std::min(chunk, total - lo);
+    // rounded to 64 bytes per worker
+    const uint64_t per = ((len + nt - 1) / nt + 63) / 64 * 64;
+    const uint64_t a = std::min(len, t * per), b = std::min(len, a + per);
+    if (b > a) emit(stage + (c % ring) * chunk + a, lo + a, b - a);
   };
   std::barrier sync(nt);
   auto work = [&](unsigned t) {
@@ -305,7 +374,6 @@ void download(const State& s, uint64_t first, uint64_t count, double* out, Downl
       sync.arrive_and_wait();  // chunk c is consumed
     }
   };
-  std::vector<std::thread> th;
   for (unsigned t = 1; t < nt; ++t) th.emplace_back(work, t);
   for (uint64_t c = 0; c < std::min<uint64_t>(ring - 1, nchunks); ++c) issue(c);
   for (uint64_t c = 0; c < nchunks; ++c) {
@@ -383,19 +451,76 @@ void release_run_state() {
   destroy_state(s);
 }
 
+// Device states given back by destroy_state, for the next state of the same
+// size, precision and device: creating and freeing one (a stream, a
+// cudaMalloc and a cudaFree) took 0.2 to 10 ms, more than a small circuit.
+// At most kIdleBytes of them, the oldest freed first.
+constexpr uint64_t kIdleBytes = uint64_t{256} << 20;
+constexpr size_t kIdleStates = 16;
+std::mutex g_idle_mu;
+std::vector<State*> g_idle;
+
+void free_state(State* s);
+
+uint64_t state_bytes(const State& s) { return s.dim() * s.amp_bytes() + s.tree_doubles * sizeof(double); }
+
+State* take_idle_state(int n, int precision, int device) {
+  std::lock_guard<std::mutex> lk(g_idle_mu);
+  for (size_t i = g_idle.size(); i-- > 0;) {
+    State* s = g_idle[i];
+    if (s->n != n || s->precision != precision || s->device != device) continue;
+    g_idle.erase(g_idle.begin() + (std::ptrdiff_t)i);
+    return s;
+  }
+  return nullptr;
+}
+
+// Keeps an idle state (its stream's work is done); returns those to free.
+std::vector<State*> keep_idle_state(State* s) {
+  std::lock_guard<std::mutex> lk(g_idle_mu);
+  std::vector<State*> drop;
+  g_idle.push_back(s);
+  uint64_t total = 0;
+  for (const State* x : g_idle) total += state_bytes(*x);
+  while (total > kIdleBytes || g_idle.size() > kIdleStates) {
+    total -= state_bytes(*g_idle.front());
+    drop.push_back(g_idle.front());
+    g_idle.erase(g_idle.begin());
+  }
+  return drop;
+}
+
+void release_idle_states() {
+  std::vector<State*> all;
+  {
+    std::lock_guard<std::mutex> lk(g_idle_mu);
+    all.swap(g_idle);
+  }
+  for (State* s : all) free_state(s);
+}
+
 State* create_state(int n, int precision) {
   if (n < 0 || n > 40) fail(KETGPU_ERR_INVALID, "n_qubits must be in [0, 40]");
   if (precision != KETGPU_C64 && precision != KETGPU_C128)
     fail(KETGPU_ERR_INVALID, "precision must be KETGPU_C64 or KETGPU_C128");
+  int device = 0;
+  KB_CUDA(cudaGetDevice(&device));
+  if (State* idle = take_idle_state(n, precision, device)) {
+    std::unique_ptr<State, void (*)(State*)> guard_idle(idle, destroy_state);
+    idle->exposed = false;
+    set_ground(*idle);
+    return guard_idle.release();
+  }
   auto st = std::make_unique<State>();
   st->n = n;
   st->precision = precision;
-  KB_CUDA(cudaGetDevice(&st->device));
+  st->device = device;
   const size_t bytes = (size_t)st->dim() * st->amp_bytes();
   size_t free_b = 0, total_b = 0;
   KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (bytes > free_b) {  // give back ketgpu_run's kept state and the scratch pools first
+  if (bytes > free_b) {  // give back what is kept between calls first
     release_run_state();
+    release_idle_states();
     release_pools();
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   }
@@ -414,8 +539,7 @@ State* create_state(int n, int precision) {
   return guard_st.release();
 }
 
-void destroy_state(State* s) {
-  if (!s) return;
+void free_state(State* s) {
   int prev = -1;
   cudaGetDevice(&prev);
   cudaSetDevice(s->device);
@@ -425,6 +549,15 @@ void destroy_state(State* s) {
   if (s->stream) cudaStreamDestroy(s->stream);
   if (prev >= 0) cudaSetDevice(prev);
   delete s;
+}
+
+void destroy_state(State* s) {
+  if (!s) return;
+  if (s->amps && s->stream && state_bytes(*s) <= kIdleBytes && cudaStreamSynchronize(s->stream) == cudaSuccess) {
+    for (State* x : keep_idle_state(s)) free_state(x);
+    return;
+  }
+  free_state(s);
 }
 
 void execute_plan(const Plan& plan, State& s) { execute(plan, s); }
@@ -481,7 +614,7 @@ KB_API int ketgpu_state_download(const ketgpu_state* s, uint64_t first, uint64_t
     if (first > st.dim() || count > st.dim() - first)
       fail(KETGPU_ERR_OUT_OF_RANGE, "amplitude range outside the state");
     DeviceGuard g(st.device);
-    download(st, first, count, out);
+    download(st, first, count, out, st.precision == KETGPU_C64);
   });
 }
 
@@ -492,10 +625,7 @@ KB_API int ketgpu_state_download_raw(const ketgpu_state* s, uint64_t first, uint
     if (first > st.dim() || count > st.dim() - first)
       fail(KETGPU_ERR_OUT_OF_RANGE, "amplitude range outside the state");
     DeviceGuard g(st.device);
-    const size_t b = st.amp_bytes();
-    KB_CUDA(cudaMemcpyAsync(out, static_cast<const char*>(st.amps) + first * b, count * b, cudaMemcpyDeviceToHost,
-                            st.stream));
-    KB_CUDA(cudaStreamSynchronize(st.stream));
+    download(st, first, count, out, false);
   });
 }
 
@@ -621,7 +751,7 @@ KB_API int ketgpu_run(int32_t n, const ketgpu_op* ops, uint64_t n_ops, const ket
     const double exec_ms = ms_since(t2);
     const auto t3 = std::chrono::steady_clock::now();
     DownloadTimes dt;
-    download(*st, 0, st->dim(), out_c128, &dt);
+    download(*st, 0, st->dim(), out_c128, o.precision == KETGPU_C64, &dt);
     const double down_ms = ms_since(t3);
     check_tc_flag();
     const double prof[6] = {plan_ms, state_ms, exec_ms, down_ms, dt.copy_wait_ms, dt.widen_ms};
@@ -641,6 +771,7 @@ KB_API int ketgpu_run_last_profile(double* out6) {
 KB_API int ketgpu_release_cache(void) {
   return guard([&] {
     release_run_state();
+    release_idle_states();
     release_pools();
   });
 }

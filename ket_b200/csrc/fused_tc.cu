@@ -37,10 +37,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -48,8 +50,6 @@
 #include "tc_layout.cuh"
 
 namespace kb {
-
-__device__ int g_tc_error = 0;
 
 namespace {
 
@@ -118,6 +118,7 @@ struct TcGeom {
   int half;
   uint64_t top_off;
   uint32_t gbit_off[kGroupBits];
+  int* error;         // set on a timeout (mapped host memory)
   // non-null: the epilogue also sums |out|^2 in FP64 and CTA b writes its sum
   // to norm_out[b]
   double* norm_out;
@@ -425,7 +426,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       if ((it & 255) == 255 && abort_flag) return false;
     }
     abort_flag = 1;
-    atomicExch(&g_tc_error, 1);
+    *reinterpret_cast<volatile int*>(g.error) = 1;
+    __threadfence_system();
     return false;
   };
   auto arrive = [](uint64_t* bar) {
@@ -1037,11 +1039,31 @@ int encode_half_tiles(const State* st, const Pass& p, TcGeom& g, CUtensorMap* ma
   return nd;
 }
 
+// The timeout flag: mapped host memory, so that the host reads it after a
+// synchronisation without a device call (a copy from a device symbol took
+// 15 us a call).  Null until the first tensor-core launch.
+std::atomic<int*> g_error_flag{nullptr};
+std::mutex g_error_mu;
+
+int* error_flag() {
+  int* p = g_error_flag.load(std::memory_order_acquire);
+  if (p) return p;
+  std::lock_guard<std::mutex> lk(g_error_mu);
+  p = g_error_flag.load(std::memory_order_relaxed);
+  if (!p) {
+    KB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    *p = 0;
+    g_error_flag.store(p, std::memory_order_release);
+  }
+  return p;
+}
+
 template <int KQ>
 void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, uint64_t active) {
   using Cfg = TcCfg<KQ>;
   TcGeom g;
   tile_geometry<KQ>(st.n, p, active, g);
+  g.error = error_flag();
   g.norm_out = norm_partials;
   if (norm_partials)  // entries past the grid stay zero for the in-order sum
     KB_CUDA(cudaMemsetAsync(norm_partials, 0, sizeof(double) * kNormBlocks, st.stream));
@@ -1197,12 +1219,10 @@ void tc_form(int n, const Pass& p, int* tma_dims, int* direct) {
 }
 
 int tc_error_flag(bool reset) {
-  int v = 0;
-  KB_CUDA(cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)));
-  if (reset && v) {
-    const int z = 0;
-    KB_CUDA(cudaMemcpyToSymbol(g_tc_error, &z, sizeof(int)));
-  }
+  int* p = g_error_flag.load(std::memory_order_acquire);
+  if (!p) return 0;
+  const int v = *reinterpret_cast<volatile int*>(p);
+  if (reset && v) *reinterpret_cast<volatile int*>(p) = 0;
   return v;
 }
 

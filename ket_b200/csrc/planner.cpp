@@ -17,7 +17,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <exception>
+#include <functional>
 #include <numeric>
 #include <string>
 #include <thread>
@@ -161,9 +161,11 @@ Pass lower_gate(const ketgpu_op& op) {
 }
 
 double gate_traffic_fraction(const ketgpu_op& op) {
-  const Pass p = lower_gate(op);
-  if (p.kind == PassKind::Phase) return std::ldexp(1.0, -p.nfixed);
-  return std::ldexp(1.0, 1 - p.nfixed);
+  switch (op.type) {  // the gates lower_gate makes phase passes
+    case KETGPU_Z: case KETGPU_S: case KETGPU_SDG: case KETGPU_T: case KETGPU_TDG: return 0.5;
+    case KETGPU_CZ: case KETGPU_CP: return 0.25;
+    default: return std::ldexp(1.0, 1 - gate_arity(op.type));
+  }
 }
 
 namespace {
@@ -281,88 +283,83 @@ bool block_on_tensor_cores(int n, int k, const PlanOptions& opt) {
 // that can be moved to the front of what is left (no earlier non-diagonal
 // gate shares a qubit with it) is collected; if that run spans more qubits
 // than one block holds, it becomes a single Diagonal pass.
-std::vector<Block> grow_blocks(int n, const ketgpu_op* ops, const std::vector<int>& order, int max_k,
-                               bool diag_runs) {
-  std::vector<Block> blocks;
-  std::vector<char> done(order.size(), 0);
-  size_t first = 0;
-  std::vector<char> blocked(n, 0), inq(n, 0);
+// A partition in flat arrays: the planner grows many and keeps one.
+struct Partition {
+  std::vector<int> gates;        // op indices, block after block
+  std::vector<size_t> end;       // where each block ends in them
+  std::vector<uint64_t> qubits;  // masks
+  std::vector<char> diag;
+  void close(uint64_t q, bool d) {
+    end.push_back(gates.size());
+    qubits.push_back(q);
+    diag.push_back(d);
+  }
+};
+
+Partition grow_blocks(int n, const ketgpu_op* ops, const std::vector<int>& order, int max_k, bool diag_runs) {
+  const size_t G = order.size();
+  Partition part;
+  part.gates.reserve(G);
+  // gates left, a linked list in order; qubit sets as masks
+  std::vector<uint64_t> mask(G);
+  std::vector<char> diag(G);
+  std::vector<size_t> next(G + 1);
+  for (size_t i = 0; i < G; ++i) {
+    mask[i] = qubit_mask(ops[order[i]]);
+    diag[i] = is_diagonal_gate(ops[order[i]].type);
+  }
+  std::iota(next.begin(), next.end(), size_t{0});  // next[j]: the gate after position j - 1
+  size_t& first = next[0];
   const uint64_t all = n >= 64 ? ~uint64_t{0} : ((uint64_t{1} << n) - 1);
-  while (true) {
-    while (first < order.size() && done[first]) ++first;
-    if (first == order.size()) break;
-    if (diag_runs && is_diagonal_gate(ops[order[first]].type)) {
-      std::vector<size_t> run;
+  std::vector<size_t> run;
+  while (first < G) {
+    if (diag_runs && diag[first]) {
+      run.clear();
       uint64_t blk = 0, span = 0;
-      for (size_t i = first; i < order.size() && blk != all; ++i) {
-        if (done[i]) continue;
-        const ketgpu_op& o = ops[order[i]];
-        const uint64_t m = qubit_mask(o);
-        if (is_diagonal_gate(o.type) && !(m & blk)) {
+      for (size_t i = first; i < G && blk != all; i = next[i + 1]) {
+        if (diag[i] && !(mask[i] & blk)) {
           run.push_back(i);
-          span |= m;
+          span |= mask[i];
         } else {
-          blk |= m;
+          blk |= mask[i];
         }
       }
       if (run.size() >= 2 && __builtin_popcountll(span) > max_k) {
-        Block b;
-        b.diag = true;
-        for (size_t i : run) {
-          done[i] = 1;
-          b.gates.push_back(order[i]);
+        size_t r = 0;
+        for (size_t prev = 0; r < run.size();) {
+          const size_t i = next[prev];
+          if (i == run[r]) {
+            part.gates.push_back(order[i]);
+            next[prev] = next[i + 1];
+            ++r;
+          } else {
+            prev = i + 1;
+          }
         }
-        for (int q = 0; q < n; ++q)
-          if ((span >> q) & 1) b.qubits.push_back(q);
-        blocks.push_back(std::move(b));
+        part.close(span, true);
         continue;
       }
     }
-    Block b;
-    std::fill(blocked.begin(), blocked.end(), 0);
-    std::fill(inq.begin(), inq.end(), 0);
-    int nq = 0, nblocked = 0;
-    for (size_t i = first; i < order.size(); ++i) {
-      if (done[i]) continue;
-      const ketgpu_op& o = ops[order[i]];
-      const int a = gate_arity(o.type);
-      bool hit = false;
-      int add = 0;
-      for (int j = 0; j < a; ++j) {
-        if (blocked[o.q[j]]) hit = true;
-        if (!inq[o.q[j]]) ++add;
-      }
-      if (b.gates.empty() || (!hit && nq + add <= max_k)) {
-        for (int j = 0; j < a; ++j)
-          if (!inq[o.q[j]]) {
-            inq[o.q[j]] = 1;
-            ++nq;
-          }
-        b.gates.push_back((int)i);
-        done[i] = 1;
+    uint64_t blocked = 0, inq = 0;
+    const size_t start = part.gates.size();
+    for (size_t prev = 0, i; (i = next[prev]) < G;) {
+      const uint64_t m = mask[i];
+      if (part.gates.size() == start || (!(m & blocked) && __builtin_popcountll(inq | m) <= max_k)) {
+        inq |= m;
+        part.gates.push_back(order[i]);
+        next[prev] = next[i + 1];
       } else {
-        for (int j = 0; j < a; ++j)
-          if (!blocked[o.q[j]]) {
-            blocked[o.q[j]] = 1;
-            ++nblocked;
-          }
-        if (nblocked == n) break;
+        blocked |= m;
+        if (blocked == all) break;
         // nothing more can join once every block qubit is blocked and the
         // block is full
-        if (nq == max_k) {
-          bool open = false;
-          for (int q = 0; q < n; ++q)
-            if (inq[q] && !blocked[q]) open = true;
-          if (!open) break;
-        }
+        if (__builtin_popcountll(inq) == max_k && !(inq & ~blocked)) break;
+        prev = i + 1;
       }
     }
-    for (int q = 0; q < n; ++q)
-      if (inq[q]) b.qubits.push_back(q);
-    for (int& gi : b.gates) gi = order[gi];
-    blocks.push_back(std::move(b));
+    part.close(inq, false);
   }
-  return blocks;
+  return part;
 }
 
 // Topological orders of a segment's gates for the greedy block growth.  The
@@ -372,47 +369,73 @@ std::vector<Block> grow_blocks(int n, const ketgpu_op* ops, const std::vector<in
 // levels of the circuit before moving on: light-cone-shaped blocks.  On the
 // 30-qubit, 40-layer brick wall at k = 5 the best band order needs 119
 // passes against 154 in program order.  Returns op indices.
-std::vector<int> band_order(const ketgpu_op* ops, const std::vector<int>& seg, int n, int w, int off) {
+struct Dependencies {  // of a segment's gates
+  std::vector<int> depth, lowest, indegree;  // ASAP depth, lowest qubit, direct predecessors
+  std::vector<int> succ_at, succ;            // successors of gate i: succ[succ_at[i] .. succ_at[i + 1])
+};
+
+Dependencies dependencies(const ketgpu_op* ops, const std::vector<int>& seg, int n) {
   const size_t G = seg.size();
-  std::vector<int> depth(G, 0), indeg(G, 0), qmin(G, 0), last(n, -1);
-  std::vector<std::vector<int>> succ(G);
+  Dependencies d;
+  d.depth.assign(G, 0);
+  d.lowest.assign(G, 0);
+  d.indegree.assign(G, 0);
+  d.succ_at.assign(G + 1, 0);
+  std::vector<int> last(n, -1), from, to;
   for (size_t i = 0; i < G; ++i) {
     const ketgpu_op& o = ops[seg[i]];
-    int d = 0, lo = n;
+    int dep = 0, lo = n;
     for (int j = 0; j < gate_arity(o.type); ++j) {
       const int q = o.q[j];
       lo = std::min(lo, q);
       if (last[q] >= 0) {
-        d = std::max(d, depth[last[q]] + 1);
-        succ[last[q]].push_back((int)i);
-        ++indeg[i];
+        dep = std::max(dep, d.depth[last[q]] + 1);
+        from.push_back(last[q]);
+        to.push_back((int)i);
+        ++d.succ_at[last[q] + 1];
+        ++d.indegree[i];
       }
       last[q] = (int)i;
     }
-    depth[i] = d;
-    qmin[i] = lo;
+    d.depth[i] = dep;
+    d.lowest[i] = lo;
   }
-  auto later = [&](int a, int b) {  // heap order: the smallest key first
-    const int ba = (depth[a] + off) / w, bb = (depth[b] + off) / w;
-    if (ba != bb) return ba > bb;
-    if (qmin[a] != qmin[b]) return qmin[a] > qmin[b];
-    if (depth[a] != depth[b]) return depth[a] > depth[b];
-    return a > b;
+  std::partial_sum(d.succ_at.begin(), d.succ_at.end(), d.succ_at.begin());
+  d.succ.resize(from.size());
+  std::vector<int> at(d.succ_at.begin(), d.succ_at.end() - 1);
+  for (size_t e = 0; e < from.size(); ++e) d.succ[at[from[e]]++] = to[e];
+  return d;
+}
+
+std::vector<int> band_order(const std::vector<int>& seg, const Dependencies& d, int w, int off) {
+  const size_t G = seg.size();
+  // (band, lowest qubit, depth, gate), smallest first
+  struct Key {
+    uint64_t hi;
+    uint32_t depth;
+    int gate;
+    bool operator>(const Key& o) const {
+      return hi != o.hi ? hi > o.hi : depth != o.depth ? depth > o.depth : gate > o.gate;
+    }
   };
-  std::vector<int> heap, out;
+  std::vector<int> indeg = d.indegree, out;
+  std::vector<Key> heap;
   out.reserve(G);
+  auto key = [&](int i) {
+    return Key{((uint64_t)((d.depth[i] + off) / w) << 8) | (uint64_t)d.lowest[i], (uint32_t)d.depth[i], i};
+  };
   for (size_t i = 0; i < G; ++i)
-    if (!indeg[i]) heap.push_back((int)i);
-  std::make_heap(heap.begin(), heap.end(), later);
+    if (!indeg[i]) heap.push_back(key((int)i));
+  std::make_heap(heap.begin(), heap.end(), std::greater<Key>());
   while (!heap.empty()) {
-    std::pop_heap(heap.begin(), heap.end(), later);
-    const int i = heap.back();
+    std::pop_heap(heap.begin(), heap.end(), std::greater<Key>());
+    const int i = heap.back().gate;
     heap.pop_back();
     out.push_back(seg[i]);
-    for (int sidx : succ[i])
-      if (--indeg[sidx] == 0) {
-        heap.push_back(sidx);
-        std::push_heap(heap.begin(), heap.end(), later);
+    for (int e = d.succ_at[i]; e < d.succ_at[i + 1]; ++e)
+      if (--indeg[d.succ[e]] == 0) {
+        heap.push_back(key(d.succ[e]));
+        std::push_heap(heap.begin(), heap.end(), std::greater<Key>());
       }
   }
   return out;
@@ -424,21 +447,23 @@ constexpr int kBandWidths[] = {3, 4, 5, 6, 7, 8};
 
 // Static cost of a partition in full-state passes: each block fused or as
 // its separate gates, whichever is cheaper; a diagonal run is one pass.
-double partition_cost(const ketgpu_op* ops, const std::vector<Block>& blocks, const PlanOptions& opt) {
+double partition_cost(const std::vector<double>& fraction, const Partition& part, const PlanOptions& opt) {
   double total = 0;
-  for (const Block& b : blocks) {
-    if (b.diag) {
-      total += 1.0;
-      continue;
-    }
+  size_t g = 0;
+  for (size_t b = 0; b < part.end.size(); ++b) {
+    const size_t count = part.end[b] - g;
     double separate = 0;
-    for (int gi : b.gates) separate += gate_traffic_fraction(ops[gi]);
-    total += b.gates.size() > 1 ? std::min(separate, fused_cost_static((int)b.qubits.size(), opt.precision,
-                                                                         opt.tensor))
-                                : separate;
+    for (; g < part.end[b]; ++g) separate += fraction[part.gates[g]];
+    if (part.diag[b]) total += 1.0;
+    else
+      total += count > 1 ? std::min(separate, fused_cost_static(__builtin_popcountll(part.qubits[b]), opt.precision,
+                                                                 opt.tensor))
+                         : separate;
   }
   return total;
 }
+
+int gate_last(const std::vector<int>& seg) { return seg.empty() ? -1 : *std::max_element(seg.begin(), seg.end()); }
 
 // Greedy growth over the program order and every band order (width,
 // offset); the partition with the least static cost, the earliest candidate
@@ -449,12 +474,15 @@ std::vector<Block> best_partition(int n, const ketgpu_op* ops, const std::vector
   for (int w : kBandWidths)
     for (int off = 0; off < w; ++off) cands.push_back({w, off});
   const size_t C = cands.size();
-  std::vector<std::vector<Block>> parts(C);
+  std::vector<Partition> parts(C);
   std::vector<double> cost(C, 0.0);
+  const Dependencies deps = dependencies(ops, seg, n);
+  std::vector<double> fraction(gate_last(seg) + 1, 0.0);  // by op index
+  for (int gi : seg) fraction[gi] = gate_traffic_fraction(ops[gi]);
   auto work = [&](size_t c) {
-    const std::vector<int> order = cands[c].first ? band_order(ops, seg, n, cands[c].first, cands[c].second) : seg;
-    parts[c] = grow_blocks(n, ops, order, std::max(1, opt.max_k), true);
-    cost[c] = partition_cost(ops, parts[c], opt);
+    parts[c] = grow_blocks(n, ops, cands[c].first ? band_order(seg, deps, cands[c].first, cands[c].second) : seg,
+                           std::max(1, opt.max_k), true);
+    cost[c] = partition_cost(fraction, parts[c], opt);
   };
   const unsigned nt = seg.size() < 256 ? 1u : std::min<unsigned>(16u, std::max(1u, std::thread::hardware_concurrency()));
   if (nt <= 1) {
@@ -471,7 +499,15 @@ std::vector<Block> best_partition(int n, const ketgpu_op* ops, const std::vector
   size_t best = 0;
   for (size_t c = 1; c < C; ++c)
     if (cost[c] < cost[best] - 1e-9) best = c;
-  return std::move(parts[best]);
+  const Partition& p = parts[best];
+  std::vector<Block> blocks(p.end.size());
+  for (size_t b = 0, g = 0; b < blocks.size(); g = p.end[b++]) {
+    blocks[b].gates.assign(p.gates.begin() + (std::ptrdiff_t)g, p.gates.begin() + (std::ptrdiff_t)p.end[b]);
+    for (int q = 0; q < n; ++q)
+      if ((p.qubits[b] >> q) & 1) blocks[b].qubits.push_back(q);
+    blocks[b].diag = p.diag[b];
+  }
+  return blocks;
 }
 
 // ket's Fuser block rule on one barrier-free segment.

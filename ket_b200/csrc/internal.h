@@ -78,6 +78,9 @@ struct State {
   mutable double* tree = nullptr;
   mutable uint64_t tree_doubles = 0;
   mutable uint64_t tree_version = ~uint64_t{0};
+  // A second stream, above the first in priority, for work that does not need
+  // the amplitudes (the draws of sample_tree_seeded); made on demand.
+  mutable cudaStream_t side = nullptr;
   // version right after set_ground: while version still equals it, the state
   // is |0...0> and its squared norm is exactly 1
   mutable uint64_t ground_version = ~uint64_t{0};
@@ -292,6 +295,11 @@ void expval_terms(const State& s, const std::vector<uint64_t>& flip,
 // Born-rule draws for host uniforms; builds the state's sampling tree only
 // when the amplitudes changed since the last build (State::version).
 void sample_tree(const State& s, const double* u, uint64_t count, uint64_t* out);
+// The same for the draws of std::mt19937{seed}.
+void sample_tree_seeded(const State& s, uint32_t seed, uint64_t count, uint64_t* out);
+// Copy device memory to a host buffer, ordered on and waiting for `stream`
+// (abi.cpp; large copies go through pinned staging).
+void fetch_bytes(const void* src, uint64_t bytes, void* out, cudaStream_t stream);
 // Number of sampling-tree builds since load (all states).
 uint64_t sample_tree_builds();
 

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <random>
 #include <type_traits>
 #include <cstring>
 #include <vector>
@@ -169,15 +170,39 @@ __global__ void __launch_bounds__(kSegThreads)
   for (uint64_t wseg = (uint64_t)blockIdx.x * (kSegThreads / 32) + warp; wseg * 32 < n_dst;
        wseg += warps_total) {
     const uint64_t base = wseg * 32 * kSeg;
-#pragma unroll 4
-    for (int r = 0; r < 32; ++r) {
-      const uint64_t i = base + (uint64_t)r * 32 + lane;
-      double v = 0;
-      if (i < n_src) {
-        if constexpr (LEAF) v = prob(src[i]);
-        else v = reinterpret_cast<const double*>(src)[i];
+    if (base + 32 * kSeg <= n_src) {
+      // 16-byte loads, eight in flight a lane (one 8-byte load at a time, four
+      // in flight: 463 us for 28 qubits, complex64; now 396)
+      constexpr int PER = 16 / (int)sizeof(T);  // values a load
+      struct alignas(16) Vec {
+        T v[PER];
+      };
+      const Vec* p = reinterpret_cast<const Vec*>(src + base) + lane;
+#pragma unroll
+      for (int h = 0; h < 32 / PER; h += 8) {
+        Vec x[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) x[r] = p[(h + r) * 32];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int e = ((h + r) * 32 + lane) * PER;
+#pragma unroll
+          for (int q = 0; q < PER; ++q) {
+            if constexpr (LEAF) sh[warp][e >> 5][(e & 31) + q] = prob(x[r].v[q]);
+            else sh[warp][e >> 5][(e & 31) + q] = x[r].v[q];
+          }
+        }
       }
-      sh[warp][r][lane] = v;
+    } else {
+      for (int r = 0; r < 32; ++r) {
+        const uint64_t i = base + (uint64_t)r * 32 + lane;
+        double v = 0;
+        if (i < n_src) {
+          if constexpr (LEAF) v = prob(src[i]);
+          else v = src[i];
+        }
+        sh[warp][r][lane] = v;
+      }
     }
     __syncwarp();
     const uint64_t j = wseg * 32 + lane;
@@ -239,12 +264,77 @@ struct Levels {
   uint64_t off[24];  // offset (in doubles) of level l >= 1 in the buffer
 };
 
-template <typename T>
+// The uniform of two successive words of std::mt19937, as libstdc++'s
+// uniform_real_distribution<double>(0, 1) forms it (its generate_canonical:
+// lo + hi * 2^32 in double, over 2^64, below 1).
+__device__ __forceinline__ double canonical(uint2 w) {
+  const double r = __dadd_rn((double)w.x, (double)w.y * 4294967296.0) * 5.42101086242752217e-20;
+  return r < 1.0 ? r : __longlong_as_double(0x3fefffffffffffffll);
+}
+__device__ __forceinline__ double canonical(double u) { return u; }
+
+// std::mt19937's output words, by one CTA.  With f the twist of two words,
+//     x[k] = x[k - 227] ^ f(x[k - 624], x[k - 623])
+// gives 227 words at a time; put into itself once,
+//     x[k] = x[k - 454] ^ f(x[k - 851], x[k - 850]) ^ f(x[k - 624], x[k - 623])
+// gives 454, from a ring of 2048 words in shared memory.  A step's output is
+// tempered and stored during the next step's loads.
+// Bound: a barrier and a shared-memory round trip a step, 4405 steps for 10^6
+// draws (0.78 ms; 1.03 with 227-word steps and the tempering in line, 5.2 on the
+// host); it runs beside the passes that read the state.
+struct MtState {
+  uint32_t x[624];
+};
+constexpr int kMtThreads = 480, kMtStep = 454;
+
+__device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b) {
+  const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+  return (y >> 1) ^ (b & 1 ? 0x9908b0dfu : 0u);
+}
+__device__ __forceinline__ uint32_t mt_temper(uint32_t v) {
+  v ^= v >> 11;
+  v ^= (v << 7) & 0x9d2c5680u;
+  v ^= (v << 15) & 0xefc60000u;
+  return v ^ (v >> 18);
+}
+
+__global__ void __launch_bounds__(kMtThreads)
+    mt19937_words(const __grid_constant__ MtState init, uint32_t words, uint32_t* __restrict__ out) {
+  __shared__ uint32_t ring[2048];
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < 624; i += kMtThreads) ring[i] = init.x[i];
+  __syncthreads();
+  if (tid < 227) {  // words 0..226, x[624 .. 850]
+    const uint32_t v = ring[tid + 397] ^ mt_twist(ring[tid], ring[tid + 1]);
+    ring[tid + 624] = v;
+    if (tid < words) out[tid] = mt_temper(v);
+  }
+  __syncthreads();
+  uint32_t last = 0, at = 0xffffffffu;  // the previous step's word and its place
+  for (uint32_t w0 = 227; w0 < words; w0 += kMtStep) {
+    const uint32_t k = w0 + 624 + tid;
+    uint32_t v = 0;
+    if (tid < kMtStep) {
+      const uint32_t a = ring[(k - 851) & 2047], b = ring[(k - 850) & 2047], c = ring[(k - 624) & 2047],
+                     d = ring[(k - 623) & 2047];
+      v = ring[(k - 454) & 2047];
+      if (at < words) out[at] = mt_temper(last);
+      v ^= mt_twist(a, b) ^ mt_twist(c, d);
+      ring[k & 2047] = v;
+      last = v;
+      at = w0 + tid;
+    }
+    __syncthreads();
+  }
+  if (at < words) out[at] = mt_temper(last);
+}
+
+template <typename T, typename U>
 __global__ void sample_kernel(const T* __restrict__ s, const double* __restrict__ buf, Levels lv,
-                              const double* __restrict__ u, uint64_t count, uint64_t* __restrict__ out) {
+                              const U* __restrict__ u, uint64_t count, uint64_t* __restrict__ out) {
   const uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= count) return;
-  const double x = u[d];
+  const double x = canonical(u[d]);
   double carry = 0;
   uint64_t lo = 0, hi = lv.size[lv.L];
   for (int l = lv.L; l >= 1; --l) {
@@ -263,11 +353,30 @@ __global__ void sample_kernel(const T* __restrict__ s, const double* __restrict_
   }
   uint64_t pick = hi - 1;
   double c = carry;
-  for (uint64_t i = lo; i < hi; ++i) {
-    c = __dadd_rn(c, prob(s[i]));
-    if (x < c) {
-      pick = i;
-      break;
+  if (hi - lo == (uint64_t)kSeg) {
+    // eight amplitudes' loads in flight, then their sums in order (one
+    // dependent load at a time: 296 us for 10^6 draws at 28 qubits, now about 200)
+    bool found = false;
+    for (uint64_t i = lo; i < hi && !found; i += 8) {
+      T a[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = s[i + j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        c = __dadd_rn(c, prob(a[j]));
+        if (!found && x < c) {
+          pick = i + j;
+          found = true;
+        }
+      }
+    }
+  } else {
+    for (uint64_t i = lo; i < hi; ++i) {
+      c = __dadd_rn(c, prob(s[i]));
+      if (x < c) {
+        pick = i;
+        break;
+      }
     }
   }
   out[d] = pick;
@@ -453,32 +562,35 @@ std::atomic<uint64_t> g_tree_builds{0};
 
 uint64_t sample_tree_builds() { return g_tree_builds.load(); }
 
-void sample_tree(const State& st, const double* u, uint64_t count, uint64_t* out) {
+namespace {
+
+Levels tree_levels(const State& st, uint64_t* total) {
   Levels lv{};
   lv.size[0] = st.dim();
-  lv.L = 0;
-  uint64_t total = 0;
+  *total = 0;
   while (lv.size[lv.L] > (uint64_t)kSeg) {
     lv.size[lv.L + 1] = (lv.size[lv.L] + kSeg - 1) / kSeg;
     ++lv.L;
-    lv.off[lv.L] = total;
-    total += lv.size[lv.L];
+    lv.off[lv.L] = *total;
+    *total += lv.size[lv.L];
   }
+  return lv;
+}
+
+// The state's tree, built on its stream if the amplitudes changed.
+Levels build_tree(const State& st) {
+  uint64_t total = 0;
+  const Levels lv = tree_levels(st, &total);
   // The tree lives with the state (1/31 of a complex128 state's size, 1/15
   // of a complex64 one) and is rebuilt only after the amplitudes changed.
   if (total && !st.tree) {
     KB_CUDA(cudaMalloc(&st.tree, sizeof(double) * total));
     st.tree_doubles = total;
   }
-  const size_t ubytes = sizeof(double) * count, obytes = sizeof(uint64_t) * count;
-  StreamScratch sc(ubytes + obytes + 64, st.device, st.stream);
+  if (!total || st.tree_version == st.version) return lv;
   double* buf = st.tree;
-  double* d_u = static_cast<double*>(sc.p);
-  uint64_t* d_out = reinterpret_cast<uint64_t*>(d_u + count);
-  KB_CUDA(cudaMemcpyAsync(d_u, u, ubytes, cudaMemcpyHostToDevice, st.stream));
-  const bool build = total && st.tree_version != st.version;
-  if (build) g_tree_builds.fetch_add(1);
-  for (int l = 1; build && l <= lv.L; ++l) {
+  g_tree_builds.fetch_add(1);
+  for (int l = 1; l <= lv.L; ++l) {
     const uint64_t nd = lv.size[l];
     const int blocks = grid_for(nd, kSegThreads);  // one warp -> 32 outputs
     if (l == 1) {
@@ -494,30 +606,86 @@ void sample_tree(const State& st, const double* u, uint64_t count, uint64_t* out
     }
     count_launch();
   }
-  if (build) {
-    top_fold<<<1, 1, 0, st.stream>>>(buf + lv.off[lv.L], lv.size[lv.L]);
-    count_launch();
-    for (int l = lv.L - 1; l >= 1; --l) {
-      const int blocks = grid_for(lv.size[l + 1], kSegThreads);
-      down_fold<<<blocks, kSegThreads, 0, st.stream>>>(buf + lv.off[l], lv.size[l], buf + lv.off[l + 1],
-                                                     lv.size[l + 1]);
-      count_launch();
-    }
-  }
-  const int blocks = (int)((count + kRThreads - 1) / kRThreads);
-  if (count) {
-    if (st.precision == KETGPU_C64)
-      sample_kernel<float2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), buf, lv,
-                                                                 d_u, count, d_out);
-    else
-      sample_kernel<double2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), buf, lv,
-                                                                  d_u, count, d_out);
+  top_fold<<<1, 1, 0, st.stream>>>(buf + lv.off[lv.L], lv.size[lv.L]);
+  count_launch();
+  for (int l = lv.L - 1; l >= 1; --l) {
+    const int blocks = grid_for(lv.size[l + 1], kSegThreads);
+    down_fold<<<blocks, kSegThreads, 0, st.stream>>>(buf + lv.off[l], lv.size[l], buf + lv.off[l + 1],
+                                                   lv.size[l + 1]);
     count_launch();
   }
   KB_CUDA(cudaGetLastError());
-  if (build) st.tree_version = st.version;
-  KB_CUDA(cudaMemcpyAsync(out, d_out, obytes, cudaMemcpyDeviceToHost, st.stream));
-  KB_CUDA(cudaStreamSynchronize(st.stream));
+  st.tree_version = st.version;
+  return lv;
+}
+
+template <typename U>
+void draw(const State& st, const Levels& lv, const U* d_u, uint64_t count, uint64_t* d_out, uint64_t* out) {
+  const unsigned blocks = (unsigned)((count + kRThreads - 1) / kRThreads);
+  if (st.precision == KETGPU_C64)
+    sample_kernel<<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), st.tree, lv, d_u, count,
+                                                       d_out);
+  else
+    sample_kernel<<<blocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), st.tree, lv, d_u, count,
+                                                       d_out);
+  count_launch();
+  KB_CUDA(cudaGetLastError());
+  fetch_bytes(d_out, sizeof(uint64_t) * count, out, st.stream);
+}
+
+// Draws from which the uniforms are made on the device.  A call of 8192 draws
+// at 12 qubits takes 79 us with them made on the device and 120 on the host;
+// one of 1000 takes 61 us on the host.
+constexpr uint64_t kDeviceDraws = 2048;
+constexpr uint64_t kMostDeviceDraws = uint64_t{1} << 30;  // 32-bit word indices
+
+}  // namespace
+
+void sample_tree(const State& st, const double* u, uint64_t count, uint64_t* out) {
+  const Levels lv = build_tree(st);
+  if (!count) {
+    KB_CUDA(cudaStreamSynchronize(st.stream));
+    return;
+  }
+  StreamScratch sc((sizeof(double) + sizeof(uint64_t)) * count, st.device, st.stream);
+  double* d_u = static_cast<double*>(sc.p);
+  KB_CUDA(cudaMemcpyAsync(d_u, u, sizeof(double) * count, cudaMemcpyHostToDevice, st.stream));
+  draw(st, lv, d_u, count, reinterpret_cast<uint64_t*>(d_u + count), out);
+}
+
+void sample_tree_seeded(const State& st, uint32_t seed, uint64_t count, uint64_t* out) {
+  if (count < kDeviceDraws || count > kMostDeviceDraws) {
+    std::vector<double> u(count);
+    std::mt19937 rng{seed};
+    std::uniform_real_distribution<double> dist(0.0, 1.0);
+    for (double& v : u) v = dist(rng);
+    sample_tree(st, u.data(), count, out);
+    return;
+  }
+  if (!st.side) {
+    int least = 0, greatest = 0;
+    KB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    KB_CUDA(cudaStreamCreateWithPriority(&st.side, cudaStreamNonBlocking, greatest));
+  }
+  // the words on the second stream, beside whatever the first one still does
+  // to the amplitudes and the tree's building
+  StreamScratch words(sizeof(uint2) * count, st.device, st.side);
+  MtState mt;
+  mt.x[0] = seed;
+  for (uint32_t i = 1; i < 624; ++i) mt.x[i] = 1812433253u * (mt.x[i - 1] ^ (mt.x[i - 1] >> 30)) + i;
+  mt19937_words<<<1, kMtThreads, 0, st.side>>>(mt, (uint32_t)(2 * count), static_cast<uint32_t*>(words.p));
+  count_launch();
+  KB_CUDA(cudaGetLastError());
+  const Levels lv = build_tree(st);
+  cudaEvent_t made;
+  KB_CUDA(cudaEventCreateWithFlags(&made, cudaEventDisableTiming));
+  cudaError_t e = cudaEventRecord(made, st.side);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st.stream, made, 0);
+  cudaEventDestroy(made);
+  check_cuda(e, "sample_tree_seeded");
+  StreamScratch sc(sizeof(uint64_t) * count, st.device, st.stream);
+  uint64_t* d_out = static_cast<uint64_t*>(sc.p);
+  draw(st, lv, static_cast<const uint2*>(words.p), count, d_out, out);
 }
 
 }  // namespace kb

@@ -207,7 +207,8 @@ int ketgpu_run(int32_t n_qubits, const ketgpu_op* ops, uint64_t n_ops,
  * ket (its run, simulator.cpp:554-558, has no phases to report). */
 int ketgpu_run_last_profile(double* out6);
 /* Free what the library keeps between calls on the device: the state of
- * ketgpu_run, destroyed states for reuse (at most 256 MB) and scratch
+ * ketgpu_run, destroyed states for reuse (at most 256 MB), the states of
+ * ketgpu_adjoint (at most 4 GB) and scratch
  * memory (at most 64 MB a device) (no-op when
  * there is none).  No counterpart in ket, whose run holds no device memory. */
 int ketgpu_release_cache(void);

@@ -93,6 +93,91 @@ void release_pools() {
     if (pool) cudaMemPoolTrimTo(pool, 0);
 }
 
+namespace {
+constexpr size_t kIdleStreams = 8;
+std::mutex g_stream_mu;
+std::vector<std::pair<int, cudaStream_t>> g_streams;  // (device, idle stream)
+}  // namespace
+
+StreamLease::StreamLease(int dev) : device(dev) {
+  {
+    std::lock_guard<std::mutex> lk(g_stream_mu);
+    for (size_t i = 0; i < g_streams.size() && !s; ++i)
+      if (g_streams[i].first == dev) {
+        s = g_streams[i].second;
+        g_streams.erase(g_streams.begin() + (std::ptrdiff_t)i);
+      }
+  }
+  if (!s) KB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+}
+
+StreamLease::~StreamLease() {
+  if (!s) return;
+  if (cudaStreamSynchronize(s) == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_stream_mu);
+    if (g_streams.size() < kIdleStreams) {
+      g_streams.emplace_back(device, s);
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+}
+
+namespace {
+struct KeptWorkspace {
+  void* p = nullptr;
+  size_t bytes = 0;
+  int device = -1;
+};
+std::mutex g_work_mu;
+KeptWorkspace g_work;
+
+void free_on(int device, void* p) {
+  if (!p) return;
+  int prev = -1;
+  cudaGetDevice(&prev);
+  cudaSetDevice(device);
+  cudaFree(p);
+  if (prev >= 0) cudaSetDevice(prev);
+}
+}  // namespace
+
+void release_workspaces() {
+  KeptWorkspace w;
+  {
+    std::lock_guard<std::mutex> lk(g_work_mu);
+    std::swap(w, g_work);
+  }
+  free_on(w.device, w.p);
+}
+
+Workspace::Workspace(size_t b, int dev) : bytes(b), device(dev) {
+  KeptWorkspace w;
+  {
+    std::lock_guard<std::mutex> lk(g_work_mu);
+    std::swap(w, g_work);
+  }
+  if (w.p && w.device == dev && w.bytes >= bytes) {
+    p = w.p;
+    bytes = w.bytes;
+    return;
+  }
+  free_on(w.device, w.p);
+  KB_CUDA(cudaMalloc(&p, bytes ? bytes : 8));
+}
+
+Workspace::~Workspace() {
+  if (!p) return;
+  if (bytes <= kWorkspaceKeep) {
+    std::lock_guard<std::mutex> lk(g_work_mu);
+    if (!g_work.p) {
+      g_work = {p, bytes, device};
+      return;
+    }
+  }
+  free_on(device, p);
+}
+
 DeviceBlock::DeviceBlock(size_t bytes, int device, cudaStream_t stream) {
   cudaMemPool_t pool = scratch_pool(device);
   if (pool) KB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream));
@@ -530,6 +615,7 @@ State* create_state(int n, int precision) {
   if (bytes > free_b) {  // give back what is kept between calls first
     release_run_state();
     release_idle_states();
+    release_workspaces();
     release_pools();
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   }
@@ -785,6 +871,7 @@ KB_API int ketgpu_release_cache(void) {
   return guard([&] {
     release_run_state();
     release_idle_states();
+    release_workspaces();
     release_pools();
   });
 }

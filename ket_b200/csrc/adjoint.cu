@@ -327,6 +327,86 @@ __global__ void __launch_bounds__(kAThreads)
   }
 }
 
+// Matrices of the circuit's gates for every parameter set, [gate][set][8].
+// A gate without a parameter has the same one for all sets (made on the host);
+// a parameterised one is formed here from its set's angle, with ket's
+// formulas.  The host loop over gates and sets, and the copy of its result,
+// were most of a small call.
+struct AdjGate {
+  double m[8];   // kind 0: the matrix
+  int32_t kind;  // 0 fixed, 1 Rx, 2 Ry, 3 Rz (or their controlled forms), 4 CP
+  int32_t pslot;
+};
+
+template <typename R>
+__global__ void gate_matrices(const AdjGate* __restrict__ gates, int ngates, const double* __restrict__ params,
+                              uint64_t nparams, uint64_t nsets, uint64_t stride, int diag_phase,
+                              R* __restrict__ out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (uint64_t)ngates * nsets) return;
+  const uint64_t gi = i / nsets, set = i % nsets;
+  const AdjGate& g = gates[gi];
+  double m[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) m[j] = g.m[j];
+  if (g.kind) {
+    const double t = params[set * nparams + g.pslot];
+    double s, c;
+    sincos(g.kind == 4 ? t : t / 2.0, &s, &c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[j] = 0.0;
+    if (g.kind == 1) {
+      m[0] = m[6] = c;
+      m[3] = m[5] = -s;
+    } else if (g.kind == 2) {
+      m[0] = m[6] = c;
+      m[2] = -s;
+      m[4] = s;
+    } else if (g.kind == 3) {
+      m[0] = m[6] = c;
+      m[1] = -s;
+      m[7] = s;
+    } else if (diag_phase) {  // the tiled sweeps take a phase as diag(1, phase)
+      m[0] = 1.0;
+      m[6] = c;
+      m[7] = s;
+    } else {
+      m[0] = c;
+      m[1] = s;
+    }
+  }
+  R* o = out + (gi * stride + set) * 8;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) o[j] = (R)m[j];
+}
+
+// One warp a result: the sum of its partials, scaled, over its pieces (gates
+// that share a parameter).  Fixed order: lane-strided per piece, then a tree.
+struct AdjPiece {
+  uint64_t at;      // first partial of set 0
+  uint64_t stride;  // from set to set
+  double scale;
+};
+
+__global__ void sum_partials(const double* __restrict__ part, const AdjPiece* __restrict__ pieces,
+                             const int32_t* __restrict__ first /* [nresults + 1] */, int nresults, uint64_t nsets,
+                             int count, double* __restrict__ out) {
+  const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= (uint64_t)nresults * nsets) return;
+  const int lane = threadIdx.x & 31;
+  const uint64_t set = w / nresults, r = w % nresults;
+  double v = 0.0;
+  for (int k = first[r]; k < first[r + 1]; ++k) {
+    const double* p = part + pieces[k].at + set * pieces[k].stride;
+    double a = 0.0;
+    for (int i = lane; i < count; i += 32) a += p[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    v += pieces[k].scale * a;
+  }
+  if (lane == 0) out[set * nresults + r] = v;
+}
+
 template <typename R>
 __global__ void ground_batch(typename C2T<R>::T* states, uint64_t dim) {
   typename C2T<R>::T one;
@@ -1192,12 +1272,9 @@ TilePlan plan_tiles_best(int n, const ketgpu_op* ops, const std::vector<int>& ga
   return per_seg.blocks.size() < per_layer.blocks.size() ? std::move(per_seg) : std::move(per_layer);
 }
 
-struct DevBuf {
-  void* p = nullptr;
-  explicit DevBuf(size_t b) { KB_CUDA(cudaMalloc(&p, b ? b : 8)); }
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
+// A call's device memory, from the library's pool, freed in stream order.
+struct DevBuf : StreamScratch {
+  using StreamScratch::StreamScratch;
   template <typename T>
   T* as() const {
     return static_cast<T*>(p);
@@ -1521,30 +1598,39 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   const int n_ckpt = (n_layers + m - 1) / m;  // segment starts at layers 0, m, 2m, ...
   const size_t G = gate_ops.size();
 
-  // memory: chunk of the batch that fits in ~60% of free memory
-  size_t free_b = 0, total_b = 0;
-  KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  // memory: chunk of the batch that fits in ~60% of free memory (not asked
+  // for when the states take little)
   const size_t per_set = dim * sizeof(T) * (2 + (size_t)n_ckpt);
-  if ((uint64_t)((free_b * 0.6) / per_set) < batch) {  // first take back ketgpu_run's kept state
-    release_run_state();
+  uint64_t chunk = batch;
+  if (batch && per_set > kPoolKeep / batch) {
+    size_t free_b = 0, total_b = 0;
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if ((uint64_t)((free_b * 0.6) / per_set) < batch) {  // first take back what is kept between calls
+      release_run_state();
+      release_idle_states();
+      release_workspaces();
+      release_pools();
+      KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    }
+    chunk = std::max<uint64_t>(1, (uint64_t)((free_b * 0.6) / per_set));
   }
-  uint64_t chunk = std::max<uint64_t>(1, (uint64_t)((free_b * 0.6) / per_set));
   chunk = std::min<uint64_t>(chunk, batch);
   chunk = std::min<uint64_t>(chunk, 65535);
 
-  cudaStream_t st;
-  KB_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  struct StreamGuard {
-    cudaStream_t s;
-    ~StreamGuard() { cudaStreamDestroy(s); }
-  } sg{st};
-
-  DevBuf psi(dim * sizeof(T) * chunk), lam(dim * sizeof(T) * chunk);
-  DevBuf ck(dim * sizeof(T) * chunk * (size_t)n_ckpt);
+  int dev = 0;
+  KB_CUDA(cudaGetDevice(&dev));
+  // psi, lambda and the checkpoints of every set of the chunk (ends after the
+  // lease, which waits for the stream)
+  Workspace work(per_set * chunk, dev);
+  StreamLease lease(dev);
+  const cudaStream_t st = lease.s;
+  T* const psi = static_cast<T*>(work.p);
+  T* const lam = psi + dim * chunk;
+  T* const ck = lam + dim * chunk;
   const int blocks = (int)std::min<uint64_t>(std::max<uint64_t>(1, (dim / 2 + kAThreads - 1) / kAThreads), 592);
-  DevBuf mats(sizeof(double) * 8 * chunk * std::max<size_t>(G, 1));
-  DevBuf hmeta(sizeof(uint64_t) * 2 * T_ + sizeof(int) * T_ + sizeof(double) * T_ + 64);
+  // the gates' matrices in the precision their sweep reads
+  DevBuf mats((tiled ? sizeof(R) : sizeof(double)) * 8 * chunk * std::max<size_t>(G, 1), dev, st);
+  DevBuf hmeta(sizeof(uint64_t) * 2 * T_ + sizeof(int) * T_ + sizeof(double) * T_ + 64, dev, st);
   {
     std::vector<char> h(sizeof(uint64_t) * 2 * T_ + sizeof(int) * T_ + sizeof(double) * T_);
     std::memcpy(h.data(), flip.data(), 8 * T_);
@@ -1576,7 +1662,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
         ht.push_back(x);
         if (pass == 0) ++ham_group0;
       }
-    d_ham = std::make_unique<DevBuf>(sizeof(HamTerm) * std::max(T_, 1));
+    d_ham = std::make_unique<DevBuf>(sizeof(HamTerm) * std::max(T_, 1), dev, st);
     KB_CUDA(cudaMemcpyAsync(d_ham->p, ht.data(), sizeof(HamTerm) * T_, cudaMemcpyHostToDevice, st));
     static bool ham_attr[2] = {false, false};
     if (!ham_attr[sizeof(R) == 8]) {
@@ -1611,23 +1697,38 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     if (pi >= (int32_t)nparams) fail(KETGPU_ERR_OUT_OF_RANGE, "adjoint: parameter index out of range");
   }
 
-  // per-set 2x2 of gate gi (U, row-major, FP64 interleaved).  The tiled
-  // sweep stores a phase gate as diag(1, phase).
-  auto gate_matrix = [&](size_t gi, uint64_t set, double* d) {
-    ketgpu_op oo = ops[gate_ops[gi]];
-    if (geo[gi].pslot >= 0) oo.p[0] = params[set * nparams + geo[gi].pslot];
-    const Pass p = lower_gate(oo);
+  // the gates as gate_matrices takes them: 2x2 U, row-major, FP64
+  // interleaved; the tiled sweep stores a phase gate as diag(1, phase)
+  std::vector<AdjGate> agates(G);
+  std::vector<uint8_t> real(G, 0);  // the matrix is real for every set
+  for (size_t gi = 0; gi < G; ++gi) {
+    const ketgpu_op& o = ops[gate_ops[gi]];
+    AdjGate& a = agates[gi];
+    a = AdjGate{};
+    a.pslot = geo[gi].pslot;
+    if (a.pslot >= 0) {
+      a.kind = geo[gi].gen;  // 1 X, 2 Y, 3 Z, 4 P11
+      real[gi] = a.kind == 2;
+      continue;
+    }
+    const Pass p = lower_gate(o);
     cplx mm[4] = {p.m[0], p.m[1], p.m[2], p.m[3]};
     if (tiled && p.kind == PassKind::Phase) {
       mm[3] = p.m[0];
       mm[0] = cplx(1.0, 0.0);
       mm[1] = mm[2] = cplx(0.0, 0.0);
     }
+    bool r = true;
     for (int j = 0; j < 4; ++j) {
-      d[2 * j] = mm[j].real();
-      d[2 * j + 1] = mm[j].imag();
+      a.m[2 * j] = mm[j].real();
+      a.m[2 * j + 1] = mm[j].imag();
+      r = r && mm[j].imag() == 0.0;
     }
-  };
+    real[gi] = r;
+  }
+  DevBuf d_agates(sizeof(AdjGate) * std::max<size_t>(G, 1), dev, st);
+  if (G) KB_CUDA(cudaMemcpyAsync(d_agates.p, agates.data(), sizeof(AdjGate) * G, cudaMemcpyHostToDevice, st));
+  DevBuf d_params(sizeof(double) * std::max<uint64_t>(chunk * nparams, 1), dev, st);
 
   // tiled plan
   TilePlan tp;
@@ -1636,17 +1737,9 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   int gx = 1;
   size_t grad_doubles = 0;
   if (tiled) {
-    std::vector<uint8_t> real(G, 1);
-    double d[8];
-    for (size_t gi = 0; gi < G; ++gi)
-      for (uint64_t b = 0; b < batch && real[gi]; ++b) {
-        gate_matrix(gi, b, d);
-        if (d[1] != 0.0 || d[3] != 0.0 || d[5] != 0.0 || d[7] != 0.0) real[gi] = 0;
-        if (geo[gi].pslot < 0) break;  // the same matrix for every set
-      }
     tp = plan_tiles_best<R>(n, ops, gate_ops, layer_of, geo, real, m);
-    d_tgates = std::make_unique<DevBuf>(sizeof(TGate) * std::max<size_t>(tp.gates.size(), 1));
-    d_tphases = std::make_unique<DevBuf>(sizeof(TPhase) * std::max<size_t>(tp.phases.size(), 1));
+    d_tgates = std::make_unique<DevBuf>(sizeof(TGate) * std::max<size_t>(tp.gates.size(), 1), dev, st);
+    d_tphases = std::make_unique<DevBuf>(sizeof(TPhase) * std::max<size_t>(tp.phases.size(), 1), dev, st);
     if (!tp.gates.empty())
       KB_CUDA(cudaMemcpyAsync(d_tgates->p, tp.gates.data(), sizeof(TGate) * tp.gates.size(),
                               cudaMemcpyHostToDevice, st));
@@ -1679,8 +1772,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     // sets, in whole rounds where the set count allows: a grid of 10 x 64
     // CTAs on 296 slots ran two full rounds and a third of 48 CTAs, leaving
     // most SMs idle for a third of each sweep.
-    int sms = 148, dev = 0;
-    KB_CUDA(cudaGetDevice(&dev));
+    int sms = 148;
     KB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint64_t slots = 2ull * (uint64_t)sms;
     gx = (int)std::min<uint64_t>(n_tiles, std::max<uint64_t>(1, (8 * slots + chunk / 2) / chunk));
@@ -1706,22 +1798,61 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   // gradient partials (tiled: per block; per-gate: [gate][set][block]), then
   // the expectation partials
   const size_t grad_region = tiled ? grad_doubles : (size_t)G * chunk * blocks;
-  DevBuf part(sizeof(double) * (grad_region + ham_doubles));
+  DevBuf part(sizeof(double) * (grad_region + ham_doubles), dev, st);
   double* d_ham_part = part.as<double>() + grad_region;
 
-  std::vector<double> hmats(8 * chunk * std::max<size_t>(G, 1));
-  std::vector<R> hmats_t(tiled ? hmats.size() : 0);  // the tiled sweeps read them in the state's precision
-  DevBuf mats_t(sizeof(R) * std::max<size_t>(hmats_t.size(), 1));
-  std::vector<double> hpart;
+  // The pieces of every parameter's gradient, then those of the expectation.
+  // (A gate's partials: [gate][set][CTA] tiled within its block, per gate
+  // [gate][set][CTA].)
+  const int per_grad = tiled ? gx : blocks, per_value = ham_split ? 2 * ham_ctas : blocks;
+  std::vector<AdjPiece> pieces;
+  std::vector<int32_t> first(nparams + 3, 0);
+  {
+    std::vector<std::vector<AdjPiece>> by_param(nparams);
+    auto add = [&](size_t gi, uint64_t at, uint64_t stride) {
+      by_param[geo[gi].pslot].push_back({at, stride, geo[gi].gen == 4 ? -2.0 : 1.0});
+    };
+    if (tiled) {
+      for (const TBlock& blk : tp.blocks) {
+        const size_t ng = blk.grad_gate.size();
+        for (size_t k = 0; k < ng; ++k)
+          add((size_t)blk.grad_gate[k], blk.part_off + k * (size_t)gx, (uint64_t)ng * gx);
+      }
+    } else {
+      for (size_t gi = 0; gi < G; ++gi)
+        if (geo[gi].pslot >= 0) add(gi, (uint64_t)gi * chunk * blocks, (uint64_t)blocks);
+    }
+    for (uint64_t k = 0; k < nparams; ++k) {
+      pieces.insert(pieces.end(), by_param[k].begin(), by_param[k].end());
+      first[k + 1] = (int32_t)pieces.size();
+    }
+    // the expectation, as a one-result list of its own
+    first[nparams + 1] = (int32_t)pieces.size();
+    pieces.push_back({(uint64_t)grad_region, (uint64_t)per_value, 1.0});
+    first[nparams + 2] = (int32_t)pieces.size();
+  }
+  DevBuf d_pieces(sizeof(AdjPiece) * pieces.size() + sizeof(int32_t) * first.size(), dev, st);
+  const AdjPiece* dp = d_pieces.as<AdjPiece>();
+  const int32_t* df = reinterpret_cast<const int32_t*>(dp + pieces.size());
+  KB_CUDA(cudaMemcpyAsync(d_pieces.p, pieces.data(), sizeof(AdjPiece) * pieces.size(), cudaMemcpyHostToDevice, st));
+  KB_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(df), first.data(), sizeof(int32_t) * first.size(),
+                          cudaMemcpyHostToDevice, st));
+  DevBuf d_result(sizeof(double) * chunk * (nparams + 1), dev, st);
+  std::vector<double> hresult;
   for (uint64_t b0 = 0; b0 < batch; b0 += chunk) {
     const uint64_t nb = std::min(chunk, batch - b0);
-    for (size_t gi = 0; gi < G; ++gi)
-      for (uint64_t b = 0; b < nb; ++b) gate_matrix(gi, b0 + b, &hmats[(gi * chunk + b) * 8]);
-    KB_CUDA(cudaMemcpyAsync(mats.p, hmats.data(), sizeof(double) * 8 * chunk * std::max<size_t>(G, 1),
-                            cudaMemcpyHostToDevice, st));
-    if (tiled) {
-      for (size_t i = 0; i < hmats.size(); ++i) hmats_t[i] = (R)hmats[i];
-      KB_CUDA(cudaMemcpyAsync(mats_t.p, hmats_t.data(), sizeof(R) * hmats_t.size(), cudaMemcpyHostToDevice, st));
+    if (nparams)
+      KB_CUDA(cudaMemcpyAsync(d_params.p, params + b0 * nparams, sizeof(double) * nb * nparams,
+                              cudaMemcpyHostToDevice, st));
+    if (G) {
+      const unsigned mb = (unsigned)((G * nb + 127) / 128);
+      if (tiled)
+        gate_matrices<R><<<mb, 128, 0, st>>>(d_agates.as<AdjGate>(), (int)G, d_params.as<double>(), nparams, nb,
+                                             chunk, 1, mats.as<R>());
+      else
+        gate_matrices<double><<<mb, 128, 0, st>>>(d_agates.as<AdjGate>(), (int)G, d_params.as<double>(), nparams, nb,
+                                                  chunk, 0, mats.as<double>());
+      count_launch();
     }
     // With every block compiled, checkpoints cost no copies: the block
     // before a checkpoint writes its tiles into the checkpoint, the next
@@ -1729,16 +1860,16 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     // the first block of a segment reads psi from its checkpoint).
     bool ck_direct = tiled && !jit_fwd.empty();
     for (size_t bi = 0; ck_direct && bi < jit_fwd.size(); ++bi) ck_direct = jit_fwd[bi] && jit_rev[bi];
-    auto ck_at = [&](int k) { return ck.as<T>() + (size_t)k * chunk * dim; };
+    auto ck_at = [&](int k) { return ck + (size_t)k * chunk * dim; };
     // forward
-    T* ground = ck_direct ? ck_at(0) : psi.as<T>();
+    T* ground = ck_direct ? ck_at(0) : psi;
     KB_CUDA(cudaMemsetAsync(ground, 0, dim * sizeof(T) * nb, st));
     ground_batch<R><<<(unsigned)nb, 1, 0, st>>>(ground, dim);
     count_launch();
     // checkpoint k = the state at the start of layer k*m
     int next_ck = 0;
     auto store_ck = [&]() {
-      KB_CUDA(cudaMemcpyAsync(ck.as<T>() + (size_t)next_ck * chunk * dim, psi.p, dim * sizeof(T) * nb,
+      KB_CUDA(cudaMemcpyAsync(ck + (size_t)next_ck * chunk * dim, psi, dim * sizeof(T) * nb,
                               cudaMemcpyDeviceToDevice, st));
       ++next_ck;
     };
@@ -1748,34 +1879,34 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
       next_ck = 1;            // checkpoint 0 is the ground state
       for (int bi = 0; bi < B; ++bi) {
         const TBlock& b = tp.blocks[bi];
-        if (cur != psi.as<T>() && next_ck < n_ckpt && next_ck * m <= b.layer) {
+        if (cur != psi && next_ck < n_ckpt && next_ck * m <= b.layer) {
           // more checkpoints due here than blocks between them
-          KB_CUDA(cudaMemcpyAsync(psi.p, cur, dim * sizeof(T) * nb, cudaMemcpyDeviceToDevice, st));
-          cur = psi.as<T>();
+          KB_CUDA(cudaMemcpyAsync(psi, cur, dim * sizeof(T) * nb, cudaMemcpyDeviceToDevice, st));
+          cur = psi;
         }
-        while (cur == psi.as<T>() && next_ck < n_ckpt && next_ck * m <= b.layer) store_ck();
-        T* out = psi.as<T>();
+        while (cur == psi && next_ck < n_ckpt && next_ck * m <= b.layer) store_ck();
+        T* out = psi;
         if (bi + 1 < B && next_ck < n_ckpt && next_ck * m <= tp.blocks[bi + 1].layer) out = ck_at(next_ck++);
         dim3 grid((unsigned)gx, (unsigned)nb);
         launch_tile<R, false>(grid, st, out, nullptr, dim, b, d_tgates->as<TGate>(), d_tphases->as<TPhase>(),
-                              mats_t.as<R>(), chunk, nullptr, jit_fwd[bi], cur);
+                              mats.as<R>(), chunk, nullptr, jit_fwd[bi], cur);
         cur = out;
       }
-      if (cur != psi.as<T>())
-        KB_CUDA(cudaMemcpyAsync(psi.p, cur, dim * sizeof(T) * nb, cudaMemcpyDeviceToDevice, st));
+      if (cur != psi)
+        KB_CUDA(cudaMemcpyAsync(psi, cur, dim * sizeof(T) * nb, cudaMemcpyDeviceToDevice, st));
     } else if (tiled) {
       for (const TBlock& b : tp.blocks) {
         while (next_ck < n_ckpt && next_ck * m <= b.layer) store_ck();
         dim3 grid((unsigned)gx, (unsigned)nb);
-        launch_tile<R, false>(grid, st, psi.as<T>(), nullptr, dim, b, d_tgates->as<TGate>(), d_tphases->as<TPhase>(),
-                              mats_t.as<R>(), chunk, nullptr,
+        launch_tile<R, false>(grid, st, psi, nullptr, dim, b, d_tgates->as<TGate>(), d_tphases->as<TPhase>(),
+                              mats.as<R>(), chunk, nullptr,
                               jit_fwd.empty() ? nullptr : jit_fwd[&b - tp.blocks.data()]);
       }
     } else {
       for (size_t gi = 0; gi < G; ++gi) {
         while (next_ck < n_ckpt && next_ck * m <= layer_of[gi]) store_ck();
         dim3 grid((unsigned)blocks, (unsigned)nb);
-        fwd_gate<R><<<grid, kAThreads, 0, st>>>(psi.as<T>(), dim, geo[gi], mats.as<double>() + gi * chunk * 8);
+        fwd_gate<R><<<grid, kAThreads, 0, st>>>(psi, dim, geo[gi], mats.as<double>() + gi * chunk * 8);
         count_launch();
       }
     }
@@ -1790,18 +1921,18 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
         for (int h = 0; h < 2; ++h) {
           if (g0 > 0) {
             ham_half<R><<<hgrid, kAThreads, sizeof(HamTerm) * g0, st>>>(
-                psi.as<T>(), lam.as<T>(), dim, h, 1, g1 == 0 ? 1 : 0, d_ham->as<HamTerm>(), g0, d_ham_part);
+                psi, lam, dim, h, 1, g1 == 0 ? 1 : 0, d_ham->as<HamTerm>(), g0, d_ham_part);
             count_launch();
           }
           if (g1 > 0) {
             ham_half<R><<<hgrid, kAThreads, sizeof(HamTerm) * g1, st>>>(
-                psi.as<T>(), lam.as<T>(), dim, h, g0 == 0 ? 1 : 0, 1, d_ham->as<HamTerm>() + g0, g1, d_ham_part);
+                psi, lam, dim, h, g0 == 0 ? 1 : 0, 1, d_ham->as<HamTerm>() + g0, g1, d_ham_part);
             count_launch();
           }
         }
       } else {
         dim3 grid((unsigned)blocks, (unsigned)nb);
-        ham_apply<R><<<grid, kAThreads, 0, st>>>(psi.as<T>(), lam.as<T>(), dim, d_flip, d_sign, d_q, d_coef, T_,
+        ham_apply<R><<<grid, kAThreads, 0, st>>>(psi, lam, dim, d_flip, d_sign, d_q, d_coef, T_,
                                                  d_ham_part);
         count_launch();
       }
@@ -1813,67 +1944,49 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
       for (int bi = B; bi-- > 0;) {
         const TBlock& b = tp.blocks[bi];
         const int seg = b.layer / m;
-        const T* src = psi.as<T>();
+        const T* src = psi;
         if (bi + 1 < B && tp.blocks[bi + 1].layer / m != seg && seg + 1 < n_ckpt) {
           if (ck_direct) src = ck_at(seg + 1);
           else
-            KB_CUDA(cudaMemcpyAsync(psi.p, ck.as<T>() + (size_t)(seg + 1) * chunk * dim, dim * sizeof(T) * nb,
+            KB_CUDA(cudaMemcpyAsync(psi, ck + (size_t)(seg + 1) * chunk * dim, dim * sizeof(T) * nb,
                                     cudaMemcpyDeviceToDevice, st));
         }
         dim3 grid((unsigned)gx, (unsigned)nb);
-        launch_tile<R, true>(grid, st, psi.as<T>(), lam.as<T>(), dim, b, d_tgates->as<TGate>(),
-                             d_tphases->as<TPhase>(), mats_t.as<R>(), chunk, part.as<double>() + b.part_off,
+        launch_tile<R, true>(grid, st, psi, lam, dim, b, d_tgates->as<TGate>(),
+                             d_tphases->as<TPhase>(), mats.as<R>(), chunk, part.as<double>() + b.part_off,
                              jit_rev.empty() ? nullptr : jit_rev[bi], src);
       }
     } else {
       for (size_t gi = G; gi-- > 0;) {
         const int seg = layer_of[gi] / m;
         if (gi + 1 < G && layer_of[gi + 1] / m != seg && seg + 1 < n_ckpt) {
-          KB_CUDA(cudaMemcpyAsync(psi.p, ck.as<T>() + (size_t)(seg + 1) * chunk * dim, dim * sizeof(T) * nb,
+          KB_CUDA(cudaMemcpyAsync(psi, ck + (size_t)(seg + 1) * chunk * dim, dim * sizeof(T) * nb,
                                   cudaMemcpyDeviceToDevice, st));
         }
         dim3 grid((unsigned)blocks, (unsigned)nb);
-        rev_gate<R><<<grid, kAThreads, 0, st>>>(psi.as<T>(), lam.as<T>(), dim, geo[gi],
+        rev_gate<R><<<grid, kAThreads, 0, st>>>(psi, lam, dim, geo[gi],
                                                 mats.as<double>() + gi * chunk * 8,
                                                 part.as<double>() + gi * chunk * blocks);
         count_launch();
       }
     }
     KB_CUDA(cudaGetLastError());
-    const size_t part_count = grad_region + ham_doubles;
-    hpart.resize(part_count);
-    KB_CUDA(cudaMemcpyAsync(hpart.data(), part.p, sizeof(double) * part_count, cudaMemcpyDeviceToHost, st));
+    auto sums = [&](const int32_t* list, int nresults, int count, double* out) {
+      const uint64_t warps = (uint64_t)nresults * nb;
+      sum_partials<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(part.as<double>(), dp, list, nresults, nb, count, out);
+      count_launch();
+    };
+    double* d_values = d_result.as<double>() + chunk * nparams;
+    if (nparams) sums(df, (int)nparams, per_grad, d_result.as<double>());
+    sums(df + nparams + 1, 1, per_value, d_values);
+    KB_CUDA(cudaGetLastError());
+    hresult.resize(nb * (nparams + 1));
+    if (nparams)
+      KB_CUDA(cudaMemcpyAsync(hresult.data(), d_result.p, sizeof(double) * nb * nparams, cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaMemcpyAsync(hresult.data() + nb * nparams, d_values, sizeof(double) * nb, cudaMemcpyDeviceToHost, st));
     KB_CUDA(cudaStreamSynchronize(st));
-    const double* hham = hpart.data() + grad_region;
-    for (uint64_t b = 0; b < nb; ++b) {
-      double v = 0;
-      const int per_set = ham_split ? 2 * ham_ctas : blocks;
-      const double* pv = hham + b * per_set;
-      for (int k = 0; k < per_set; ++k) v += pv[k];
-      values[b0 + b] = v;
-      double* gr = grads + (b0 + b) * nparams;
-      for (uint64_t k = 0; k < nparams; ++k) gr[k] = 0.0;
-      if (tiled) {
-        for (const TBlock& blk : tp.blocks) {
-          const size_t ng = blk.grad_gate.size();
-          for (size_t k = 0; k < ng; ++k) {
-            const size_t gi = (size_t)blk.grad_gate[k];
-            const double* pg = &hpart[blk.part_off + (b * ng + k) * gx];
-            double acc = 0;
-            for (int c = 0; c < gx; ++c) acc += pg[c];
-            gr[geo[gi].pslot] += (geo[gi].gen == 4) ? -2.0 * acc : acc;
-          }
-        }
-      } else {
-        for (size_t gi = 0; gi < G; ++gi) {
-          if (geo[gi].pslot < 0) continue;
-          double acc = 0;
-          const double* pg = &hpart[gi * chunk * blocks + b * blocks];
-          for (int k = 0; k < blocks; ++k) acc += pg[k];
-          gr[geo[gi].pslot] += (geo[gi].gen == 4) ? -2.0 * acc : acc;
-        }
-      }
-    }
+    std::copy(hresult.begin(), hresult.begin() + (std::ptrdiff_t)(nb * nparams), grads + b0 * nparams);
+    std::copy(hresult.begin() + (std::ptrdiff_t)(nb * nparams), hresult.end(), values + b0);
   }
 }
 

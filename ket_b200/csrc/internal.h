@@ -282,6 +282,33 @@ void norm_from_partials(const State& s, const double* partials, double* out);
 void noalloc_prepare(int device);
 // Free the device state that ketgpu_run keeps between calls (if any).
 void release_run_state();
+// Free the destroyed states kept for reuse.
+void release_idle_states();
+// Device memory for one call that may be large: the last call's is kept for
+// the next when it is at most kWorkspaceKeep (allocating and freeing 400 MB
+// took half of a call; the stream-ordered pool maps 50 GB far more slowly
+// than cudaMalloc).  The owner's work on it is done when it ends.
+constexpr uint64_t kWorkspaceKeep = uint64_t{4} << 30;
+struct Workspace {
+  void* p = nullptr;
+  size_t bytes;
+  int device;
+  Workspace(size_t bytes, int dev);
+  ~Workspace();
+  Workspace(const Workspace&) = delete;
+  Workspace& operator=(const Workspace&) = delete;
+};
+void release_workspaces();
+// A non-blocking stream for one call, from a few kept per device (making and
+// destroying one costs about 50 us).
+struct StreamLease {
+  cudaStream_t s = nullptr;
+  int device;
+  explicit StreamLease(int dev);
+  ~StreamLease();  // waits for the stream's work
+  StreamLease(const StreamLease&) = delete;
+  StreamLease& operator=(const StreamLease&) = delete;
+};
 // The first dim amplitudes *= sqrt(target[0] / current[0]), factor read on the
 // device.
 void rescale_state(const State& s, uint64_t dim, const double* target, const double* current);

@@ -60,13 +60,39 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 template <typename T>
 __global__ void norm_partial(const T* __restrict__ s, uint64_t dim, double* __restrict__ part) {
   __shared__ double sh[32];
-  double acc = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const T v = s[i];
-    const double x = AmpT<T>::re(v), y = AmpT<T>::im(v);
-    acc += x * x + y * y;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // 16-byte loads, eight in flight, a sum each (one 8-byte load at a time:
+  // 77 us for 24 qubits, complex64)
+  constexpr int PER = 16 / (int)sizeof(T);
+  struct alignas(16) Vec {
+    T v[PER];
+  };
+  const Vec* p = reinterpret_cast<const Vec*>(s);
+  const uint64_t nv = dim / PER;
+  double a[8] = {};
+  auto square = [](const Vec& v) {
+    double r = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const double x = AmpT<T>::re(v.v[q]), y = AmpT<T>::im(v.v[q]);
+      r += x * x + y * y;
+    }
+    return r;
+  };
+  for (; i + 7 * stride < nv; i += 8 * stride) {
+    Vec v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = p[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a[u] += square(v[u]);
   }
+  for (; i < nv; i += stride) a[0] += square(p[i]);
+  if (PER > 1 && (dim & 1) && blockIdx.x == 0 && threadIdx.x == 0) {  // a 1-amplitude state
+    const double x = AmpT<T>::re(s[dim - 1]), y = AmpT<T>::im(s[dim - 1]);
+    a[1] += x * x + y * y;
+  }
+  const double acc = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
   const double r = block_sum(acc, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = r;
 }

@@ -373,6 +373,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  // The next pass may be launched: its CTAs take the SMs as this one's leave
+  // and set up before they wait for the whole of it (below).
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     for (int i = 0; i < SB; ++i) {
       mbar_init(smem_u32(&bar_full[i]), g.tma_dims ? 1 : kProducers + 1);
@@ -404,6 +407,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the state is the previous pass's from here
 
   const uint64_t first = blockIdx.x;
   const uint64_t stride = gridDim.x;
@@ -1100,14 +1104,19 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   uint64_t grid = (uint64_t)sms[st.device];
   if (grid > g.n_tiles) grid = g.n_tiles;
   if (norm_partials && grid > (uint64_t)kNormBlocks) fail(KETGPU_ERR_LOGIC, "tensor-core norm partials");
-  if (norm_partials)
-    fused_tc_kernel<KQ, true><<<(unsigned)grid, kTcThreads, Cfg::SMEM, st.stream>>>(
-        static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image), tmap);
-  else
-    fused_tc_kernel<KQ, false><<<(unsigned)grid, kTcThreads, Cfg::SMEM, st.stream>>>(
-        static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image), tmap);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = Cfg::SMEM;
+  cfg.stream = st.stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  KB_CUDA(cudaLaunchKernelEx(&cfg, norm_partials ? fused_tc_kernel<KQ, true> : fused_tc_kernel<KQ, false>,
+                             static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image), tmap));
   count_launch();
-  KB_CUDA(cudaGetLastError());
 }
 
 // IEEE binary16 bits of v, rounded to nearest, ties to even (host only), by

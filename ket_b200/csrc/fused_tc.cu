@@ -875,56 +875,41 @@ int sm_count_tc(int device) {
   return v;
 }
 
-// Shared-memory wavefronts of the worst converter read of a tensor-copy tile
-// (host only): lane l of converter warp q reads, for each combination c, the
-// 8-byte amplitude of group 32q + l at its natural tile offset under the
-// 128-byte swizzle.  A warp's 32 reads need at least 2 wavefronts; more
-// means lanes whose groups lie 1 KB or more apart share banks.
-int tma_read_wavefronts(const TcGeom& g, int tb, int dim) {
-  int worst = 0;
-  for (int q = 0; q < 4; ++q)
-    for (int c = 0; c < dim; ++c) {
-      uint32_t ctile = 0;
-      for (int b = 0, jb = 0; jb < tb; ++jb)
-        if (g.is_target[jb]) {
-          if ((c >> b) & 1) ctile |= 8u << jb;
-          ++b;
-        }
-      uint32_t words[32][2];
-      for (int l = 0; l < 32; ++l) {
-        const int lane_row = 32 * q + l;
-        uint32_t gtile = 0;
-        for (int jb = 0, gb = 0; jb < tb; ++jb)
-          if (!g.is_target[jb]) {
-            if ((lane_row >> gb) & 1) gtile |= 8u << jb;
-            ++gb;
+// Shared-memory wavefronts of a converter read of a tensor-copy tile (host
+// only): lane l of a converter warp reads, for each combination, the 8-byte
+// amplitude of group 32q + l at its natural tile offset under the 128-byte
+// swizzle.  Addresses are XOR-linear in the group, and XOR with the
+// combination's and the warp's offset permutes the 16 pairs of banks, so
+// every read of every warp falls on 2^rank of them alike, rank that of the
+// five lane bits' offsets in the address bits 3..6.  A warp's 32 reads need
+// at least 2 wavefronts; more means lanes whose groups lie 1 KB or more apart
+// share banks.  (Counting the banks of every read took 130 us a launch.)
+int tma_read_wavefronts(const TcGeom& g, int tb) {
+  uint32_t basis[4] = {0, 0, 0, 0};
+  int rank = 0;
+  for (int jb = 0, gb = 0; jb < tb && gb < 5; ++jb)
+    if (!g.is_target[jb]) {
+      const uint32_t off = 8u << jb;
+      uint32_t v = ((off ^ ((off >> 3) & 0x70u)) >> 3) & 15u;
+      for (int i = 3; i >= 0 && v; --i)
+        if ((v >> i) & 1) {
+          if (!basis[i]) {
+            basis[i] = v;
+            ++rank;
+            break;
           }
-        const uint32_t off = ctile | gtile;
-        const uint32_t addr = off ^ ((off >> 3) & 0x70u);
-        words[l][0] = addr >> 2;
-        words[l][1] = (addr >> 2) + 1;
-      }
-      for (int bank = 0; bank < 32; ++bank) {
-        uint32_t seen[64];
-        int ns = 0;
-        for (int l = 0; l < 32; ++l)
-          for (int w = 0; w < 2; ++w)
-            if ((words[l][w] & 31u) == (uint32_t)bank) {
-              bool dup = false;
-              for (int i = 0; i < ns; ++i) dup |= seen[i] == words[l][w];
-              if (!dup) seen[ns++] = words[l][w];
-            }
-        worst = ns > worst ? ns : worst;
-      }
+          v ^= basis[i];
+        }
+      ++gb;
     }
-  return worst;
+  return 32 >> rank;
 }
 
 // Whether a block takes the tensor-copy producer (before the tile-run limits).
 bool tma_wanted(const TcGeom& g, const Pass& p, int tb) {
   const int lowest = p.qubits[0];
   if (lowest >= tc_tma_min()) return true;
-  return lowest == 1 && tc_tma_min() <= 2 && tma_read_wavefronts(g, tb, 1 << p.k) <= 2;
+  return lowest == 1 && tc_tma_min() <= 2 && tma_read_wavefronts(g, tb) <= 2;
 }
 
 // Tile layout of a block on an n-qubit state (host only): the tile qubits,

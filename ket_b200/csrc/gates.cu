@@ -607,6 +607,11 @@ void set_ground(const State& s) {
   KB_CUDA(cudaGetLastError());
 }
 
+// The check of a state whose address was handed out costs a call 12 us and
+// more; below this size a pass on the whole state is no slower than one on
+// part of it (20 qubits, complex128, 16 MB: 556 -> 510 us with the check).
+constexpr uint64_t kGroundCheckBytes = uint64_t{8} << 20;
+
 PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false) {
   const uint64_t all = s.dim() - 1;
   if (plan.finite && s.version == s.active_version && s.active != all) {
@@ -616,7 +621,7 @@ PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), a
       if (!s.exposed) {
         active_ = s.active;
         keep_ = true;
-      } else if (s.version == s.ground_version && is_ground(s)) {
+      } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version && is_ground(s)) {
         active_ = 0;
       }
     }

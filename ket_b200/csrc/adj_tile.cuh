@@ -45,7 +45,8 @@ struct TGate {
   uint8_t tbit;    // kTDiag: tile bit of the target
   uint8_t cm_r;    // controls held in registers, as a register-index mask
   uint8_t gen;     // gradient generator: 0 none, 1 X, 2 Y, 3 Z, 4 P11
-  uint8_t real;    // kTPair: the matrix is real for every parameter set
+  uint8_t real;    // kTPair: the matrix is real for every parameter set;
+                   // kTDiag: the entry of target bit 0 is 1
   uint16_t cm_g;   // controls not held in registers, as a tile-bit mask
   int16_t grad;    // gradient slot within the block, or -1
   int32_t mat;     // gate index into the per-set matrix table
@@ -253,6 +254,7 @@ __device__ __forceinline__ float pk_diag(PackState& a, PackState& l, const TGate
         minus1 = fma2(l.i[jo], a.r[jo], minus1);
       }
     }
+    if (TS > 0 && g.real && !bit) continue;  // times 1
     pk_phase(a.r[jo], a.i[jo], pr, pi, npi);
     if (REV) pk_phase(l.r[jo], l.i[jo], pr, pi, npi);
   }

@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(kAThreads)
 // were most of a small call.
 struct AdjGate {
   double m[8];   // kind 0: the matrix
-  int32_t kind;  // 0 fixed, 1 Rx, 2 Ry, 3 Rz (or their controlled forms), 4 CP
+  int32_t kind;  // 0 fixed, 1 Rx, 2 Ry, 3 Rz (or their controlled forms), 4 CP,
+                 // 5 Rz without its global phase: diag(1, e^{it})
   int32_t pslot;
 };
 
@@ -352,7 +353,7 @@ __global__ void gate_matrices(const AdjGate* __restrict__ gates, int ngates, con
   if (g.kind) {
     const double t = params[set * nparams + g.pslot];
     double s, c;
-    sincos(g.kind == 4 ? t : t / 2.0, &s, &c);
+    sincos(g.kind >= 4 ? t : t / 2.0, &s, &c);
 #pragma unroll
     for (int j = 0; j < 8; ++j) m[j] = 0.0;
     if (g.kind == 1) {
@@ -578,6 +579,7 @@ __device__ __forceinline__ R tile_diag_reg(typename C2T<R>::T* p, typename C2T<R
         if (gen == 3) part += bit ? -im : im;
         else if (bit) part += im;  // P11
       }
+      if (!bit && g.real) continue;  // times 1
       cmul(p[j], bit ? m3r : m0r, bit ? m3i : m0i);
       if (REV) cmul(q[j], bit ? m3r : m0r, bit ? m3i : m0i);
     }
@@ -598,6 +600,7 @@ __device__ __forceinline__ R tile_diag_grp(typename C2T<R>::T* p, typename C2T<R
   for (int j = 0; j < (1 << RB); ++j) {
     if (RC && (j & g.cm_r) != g.cm_r) continue;
     if (REV && gen) part += q[j].x * p[j].y - q[j].y * p[j].x;
+    if (!bit && g.real) continue;  // times 1
     cmul(p[j], pr, pi);
     if (REV) cmul(q[j], pr, pi);
   }
@@ -1013,6 +1016,7 @@ struct TBlock {
   int phase_first = 0, n_phases = 0;  // into the concatenated TPhase array
   std::vector<int> grad_gate;         // gradient slot -> gate list index
   size_t part_off = 0;                // into the gradient partials (doubles)
+  uint64_t active_tiles = 0;          // tiles that can be nonzero after the block
 };
 
 struct TilePlan {
@@ -1526,7 +1530,10 @@ std::atomic<uint64_t> g_jit_launches{0};
 template <typename R, bool REV>
 void launch_tile(dim3 grid, cudaStream_t st, typename C2T<R>::T* psi, typename C2T<R>::T* lam, uint64_t dim,
                  const TBlock& b, const TGate* gates, const TPhase* phases, const R* mats, uint64_t chunk,
-                 double* partial, cudaKernel_t jit = nullptr, const typename C2T<R>::T* psi_src = nullptr) {
+                 double* partial, cudaKernel_t jit = nullptr, const typename C2T<R>::T* psi_src = nullptr,
+                 bool all_tiles = false) {
+  TileGeom tg = b.geom;
+  if (!all_tiles) tg.n_tiles = std::min(tg.n_tiles, b.active_tiles);
   const int ngrad = REV ? (int)b.grad_gate.size() : 0;
   if constexpr (sizeof(R) == 4) {
     if (jit) {
@@ -1534,7 +1541,6 @@ void launch_tile(dim3 grid, cudaStream_t st, typename C2T<R>::T* psi, typename C
       const float2* asrc = psi_src ? psi_src : psi;
       float2* a1 = lam;
       uint64_t d = dim;
-      TileGeom tg = b.geom;
       const TGate* gp = gates + b.gate_first;
       int ng = b.n_gates;
       const float* mp = mats;
@@ -1553,11 +1559,11 @@ void launch_tile(dim3 grid, cudaStream_t st, typename C2T<R>::T* psi, typename C
     KB_CUDA(cudaMemcpyAsync(psi, psi_src, dim * sizeof(typename C2T<R>::T) * grid.y, cudaMemcpyDeviceToDevice, st));
   const size_t smem = tile_smem<R>(REV, b.n_gates, ngrad);
   if constexpr (sizeof(R) == 4)
-    tile_sweep_c64<REV><<<grid, kTileThreads, smem, st>>>(psi, lam, dim, b.geom, gates + b.gate_first, b.n_gates,
+    tile_sweep_c64<REV><<<grid, kTileThreads, smem, st>>>(psi, lam, dim, tg, gates + b.gate_first, b.n_gates,
                                                           phases + b.phase_first, b.n_phases, mats, chunk, ngrad,
                                                           partial);
   else
-    tile_sweep<R, REV><<<grid, kTileThreads, smem, st>>>(psi, lam, dim, b.geom, gates + b.gate_first, b.n_gates,
+    tile_sweep<R, REV><<<grid, kTileThreads, smem, st>>>(psi, lam, dim, tg, gates + b.gate_first, b.n_gates,
                                                          phases + b.phase_first, b.n_phases, mats, chunk, ngrad,
                                                          partial);
   count_launch();
@@ -1726,6 +1732,28 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     }
     real[gi] = r;
   }
+  if (tiled) {
+    // An uncontrolled Rz loses its phase e^{-it/2}: a phase common to psi and
+    // lambda = H psi drops out of the expectation and of every gradient, and
+    // diag(1, e^{it}) leaves half of the amplitudes alone.  Diagonal gates
+    // with a 1 for target bit 0 are marked for the sweeps.
+    for (size_t gi = 0; gi < G; ++gi) {
+      const int type = ops[gate_ops[gi]].type;
+      AdjGate& a = agates[gi];
+      if (type == KETGPU_RZ) {
+        if (a.pslot >= 0) {
+          a.kind = 5;
+        } else {
+          const double t = ops[gate_ops[gi]].p[0];
+          a.m[0] = 1.0;
+          a.m[1] = 0.0;
+          a.m[6] = std::cos(t);
+          a.m[7] = std::sin(t);
+        }
+      }
+      if (is_diagonal_gate(type)) real[gi] = type != KETGPU_CRZ;
+    }
+  }
   DevBuf d_agates(sizeof(AdjGate) * std::max<size_t>(G, 1), dev, st);
   if (G) KB_CUDA(cudaMemcpyAsync(d_agates.p, agates.data(), sizeof(AdjGate) * G, cudaMemcpyHostToDevice, st));
   DevBuf d_params(sizeof(double) * std::max<uint64_t>(chunk * nparams, 1), dev, st);
@@ -1768,6 +1796,26 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
       }
     }
     const uint64_t n_tiles = uint64_t{1} << (n - TB);
+    // From |0...0>, psi after block b is zero beyond the indices below the
+    // highest qubit that gates have acted on so far, and the reverse sweep
+    // needs lambda only where psi is nonzero: block b runs on that many tiles
+    // (with finite numbers: 0 * inf).  At 24 qubits the first layer's three
+    // blocks cover 1, 64 and all 4096 tiles.
+    bool finite = true;
+    for (uint64_t i = 0; i < batch * nparams && finite; ++i) finite = std::isfinite(params[i]);
+    for (int t = 0; t < T_ && finite; ++t) finite = std::isfinite(coeffs[t]);
+    for (int gi : gate_ops)
+      for (double v : ops[gi].p) finite = finite && std::isfinite(v);
+    int top = 0;
+    for (TBlock& b : tp.blocks) {
+      for (int k = 0; k < b.n_gates; ++k) {
+        const ketgpu_op& o = ops[gate_ops[tp.gates[b.gate_first + k].mat]];
+        for (int j = 0; j < gate_arity(o.type); ++j) top = std::max(top, o.q[j] + 1);
+      }
+      int outside = 0;  // qubits below `top` that are not in the tile
+      for (int q = 0; q < top; ++q) outside += std::find(b.geom.pos, b.geom.pos + TB, q) == b.geom.pos + TB;
+      b.active_tiles = finite ? uint64_t{1} << outside : n_tiles;
+    }
     // About eight rounds of every resident CTA (two per SM) over the chunk's
     // sets, in whole rounds where the set count allows: a grid of 10 x 64
     // CTAs on 296 slots ran two full rounds and a third of 48 CTAs, leaving
@@ -1863,6 +1911,8 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     auto ck_at = [&](int k) { return ck + (size_t)k * chunk * dim; };
     // forward
     T* ground = ck_direct ? ck_at(0) : psi;
+    // (a block that runs on part of the tiles leaves the rest of psi as it is)
+    if (ck_direct) KB_CUDA(cudaMemsetAsync(psi, 0, dim * sizeof(T) * nb, st));
     KB_CUDA(cudaMemsetAsync(ground, 0, dim * sizeof(T) * nb, st));
     ground_batch<R><<<(unsigned)nb, 1, 0, st>>>(ground, dim);
     count_launch();
@@ -1889,7 +1939,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
         if (bi + 1 < B && next_ck < n_ckpt && next_ck * m <= tp.blocks[bi + 1].layer) out = ck_at(next_ck++);
         dim3 grid((unsigned)gx, (unsigned)nb);
         launch_tile<R, false>(grid, st, out, nullptr, dim, b, d_tgates->as<TGate>(), d_tphases->as<TPhase>(),
-                              mats.as<R>(), chunk, nullptr, jit_fwd[bi], cur);
+                              mats.as<R>(), chunk, nullptr, jit_fwd[bi], cur, out != psi);
         cur = out;
       }
       if (cur != psi)

@@ -48,3 +48,45 @@ def test_shared_parameters(oracle, n, batch, precision):
         assert abs(values[row] - v) < TOL[precision]
         assert np.abs(grads[row] - gr).max() < TOL[precision]
     assert not grads[:, 5].any()
+
+
+@pytest.mark.parametrize("order", ["up", "down", "few"])
+@pytest.mark.parametrize("n,precision", [(13, "c64"), (13, "c128"), (16, "c64")])  # 16: blocks compiled at run time
+@pytest.mark.parametrize("ckpt", [1, 2, 0])
+def test_qubits_that_join_late_or_never(oracle, order, n, precision, ckpt):
+    """Blocks before all qubits have been acted on run on part of the tiles;
+    the Hamiltonian reaches every qubit."""
+    import ket_b200 as kb
+    from ket_b200.autograd import adjoint_expval
+    qs = list(range(n))
+    if order == "down":
+        qs = qs[::-1]
+    elif order == "few":
+        qs = [2, 3, 9]
+    c, index, k = kb.Circuit(n), [], 0
+    for layer in range(4):
+        use = qs[: max(2, (layer + 1) * len(qs) // 4)]
+        for q in use:
+            for name in ("ry", "rz", "rx"):
+                getattr(c, name)(q, 0.0)
+                index.append(k)
+                k += 1
+            c.rz(q, 0.3 + layer)
+            index.append(-1)
+        for a, b in zip(use[:-1], use[1:]):
+            c.cx(a, b)
+            index.append(-1)
+        c.crz(use[0], use[-1], 0.0)
+        index.append(k)
+        k += 1
+        c.barrier()
+        index.append(-1)
+    index = np.array(index, dtype=np.int32)
+    g = np.random.default_rng(n)
+    theta = g.uniform(-3, 3, (2, k))
+    terms = [(float(g.standard_normal()), "".join(g.choice(list("IXYZ"), n))) for _ in range(6)]
+    values, grads = adjoint_expval(c, index, theta, terms, precision, checkpoint_every=ckpt)
+    for row in range(2):
+        v, gr = oracle.adjoint(n, c.to_ops(), index, theta[row], terms)
+        assert abs(values[row] - v) < TOL[precision]
+        assert np.abs(grads[row] - gr).max() < TOL[precision]

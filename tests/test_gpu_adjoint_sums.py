@@ -90,3 +90,29 @@ def test_qubits_that_join_late_or_never(oracle, order, n, precision, ckpt):
         v, gr = oracle.adjoint(n, c.to_ops(), index, theta[row], terms)
         assert abs(values[row] - v) < TOL[precision]
         assert np.abs(grads[row] - gr).max() < TOL[precision]
+
+
+@pytest.mark.parametrize("terms", [1, 31, 32, 33, 70, 300, 1101])  # 1101: beyond the shared-memory form
+@pytest.mark.parametrize("n", [1, 2, 3, 9, 13])
+@pytest.mark.parametrize("precision", ["c64", "c128"])
+def test_hamiltonians_of_every_length(oracle, n, terms, precision):
+    """lambda = H psi: term counts around the 32-term masks, states of less
+    than a CTA's word count, strings with and without Y and X on qubit 0."""
+    import ket_b200 as kb
+    from ket_b200.autograd import adjoint_expval
+    c, index = kb.Circuit(n), []
+    for q in range(n):
+        c.ry(q, 0.0)
+        c.rx(q, 0.0)
+        index += [2 * q, 2 * q + 1]
+    for q in range(n - 1):
+        c.cx(q, q + 1)
+        index.append(-1)
+    index = np.array(index, dtype=np.int32)
+    g = np.random.default_rng(terms + n)
+    theta = g.uniform(-3, 3, (1, 2 * n))
+    ham = [(float(g.standard_normal()) / terms, "".join(g.choice(list("IXYZ"), n))) for _ in range(terms)]
+    values, grads = adjoint_expval(c, index, theta, ham, precision)
+    v, gr = oracle.adjoint(n, c.to_ops(), index, theta[0], ham)
+    assert abs(values[0] - v) < TOL[precision]
+    assert np.abs(grads[0] - gr).max() < TOL[precision]

@@ -328,27 +328,160 @@ __device__ __forceinline__ float pk_dispatch(int op, PackState& a, PackState& l,
 #undef KB_PK_CASE
 
 // ---------------------------------------------------------------------------
+// Gate bodies of the per-block kernels.  A pack is one amplitude, (re, im), as
+// it lies in shared memory: a phase's loads and stores are whole 8-byte words
+// with no register moves, and all four register slots can be targets (the
+// form above, two amplitudes a pack, spent 27% of its instructions on moves and
+// needs a fourth or fifth phase per block).  A real 2x2 and the Y gradient act
+// on packs alike.  A complex 2x2 takes the halves swapped, (cr, cr) * (re, im)
+// + (-ci, ci) * (im, re).  A phase and the X and Z gradients, whose only packed
+// work would be on swapped halves, use scalar instructions: as many, and no
+// moves.  Coefficients as above, but [8..11] hold (-c0i, c0i) ... (-c3i, c3i).
+struct NatState {
+  f2 a[16];
+};
+
+__device__ __forceinline__ f2 swap_halves(f2 v) {
+  float lo, hi;
+  upk2(v, lo, hi);
+  return pk2(hi, lo);
+}
+// x times (cr, ci).
+__device__ __forceinline__ f2 nk_mul(f2 x, float cr, float ci) {
+  float r, i;
+  upk2(x, r, i);
+  return pk2(fmaf(cr, r, -ci * i), fmaf(cr, i, ci * r));
+}
+// plus += l_re a_im, minus += l_im a_re: Im(conj(l) a) is their difference.
+__device__ __forceinline__ void nk_im(f2 l, f2 a, float& plus, float& minus) {
+  float lr, li, ar, ai;
+  upk2(l, lr, li);
+  upk2(a, ar, ai);
+  plus = fmaf(lr, ai, plus);
+  minus = fmaf(li, ar, minus);
+}
+
+template <bool REAL>
+__device__ __forceinline__ void nk_2x2(f2& a, f2& b, const f2* c) {
+  f2 x, y;
+  if (REAL) {
+    x = fma2(c[0], a, mul2p(c[2], b));
+    y = fma2(c[4], a, mul2p(c[6], b));
+  } else {
+    const f2 sa = swap_halves(a), sb = swap_halves(b);
+    x = fma2(c[0], a, fma2(c[8], sa, fma2(c[2], b, mul2p(c[9], sb))));
+    y = fma2(c[4], a, fma2(c[10], sa, fma2(c[6], b, mul2p(c[11], sb))));
+  }
+  a = x;
+  b = y;
+}
+
+__device__ __forceinline__ void nk_exchange(f2& a, f2& b) {
+  const f2 t = a;
+  a = b;
+  b = t;
+}
+
+// Swap on slot S: X, CX, CCX.
+template <int S, bool REV>
+__device__ __forceinline__ float nk_swap(NatState& a, NatState& l, const TGate& g) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if ((j & (1 << S)) || (j & g.cm_r) != g.cm_r) continue;
+    nk_exchange(a.a[j], a.a[j | (1 << S)]);
+    if (REV) nk_exchange(l.a[j], l.a[j | (1 << S)]);
+  }
+  return 0.f;
+}
+
+template <int A, int B, bool REV>
+__device__ __forceinline__ float nk_swap2(NatState& a, NatState& l, const TGate& g) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (!(j & (1 << A)) || (j & (1 << B)) || (j & g.cm_r) != g.cm_r) continue;
+    nk_exchange(a.a[j], a.a[j ^ (1 << A) ^ (1 << B)]);
+    if (REV) nk_exchange(l.a[j], l.a[j ^ (1 << A) ^ (1 << B)]);
+  }
+  return 0.f;
+}
+
+// 2x2 on slot S.  Reverse: the gradient term Im <l|G|a> first (1 X, 2 Y, 3 Z).
+template <int S, bool REAL, int GEN, bool REV>
+__device__ __forceinline__ float nk_pair(NatState& a, NatState& l, const TGate& g, const f2* c) {
+  f2 plus = 0, minus = 0;
+  float p0 = 0.f, m0 = 0.f, p1 = 0.f, m1 = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if ((j & (1 << S)) || (j & g.cm_r) != g.cm_r) continue;
+    const int j1 = j | (1 << S);
+    if (REV && GEN == 1) {  // X: Im(conj(l0) a1) + Im(conj(l1) a0)
+      nk_im(l.a[j], a.a[j1], p0, m0);
+      nk_im(l.a[j1], a.a[j], p1, m1);
+    } else if (REV && GEN == 2) {  // Y: (l1r a0r + l1i a0i) - (l0r a1r + l0i a1i)
+      plus = fma2(l.a[j1], a.a[j], plus);
+      minus = fma2(l.a[j], a.a[j1], minus);
+    } else if (REV && GEN == 3) {  // Z: Im(conj(l0) a0) - Im(conj(l1) a1)
+      nk_im(l.a[j], a.a[j], p0, m0);
+      nk_im(l.a[j1], a.a[j1], p1, m1);
+    }
+    nk_2x2<REAL>(a.a[j], a.a[j1], c);
+    if (REV) nk_2x2<REAL>(l.a[j], l.a[j1], c);
+  }
+  if (!REV || GEN == 0) return 0.f;
+  if (GEN == 1) return (p0 - m0) + (p1 - m1);
+  return GEN == 2 ? hsum2(plus) - hsum2(minus) : (p0 - m0) - (p1 - m1);
+}
+
+// Diagonal gate; TS: register slot of the target, or -1 for a group bit.
+template <int TS, int GEN, bool REV>
+__device__ __forceinline__ float nk_diag(NatState& a, NatState& l, const TGate& g, const f2* c, int gbase) {
+  const bool gbit = TS < 0 ? ((gbase >> g.tbit) & 1) : false;
+  float p0 = 0.f, m0 = 0.f, p1 = 0.f, m1 = 0.f;  // target bit 0 / 1
+  float unused, cr0, ci0, cr1, ci1;
+  upk2(c[0], cr0, unused);
+  upk2(c[8], unused, ci0);
+  upk2(c[6], cr1, unused);
+  upk2(c[11], unused, ci1);
+  if (TS < 0 && gbit) cr0 = cr1, ci0 = ci1;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if ((j & g.cm_r) != g.cm_r) continue;
+    const bool bit = TS >= 0 ? ((j >> (TS < 0 ? 0 : TS)) & 1) : false;  // compile time
+    if (REV && GEN && (bit || TS < 0 || GEN == 3)) {
+      if (bit) nk_im(l.a[j], a.a[j], p1, m1);
+      else nk_im(l.a[j], a.a[j], p0, m0);
+    }
+    if (TS >= 0 && g.real && !bit) continue;  // times 1
+    a.a[j] = nk_mul(a.a[j], bit ? cr1 : cr0, bit ? ci1 : ci0);
+    if (REV) l.a[j] = nk_mul(l.a[j], bit ? cr1 : cr0, bit ? ci1 : ci0);
+  }
+  if (!(REV && GEN)) return 0.f;
+  const float t0 = p0 - m0, t1 = p1 - m1;
+  if (TS < 0) return GEN == 3 ? (gbit ? -t0 : t0) : (gbit ? t0 : 0.f);  // every element has target bit gbit
+  return GEN == 3 ? t0 - t1 : t1;
+}
+
+// ---------------------------------------------------------------------------
 // Pieces of a complex64 tiled sweep, used by the per-block kernels that are
 // generated with their phases and gates as compile-time constants.
 
-// Per-CTA set-up: tile offset tables, the block's gate records and this
-// set's packed coefficients (U forward, U^dag reverse), and `acc_words`
+// Per-CTA set-up: tile offset tables and this set's packed coefficients (U forward, U^dag reverse), and `acc_words`
 // zeroed 4-byte words of gradient sums.
 template <bool REV>
 __device__ __forceinline__ void c64_setup(const TileGeom& tg, const TGate* __restrict__ gates, int ngates,
                                           const float* __restrict__ mats, uint64_t mat_stride, int set,
-                                          int acc_words, uint64_t* off_lo, uint64_t* off_hi, f2* spk,
-                                          float* acc) {
-  constexpr int TB = TileCfg<float>::TB;
+                                          int acc_words, uint64_t* off, f2* spk, float* acc) {
+  // byte offsets of tile element tid + 256 r from the tile's base are those of
+  // tid (off[tid]) plus those of 256 r (off[256 + r])
   const int tid = threadIdx.x;
-  if (tid < 128) {
-    const int half = tid >> 6, e = tid & 63;
-    uint64_t off = 0;
-    for (int b = 0; b < 6; ++b) {
-      const int tb = 6 * half + b;
-      if (tb < TB && ((e >> b) & 1)) off |= (uint64_t)1 << tg.pos[tb];
-    }
-    (half ? off_hi : off_lo)[e] = off;
+  uint64_t o = 0, hi = 0;
+  for (int b = 0; b < 8; ++b)
+    if ((tid >> b) & 1) o |= (uint64_t)8 << tg.pos[b];
+  off[tid] = o;
+  if (tid < 16) {
+    for (int b = 0; b < 4; ++b)
+      if ((tid >> b) & 1) hi |= (uint64_t)8 << tg.pos[8 + b];
+    off[kTileThreads + tid] = hi;
   }
   for (int i = tid; i < ngates; i += kTileThreads) {
     const float* m = mats + ((uint64_t)gates[i].mat * mat_stride + set) * 8;
@@ -364,13 +497,8 @@ __device__ __forceinline__ void c64_setup(const TileGeom& tg, const TGate* __res
     f2* c = spk + 16 * i;
     for (int k = 0; k < 4; ++k) {
       c[2 * k] = pk2(cr[k], cr[k]);
-      c[2 * k + 1] = pk2(ci[k], ci[k]);
-      c[8 + k] = pk2(-ci[k], -ci[k]);
+      c[8 + k] = pk2(-ci[k], ci[k]);
     }
-    c[12] = pk2(cr[0], cr[3]);
-    c[13] = pk2(ci[0], ci[3]);
-    c[14] = pk2(-ci[0], -ci[3]);
-    c[15] = 0;
   }
   if (REV)
     for (int i = tid; i < acc_words; i += kTileThreads) acc[i] = 0.f;
@@ -387,72 +515,59 @@ __device__ __forceinline__ uint64_t c64_tile_base(const TileGeom& tg, uint64_t t
 }
 
 template <bool REV>
-__device__ __forceinline__ void c64_prefetch(const TileGeom& tg, const uint64_t* off_lo, const uint64_t* off_hi,
-                                             uint64_t t, float2* buf, const float2* s, const float2* l) {
+__device__ __forceinline__ void c64_prefetch(const TileGeom& tg, const uint64_t* off, uint64_t t, float2* buf,
+                                             const float2* s, const float2* l) {
   constexpr int TILE = 1 << TileCfg<float>::TB;
-  const uint64_t base = c64_tile_base(tg, t);
-#pragma unroll 2
+  const int tid = threadIdx.x, ptid = tphys<float>(tid);
+  const uint64_t at = 8 * c64_tile_base(tg, t) + off[tid];
+  const char* ps = reinterpret_cast<const char*>(s) + at;
+  const char* pl = reinterpret_cast<const char*>(l) + at;
+#pragma unroll
   for (int r = 0; r < 16; ++r) {
-    const int e = threadIdx.x + r * kTileThreads;
-    const uint64_t o = base + (off_lo[e & 63] | off_hi[e >> 6]);
-    tile_cp_async(buf + tphys<float>(e), s + o);
-    if (REV) tile_cp_async(buf + TILE + tphys<float>(e), l + o);
+    const uint64_t o = off[kTileThreads + r];
+    float2* d = buf + (ptid ^ tphys<float>(r * kTileThreads));
+    tile_cp_async(d, reinterpret_cast<const float2*>(ps + o));
+    if (REV) tile_cp_async(d + TILE, reinterpret_cast<const float2*>(pl + o));
   }
 }
 
 template <bool REV>
-__device__ __forceinline__ void c64_store_tile(const TileGeom& tg, const uint64_t* off_lo, const uint64_t* off_hi,
-                                               uint64_t t, const float2* sp, const float2* sl, float2* s, float2* l) {
-  const uint64_t base = c64_tile_base(tg, t);
-  const volatile uint64_t* vlo = off_lo;
-  const volatile uint64_t* vhi = off_hi;
-#pragma unroll 2
+__device__ __forceinline__ void c64_store_tile(const TileGeom& tg, const uint64_t* off, uint64_t t, const float2* sp,
+                                               const float2* sl, float2* s, float2* l) {
+  const volatile uint64_t* voff = off;
+  const int tid = threadIdx.x, ptid = tphys<float>(tid);
+  const uint64_t at = 8 * c64_tile_base(tg, t) + voff[tid];
+  char* ps = reinterpret_cast<char*>(s) + at;
+  char* pl = reinterpret_cast<char*>(l) + at;
+#pragma unroll
   for (int r = 0; r < 16; ++r) {
-    const int e = threadIdx.x + r * kTileThreads;
-    const uint64_t o = base + (vlo[e & 63] | vhi[e >> 6]);
-    s[o] = sp[tphys<float>(e)];
-    if (REV) l[o] = sl[tphys<float>(e)];
+    const uint64_t o = voff[kTileThreads + r];
+    const int e = ptid ^ tphys<float>(r * kTileThreads);
+    *reinterpret_cast<float2*>(ps + o) = sp[e];
+    if (REV) *reinterpret_cast<float2*>(pl + o) = sl[e];
   }
 }
 
-// Shared-memory addresses of pack jo: pg ^ (pb1, pb2, pb3 by the bits of jo),
-// and the same ^ pb0 for its upper half.
+// Shared-memory address of element j: pg ^ (pb0 .. pb3 by the bits of j).
 template <bool REV>
 __device__ __forceinline__ void c64_load_phase(const float2* sp, const float2* sl, int pg, int pb0, int pb1, int pb2,
-                                               int pb3, PackState& A, PackState& L) {
+                                               int pb3, NatState& A, NatState& L) {
 #pragma unroll
-  for (int jo = 0; jo < 8; ++jo) {
-    const int a0 = pg ^ ((jo & 1) ? pb1 : 0) ^ ((jo & 2) ? pb2 : 0) ^ ((jo & 4) ? pb3 : 0);
-    const int a1 = a0 ^ pb0;
-    const float2 x = sp[a0], y = sp[a1];
-    A.r[jo] = pk2(x.x, y.x);
-    A.i[jo] = pk2(x.y, y.y);
-    if (REV) {
-      const float2 u = sl[a0], v = sl[a1];
-      L.r[jo] = pk2(u.x, v.x);
-      L.i[jo] = pk2(u.y, v.y);
-    }
+  for (int j = 0; j < 16; ++j) {
+    const int p = pg ^ ((j & 1) ? pb0 : 0) ^ ((j & 2) ? pb1 : 0) ^ ((j & 4) ? pb2 : 0) ^ ((j & 8) ? pb3 : 0);
+    A.a[j] = reinterpret_cast<const f2*>(sp)[p];
+    if (REV) L.a[j] = reinterpret_cast<const f2*>(sl)[p];
   }
 }
 
 template <bool REV>
 __device__ __forceinline__ void c64_store_phase(float2* sp, float2* sl, int pg, int pb0, int pb1, int pb2, int pb3,
-                                                const PackState& A, const PackState& L) {
+                                                const NatState& A, const NatState& L) {
 #pragma unroll
-  for (int jo = 0; jo < 8; ++jo) {
-    const int a0 = pg ^ ((jo & 1) ? pb1 : 0) ^ ((jo & 2) ? pb2 : 0) ^ ((jo & 4) ? pb3 : 0);
-    const int a1 = a0 ^ pb0;
-    float xr, yr, xi, yi;
-    upk2(A.r[jo], xr, yr);
-    upk2(A.i[jo], xi, yi);
-    sp[a0] = make_float2(xr, xi);
-    sp[a1] = make_float2(yr, yi);
-    if (REV) {
-      upk2(L.r[jo], xr, yr);
-      upk2(L.i[jo], xi, yi);
-      sl[a0] = make_float2(xr, xi);
-      sl[a1] = make_float2(yr, yi);
-    }
+  for (int j = 0; j < 16; ++j) {
+    const int p = pg ^ ((j & 1) ? pb0 : 0) ^ ((j & 2) ? pb1 : 0) ^ ((j & 4) ? pb2 : 0) ^ ((j & 8) ? pb3 : 0);
+    reinterpret_cast<f2*>(sp)[p] = A.a[j];
+    if (REV) reinterpret_cast<f2*>(sl)[p] = L.a[j];
   }
 }
 

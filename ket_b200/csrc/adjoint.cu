@@ -1150,9 +1150,9 @@ TileOp tile_op_of(const Pass& p, const int* tpos_of_qubit) {
 
 template <typename R>
 TilePlan plan_tiles(int n, const ketgpu_op* ops, const std::vector<int>& gate_ops, const std::vector<int>& layer_of,
-                    const std::vector<GateGeom>& geo, const std::vector<uint8_t>& real, int seg_layers) {
+                    const std::vector<GateGeom>& geo, const std::vector<uint8_t>& real, int seg_layers,
+                    bool kPacked) {
   constexpr int TB = TileCfg<R>::TB, RB = TileCfg<R>::RB;
-  constexpr bool kPacked = sizeof(R) == 4;  // complex64 sweeps pack pairs of amplitudes
   TilePlan tp;
   const int G = (int)gate_ops.size();
   std::vector<uint64_t> qmask(G);
@@ -1335,6 +1335,10 @@ TilePlan plan_tiles(int n, const ketgpu_op* ops, const std::vector<int>& gate_op
   return tp;
 }
 
+// packed: the phases of the interpreted complex64 sweep, whose packs hold two
+// amplitudes (slot 0 is the pack bit); otherwise all slots are targets.  The
+// blocks and their gates are the same.
+//
 // The tiled plan with blocks per layer, or per checkpoint segment of m
 // layers when that needs fewer blocks (fewer HBM passes; a block that spans
 // layers holds more gates and register phases, so on a tie the per-layer
@@ -1342,10 +1346,10 @@ TilePlan plan_tiles(int n, const ketgpu_op* ops, const std::vector<int>& gate_op
 template <typename R>
 TilePlan plan_tiles_best(int n, const ketgpu_op* ops, const std::vector<int>& gate_ops,
                          const std::vector<int>& layer_of, const std::vector<GateGeom>& geo,
-                         const std::vector<uint8_t>& real, int m) {
-  TilePlan per_layer = plan_tiles<R>(n, ops, gate_ops, layer_of, geo, real, 1);
+                         const std::vector<uint8_t>& real, int m, bool packed = sizeof(R) == 4) {
+  TilePlan per_layer = plan_tiles<R>(n, ops, gate_ops, layer_of, geo, real, 1, packed);
   if (m <= 1) return per_layer;
-  TilePlan per_seg = plan_tiles<R>(n, ops, gate_ops, layer_of, geo, real, m);
+  TilePlan per_seg = plan_tiles<R>(n, ops, gate_ops, layer_of, geo, real, m, packed);
   return per_seg.blocks.size() < per_layer.blocks.size() ? std::move(per_seg) : std::move(per_layer);
 }
 
@@ -1463,17 +1467,6 @@ cudaKernel_t jit_kernel(const std::string& src) {
 
 int tphys_host(int e) { return e ^ (((e >> 4) ^ (e >> 8)) & 15); }
 
-int pk_opcode_host(const TGate& g, bool rev) {
-  const int rc = g.cm_r ? 1 : 0;
-  const int gen = rev ? g.gen : 0;
-  switch (g.kind) {
-    case kTPair: return (g.s0 - 1) * 16 + (g.real ? 8 : 0) + gen * 2 + rc;
-    case kTPairSwap: return 48 + (g.s0 - 1) * 2 + rc;
-    case kTSwap2: return 54 + (g.s0 == 1 ? (g.s1 == 2 ? 0 : 1) : 2) * 2 + rc;
-    default: return 60 + (g.tslot + 1) * 6 + (gen == 3 ? 1 : gen == 4 ? 2 : 0) * 2 + rc;
-  }
-}
-
 // The kernel of one complex64 block: phases (in sweep order) and their gates
 // as constants.  Parameters as tile_sweep_c64, without the phase table.
 // Gradient slots per thread for a reverse block with `ngrad` gradients: the
@@ -1507,24 +1500,24 @@ std::string jit_source(const std::vector<TPhase>& phases, const std::vector<TGat
   line("  float* accf = reinterpret_cast<float*>(spk + 16 * ngates);");
   line("  double* acc = reinterpret_cast<double*>(accf);");
   line("  constexpr int GS = " + std::to_string(gs) + ";  // per-thread gradient slots (0: per-warp sums)");
-  line("  __shared__ uint64_t off_lo[64], off_hi[64];");
+  line("  __shared__ uint64_t off[kTileThreads + 16];");
   line("  const int tid = threadIdx.x;");
   line("  const int set = blockIdx.y;");
   line("  float2* s = psi + (uint64_t)set * dim;  // tiles are stored here");
   line("  const float2* sin = psi_src + (uint64_t)set * dim;  // and loaded from here (psi, or a checkpoint)");
   line("  float2* l = REV ? lam + (uint64_t)set * dim : nullptr;");
   line("  c64_setup<REV>(tg, gates, ngates, mats, mat_stride, set, GS ? kTileThreads * GS : 2 * kTileWarps * ngrad,");
-  line("                 off_lo, off_hi, spk, accf);");
+  line("                 off, spk, accf);");
   line("  __syncthreads();");
   line("  int cur = 0;");
-  line("  if (!SINGLE && blockIdx.x < tg.n_tiles) c64_prefetch<REV>(tg, off_lo, off_hi, blockIdx.x, bufs, sin, l);");
+  line("  if (!SINGLE && blockIdx.x < tg.n_tiles) c64_prefetch<REV>(tg, off, blockIdx.x, bufs, sin, l);");
   line("  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");");
   line("  for (uint64_t t = blockIdx.x; t < tg.n_tiles; t += gridDim.x) {");
   line("    float2* sp = bufs + (SINGLE ? 0 : cur) * BUF;");
   line("    float2* sl = sp + TILE;");
-  line("    if (SINGLE) c64_prefetch<REV>(tg, off_lo, off_hi, t, bufs, sin, l);");
+  line("    if (SINGLE) c64_prefetch<REV>(tg, off, t, bufs, sin, l);");
   line("    else if (t + gridDim.x < tg.n_tiles)");
-  line("      c64_prefetch<REV>(tg, off_lo, off_hi, t + gridDim.x, bufs + (cur ^ 1) * BUF, sin, l);");
+  line("      c64_prefetch<REV>(tg, off, t + gridDim.x, bufs + (cur ^ 1) * BUF, sin, l);");
   line("    asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");");
   line("    if (SINGLE) asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");");
   line("    else asm volatile(\"cp.async.wait_group 1;\\n\" ::: \"memory\");");
@@ -1541,22 +1534,31 @@ std::string jit_source(const std::vector<TPhase>& phases, const std::vector<TGat
     line("    {");
     line("      const int gbase = " + gb + ";");
     line("      const int pg = tphys<float>(gbase);");
-    line("      PackState A, L;");
+    line("      NatState A, L;");
     std::string pb;
     for (int b = 0; b < 4; ++b) pb += ", " + std::to_string(tphys_host(1 << P.r[b]));
     line("      c64_load_phase<REV>(sp, sl, pg" + pb + ", A, L);");
     for (int c = 0; c < P.count; ++c) {
       const int gi = rev ? P.first + P.count - 1 - c : P.first + c;
       const TGate& g = gates[gi];
-      const int op = pk_opcode_host(g, rev);
       char buf[512];
       std::snprintf(buf, sizeof buf,
                     "      { constexpr TGate g{%d, %d, %d, %d, %d, %d, %d, %d, %d, %d, %d}; float part = 0.f;",
                     (int)g.kind, (int)g.s0, (int)g.s1, (int)g.tslot, (int)g.tbit, (int)g.cm_r, (int)(rev ? g.gen : 0),
                     (int)g.real, (int)g.cm_g, (int)g.grad, 0);  // mat: read from the gate table at set-up
       line(buf);
-      const std::string call = "part = pk_exec<" + std::to_string(op) + ", REV>(A, L, g, spk + 16 * " +
-                               std::to_string(gi) + ", gbase);";
+      const auto num = [](int v) { return std::to_string(v); };
+      const int gen = rev ? g.gen : 0;
+      const std::string coef = "spk + 16 * " + num(gi);
+      std::string call;
+      if (g.kind == kTPair)
+        call = "part = nk_pair<" + num(g.s0) + ", " + (g.real ? "true" : "false") + ", " + num(gen) + ", REV>(A, L, g, " +
+               coef + ");";
+      else if (g.kind == kTPairSwap) call = "part = nk_swap<" + num(g.s0) + ", REV>(A, L, g);";
+      else if (g.kind == kTSwap2) call = "part = nk_swap2<" + num(g.s0) + ", " + num(g.s1) + ", REV>(A, L, g);";
+      else
+        call = "part = nk_diag<" + num(g.tslot) + ", " + num(gen == 3 || gen == 4 ? gen : 0) + ", REV>(A, L, g, " + coef +
+               ", gbase);";
       if (g.cm_g) line("        if ((gbase & " + std::to_string((int)g.cm_g) + ") == " + std::to_string((int)g.cm_g) +
                        ") " + call);
       else line("        " + call);
@@ -1570,7 +1572,7 @@ std::string jit_source(const std::vector<TPhase>& phases, const std::vector<TGat
     line("      __syncthreads();");
     line("    }");
   }
-  line("    c64_store_tile<REV>(tg, off_lo, off_hi, t, sp, sl, s, l);");
+  line("    c64_store_tile<REV>(tg, off, t, sp, sl, s, l);");
   line("    __syncthreads();");
   line("    cur ^= 1;");
   line("  }");
@@ -1860,11 +1862,12 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     if (want_jit && nvrtc().ok) {
       jit_fwd.assign(tp.blocks.size(), nullptr);
       jit_rev.assign(tp.blocks.size(), nullptr);
-      for (size_t bi = 0; bi < tp.blocks.size(); ++bi) {
-        const TBlock& b = tp.blocks[bi];
-        const std::vector<TPhase> ph(tp.phases.begin() + b.phase_first,
-                                     tp.phases.begin() + b.phase_first + b.n_phases);
-        const std::vector<TGate> gs(tp.gates.begin() + b.gate_first, tp.gates.begin() + b.gate_first + b.n_gates);
+      const TilePlan tj = plan_tiles_best<R>(n, ops, gate_ops, layer_of, geo, real, m, false);
+      for (size_t bi = 0; bi < tj.blocks.size(); ++bi) {
+        const TBlock& b = tj.blocks[bi];
+        const std::vector<TPhase> ph(tj.phases.begin() + b.phase_first,
+                                     tj.phases.begin() + b.phase_first + b.n_phases);
+        const std::vector<TGate> gs(tj.gates.begin() + b.gate_first, tj.gates.begin() + b.gate_first + b.n_gates);
         jit_fwd[bi] = jit_kernel(jit_source(ph, gs, false));
         jit_rev[bi] = jit_kernel(jit_source(ph, gs, true));
         if (jit_fwd[bi])

@@ -400,6 +400,272 @@ __global__ void __launch_bounds__(kAThreads)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Resident form, for states that fit the shared memory of one CTA: one CTA a
+// parameter set runs the whole circuit forwards, H psi (where that is little
+// work, else between two launches) and the reverse sweep with psi and lambda
+// in shared memory, one barrier a gate.  The arithmetic of a gate is that of
+// the per-gate kernels.
+//
+// What bounds it is the chain of gates: a gate of a small state is a few
+// hundred cycles of shared-memory reads, products and a barrier, against a
+// launch (about 3 us on the device, 5 us in the stream) in the per-gate form.
+// So everything that a gate needs is staged ahead (records and matrices, 64
+// gates at a time), and the FP64 partial sums of a gradient stay one per
+// thread until 16 gates have them, when each warp sums whole rows.
+// A call with 4 layers and 16 terms, 8 sets: 8 qubits complex64 1255 -> 493
+// us, 10 qubits 1459 -> 538, 10 qubits complex128 1440 -> 508 (per gate
+// before), of which some 400 us are the host's.  256 threads a CTA: with 512
+// or 1024 a few sets take as long, 1024 sets of 11 qubits 2.33 and 2.25 ms
+// against 1.97.  Up to 11 qubits: at 12 (complex64) one tile holds a state too, and the
+// tiled sweeps, with 16 amplitudes a thread in registers, take 776 us against 786 (8
+// sets) and 1116 against 1094 (256 sets); at 11 (complex128) they take 683
+// against 600 and, for 1024 sets, 2.36 against 2.18 ms.
+constexpr int kResThreads = 256;  // at most
+constexpr int kResGates = 64;     // gates staged at a time
+constexpr int kResRows = 16;      // gradient rows between two sums
+constexpr int kResMaxQubits = 11;
+// H psi by the set's own CTA up to this many amplitudes x terms; there (11
+// qubits, 128 terms) it takes as long as the launches that spread it over the
+// chip: 8 sets 778 against 730 us, 512 sets 1126 against 1117.
+constexpr uint64_t kResHamWork = 1u << 18;
+
+struct ResGate {
+  uint32_t p0, p1;
+  int32_t ck;  // the state after this gate is this checkpoint (0: none)
+  int16_t fixed[3];
+  uint8_t nfixed, kind, gen, grad;  // grad: has a row of gradient partials
+};
+
+struct ResTerm {
+  uint32_t flip, sign;
+  double c;  // real: c, imaginary: i c
+  uint32_t imag, pad;
+};
+
+enum { kResForward = 1, kResHam = 2, kResReverse = 4 };
+
+__device__ __forceinline__ uint32_t res_index(const ResGate& g, uint32_t i) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    if (j < g.nfixed) i = ((i >> g.fixed[j]) << (g.fixed[j] + 1)) | (i & ((1u << g.fixed[j]) - 1));
+  return i;
+}
+
+template <typename R>
+struct ResMat {
+  R r[4], i[4];
+};
+
+template <typename R, typename T>
+__device__ __forceinline__ T res_mul(R mr, R mi, T a) {
+  T o;
+  o.x = mr * a.x - mi * a.y;
+  o.y = mr * a.y + mi * a.x;
+  return o;
+}
+
+template <typename R, typename T>
+__device__ __forceinline__ void res_pair(const ResMat<R>& m, T a, T c, T& x, T& y) {
+  x.x = m.r[0] * a.x - m.i[0] * a.y + m.r[1] * c.x - m.i[1] * c.y;
+  x.y = m.r[0] * a.y + m.i[0] * a.x + m.r[1] * c.y + m.i[1] * c.x;
+  y.x = m.r[2] * a.x - m.i[2] * a.y + m.r[3] * c.x - m.i[3] * c.y;
+  y.y = m.r[2] * a.y + m.i[2] * a.x + m.r[3] * c.y + m.i[3] * c.x;
+}
+
+size_t resident_smem(size_t state_bytes, int threads, size_t real_bytes) {
+  return 2 * state_bytes + sizeof(double) * kResRows * (size_t)threads + kResGates * (sizeof(ResGate) + 8 * real_bytes);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kResThreads)
+    adjoint_resident(typename C2T<R>::T* __restrict__ psi, typename C2T<R>::T* __restrict__ lam,
+                     typename C2T<R>::T* __restrict__ ck, int n, const ResGate* __restrict__ gates, int ngates,
+                     const double* __restrict__ mats, uint64_t chunk, const ResTerm* __restrict__ terms, int nterms,
+                     int phases, double* __restrict__ gpart, double* __restrict__ vpart) {
+  using T = typename C2T<R>::T;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  __shared__ double wsum[kResThreads / 32];
+  const uint32_t dim = 1u << n, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const uint64_t set = blockIdx.x;
+  T* s = reinterpret_cast<T*>(rsm);
+  T* l = s + dim;
+  double* rows = reinterpret_cast<double*>(l + dim);  // [row][thread]
+  R* cm = reinterpret_cast<R*>(rows + kResRows * nt);
+  ResGate* cg = reinterpret_cast<ResGate*>(cm + 8 * kResGates);
+  auto stage = [&](int first, int count) {
+    __syncthreads();
+    for (int i = (int)tid; i < 8 * count; i += (int)nt)
+      cm[i] = (R)mats[((uint64_t)(first + (i >> 3)) * chunk + set) * 8 + (i & 7)];
+    for (int i = (int)tid; i < count; i += (int)nt) cg[i] = gates[first + i];
+    __syncthreads();
+  };
+  auto count_of = [&](const ResGate& g) { return dim >> g.nfixed; };
+
+  if (phases & kResForward) {
+    for (uint32_t i = tid; i < dim; i += nt) {
+      T z;
+      z.x = i == 0 ? (R)1 : (R)0;
+      z.y = (R)0;
+      s[i] = z;
+    }
+    for (int c0 = 0; c0 < ngates; c0 += kResGates) {
+      const int cn = min(kResGates, ngates - c0);
+      stage(c0, cn);
+      for (int k = 0; k < cn; ++k) {
+        const ResGate g = cg[k];
+        const R* e = cm + 8 * k;
+        ResMat<R> m;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m.r[j] = e[2 * j], m.i[j] = e[2 * j + 1];
+        const uint32_t count = count_of(g);
+        if (g.kind == 2) {
+          for (uint32_t i = tid; i < count; i += nt) {
+            const uint32_t b = res_index(g, i) | g.p0;
+            s[b] = res_mul<R, T>(m.r[0], m.i[0], s[b]);
+          }
+        } else {
+          for (uint32_t i = tid; i < count; i += nt) {
+            const uint32_t b = res_index(g, i);
+            const T a = s[b | g.p0], c = s[b | g.p1];
+            T x = c, y = a;
+            if (g.kind == 0) res_pair<R, T>(m, a, c, x, y);
+            s[b | g.p0] = x;
+            s[b | g.p1] = y;
+          }
+        }
+        __syncthreads();
+        if (g.ck) {  // the same thread reads it back
+          T* o = ck + ((uint64_t)g.ck * chunk + set) * dim;
+          for (uint32_t i = tid; i < dim; i += nt) o[i] = s[i];
+          __syncthreads();
+        }
+      }
+    }
+    __syncthreads();
+    if (!(phases & kResHam))
+      for (uint32_t i = tid; i < dim; i += nt) psi[set * dim + i] = s[i];
+  } else {
+    for (uint32_t i = tid; i < dim; i += nt) {
+      s[i] = psi[set * dim + i];
+      l[i] = lam[set * dim + i];
+    }
+  }
+
+  if (phases & kResHam) {
+    double e = 0.0;
+    for (uint32_t y = tid; y < dim; y += nt) {
+      double re = 0.0, im = 0.0;
+#pragma unroll 4
+      for (int t = 0; t < nterms; ++t) {
+        const ResTerm h = terms[t];
+        const uint32_t x = y ^ h.flip;
+        const T a = s[x];
+        const double c = (__popc(x & h.sign) & 1) ? -h.c : h.c;
+        const double ar = a.x, ai = a.y;
+        re = fma(c, h.imag ? -ai : ar, re);
+        im = fma(c, h.imag ? ar : ai, im);
+      }
+      T o;
+      o.x = (R)re;
+      o.y = (R)im;
+      l[y] = o;
+      const T p = s[y];
+      e += (double)p.x * re + (double)p.y * im;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+    if (lane == 0) wsum[warp] = e;
+    __syncthreads();
+    if (tid == 0) {
+      double v = 0.0;
+      for (uint32_t w = 0; w < nt / 32; ++w) v += wsum[w];
+      vpart[set] = v;
+    }
+  }
+
+  if (phases & kResReverse) {
+    int row = 0;
+    int32_t row_gate[kResRows];
+    auto sum_rows = [&]() {  // row r of `rows` belongs to gate row_gate[r]
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kResRows; ++r) {
+        if (r < row && (uint32_t)r % (nt / 32) == warp) {
+          double v = 0.0;
+          for (uint32_t i = lane; i < nt; i += 32) v += rows[r * nt + i];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0) gpart[(uint64_t)row_gate[r] * chunk + set] = v;
+        }
+      }
+      __syncthreads();
+      row = 0;
+    };
+    for (int c0 = (ngates - 1) / kResGates * kResGates; c0 >= 0 && ngates > 0; c0 -= kResGates) {
+      const int cn = min(kResGates, ngates - c0);
+      stage(c0, cn);
+      for (int k = cn; k-- > 0;) {
+        const ResGate g = cg[k];
+        const R* e = cm + 8 * k;
+        ResMat<R> m;  // U^dag
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int d = (j & 1) * 2 + (j >> 1);
+          m.r[j] = e[2 * d], m.i[j] = -e[2 * d + 1];
+        }
+        if (g.ck) {
+          const T* o = ck + ((uint64_t)g.ck * chunk + set) * dim;
+          for (uint32_t i = tid; i < dim; i += nt) s[i] = o[i];
+          __syncthreads();
+        }
+        const uint32_t count = count_of(g);
+        double acc = 0.0;
+        if (g.kind == 2) {
+          for (uint32_t i = tid; i < count; i += nt) {
+            const uint32_t b = res_index(g, i) | g.p0;
+            const T a = s[b], v = l[b];
+            if (g.gen == 4) acc += (double)v.x * (double)a.y - (double)v.y * (double)a.x;
+            s[b] = res_mul<R, T>(m.r[0], m.i[0], a);
+            l[b] = res_mul<R, T>(m.r[0], m.i[0], v);
+          }
+        } else {
+          for (uint32_t i = tid; i < count; i += nt) {
+            const uint32_t b = res_index(g, i);
+            const T a0 = s[b | g.p0], a1 = s[b | g.p1], l0 = l[b | g.p0], l1 = l[b | g.p1];
+            if (g.gen) {  // Im(conj(l0) (G psi)_0 + conj(l1) (G psi)_1)
+              const T u = g.gen == 3 ? a0 : a1, w = g.gen == 3 ? a1 : a0;
+              const double ur = u.x, ui = u.y, wr = w.x, wi = w.y;
+              const double p0r = l0.x, p0i = l0.y, p1r = l1.x, p1i = l1.y;
+              if (g.gen == 1) acc += p0r * ui - p0i * ur + p1r * wi - p1i * wr;
+              else if (g.gen == 2) acc += -p0r * ur - p0i * ui + p1r * wr + p1i * wi;  // (-i a1, i a0)
+              else acc += p0r * ui - p0i * ur - p1r * wi + p1i * wr;
+            }
+            T x = a1, y = a0;
+            if (g.kind == 0) res_pair<R, T>(m, a0, a1, x, y);
+            s[b | g.p0] = x;
+            s[b | g.p1] = y;
+            x = l1, y = l0;
+            if (g.kind == 0) res_pair<R, T>(m, l0, l1, x, y);
+            l[b | g.p0] = x;
+            l[b | g.p1] = y;
+          }
+        }
+        if (g.grad) {
+#pragma unroll
+          for (int r = 0; r < kResRows; ++r)
+            if (r == row) row_gate[r] = c0 + k;
+          rows[row * nt + tid] = acc;
+          ++row;
+        }
+        if (row == kResRows) sum_rows();
+        else __syncthreads();
+      }
+    }
+    if (row) sum_rows();
+  }
+}
+
 // Matrices of the circuit's gates for every parameter set, [gate][set][8].
 // A gate without a parameter has the same one for all sets (made on the host);
 // a parameterised one is formed here from its set's angle, with ket's
@@ -1658,8 +1924,10 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   constexpr int TB = TileCfg<R>::TB;
   const uint64_t dim = uint64_t{1} << n;
   const int T_ = (int)flip.size();
+  const bool resident = method == KETGPU_ADJOINT_AUTO && n <= kResMaxQubits;
   const bool tiled = method == KETGPU_ADJOINT_TILED || method == KETGPU_ADJOINT_TILED_JIT ||
-                     (method == KETGPU_ADJOINT_AUTO && n >= TB);
+                     (method == KETGPU_ADJOINT_AUTO && n >= TB && !resident);
+  const bool ham_inside = resident && dim * (uint64_t)T_ <= kResHamWork;
   // per-block compiled kernels: complex64, asked for, or chosen at sizes
   // where the sweeps take long enough to repay a compile
   const bool want_jit = sizeof(R) == 4 && tiled &&
@@ -1713,11 +1981,21 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   T* const psi = static_cast<T*>(work.p);
   T* const lam = psi + dim * chunk;
   T* const ck = lam + dim * chunk;
-  const int blocks = (int)std::min<uint64_t>(std::max<uint64_t>(1, (dim / 2 + kAThreads - 1) / kAThreads), 592);
+  const int blocks = resident ? 1
+                              : (int)std::min<uint64_t>(std::max<uint64_t>(1, (dim / 2 + kAThreads - 1) / kAThreads), 592);
+  const int ham_blocks = (int)std::min<uint64_t>(std::max<uint64_t>(1, (dim / 2 + kAThreads - 1) / kAThreads), 592);
   // the gates' matrices in the precision their sweep reads
   DevBuf mats((tiled ? sizeof(R) : sizeof(double)) * 8 * chunk * std::max<size_t>(G, 1), dev, st);
   DevBuf hmeta(sizeof(uint64_t) * 2 * T_ + sizeof(int) * T_ + sizeof(double) * T_ + 64, dev, st);
-  {
+  if (ham_inside) {  // the terms as the resident form takes them, i^q folded in
+    static_assert(sizeof(ResTerm) <= 28, "the room of a term");
+    std::vector<ResTerm> h(T_);
+    for (int t = 0; t < T_; ++t) {
+      const int q = phq[t] & 3;
+      h[t] = {(uint32_t)flip[t], (uint32_t)sign[t], q >= 2 ? -coeffs[t] : coeffs[t], (uint32_t)(q & 1), 0};
+    }
+    KB_CUDA(cudaMemcpyAsync(hmeta.p, h.data(), sizeof(ResTerm) * h.size(), cudaMemcpyHostToDevice, st));
+  } else {
     std::vector<char> h(sizeof(uint64_t) * 2 * T_ + sizeof(int) * T_ + sizeof(double) * T_);
     std::memcpy(h.data(), flip.data(), 8 * T_);
     std::memcpy(h.data() + 8 * T_, sign.data(), 8 * T_);
@@ -1731,7 +2009,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   constexpr int kHamPer = 16 / (int)sizeof(T);
   std::unique_ptr<DevBuf> d_ham;
   HamClasses hcls[2] = {};
-  const bool ham_split = T_ <= kHamSmemTerms && dim >= 2 * (uint64_t)kHamPer;
+  const bool ham_split = !ham_inside && T_ <= kHamSmemTerms && dim >= 2 * (uint64_t)kHamPer;
   if (ham_split) {
     std::vector<HamTerm> ht;
     for (int pass = 0; pass < 2; ++pass) {
@@ -1843,6 +2121,32 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   if (G) KB_CUDA(cudaMemcpyAsync(d_agates.p, agates.data(), sizeof(AdjGate) * G, cudaMemcpyHostToDevice, st));
   DevBuf d_params(sizeof(double) * std::max<uint64_t>(chunk * nparams, 1), dev, st);
 
+  // the gates as the resident form takes them
+  std::unique_ptr<DevBuf> d_res;
+  const int res_threads = (int)std::min<uint64_t>(kResThreads, std::max<uint64_t>(32, dim / 4));
+  const size_t res_smem = resident_smem(dim * sizeof(T), res_threads, sizeof(R));
+  if (resident) {
+    std::vector<ResGate> rg(G);
+    for (size_t gi = 0; gi < G; ++gi) {
+      const GateGeom& g = geo[gi];
+      ResGate& r = rg[gi];
+      r = ResGate{};
+      r.p0 = (uint32_t)g.p0;
+      r.p1 = (uint32_t)g.p1;
+      for (int j = 0; j < g.nfixed; ++j) r.fixed[j] = (int16_t)g.fixed[j];
+      r.nfixed = (uint8_t)g.nfixed;
+      r.kind = (uint8_t)g.kind;
+      r.gen = (uint8_t)g.gen;
+      r.grad = g.pslot >= 0;
+      // the state after the last gate of a segment starts the next one
+      const int seg = layer_of[gi] / m;
+      if (gi + 1 < G && layer_of[gi + 1] / m != seg && seg + 1 < n_ckpt) r.ck = seg + 1;
+    }
+    d_res = std::make_unique<DevBuf>(sizeof(ResGate) * std::max<size_t>(G, 1), dev, st);
+    if (G) KB_CUDA(cudaMemcpyAsync(d_res->p, rg.data(), sizeof(ResGate) * G, cudaMemcpyHostToDevice, st));
+    KB_CUDA(cudaFuncSetAttribute(adjoint_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_smem));
+  }
+
   // tiled plan
   TilePlan tp;
   std::vector<cudaKernel_t> jit_fwd, jit_rev;
@@ -1928,7 +2232,8 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
       attr_set[sizeof(R) == 8] = true;
     }
   }
-  const size_t ham_doubles = ham_split ? chunk * 2 * (size_t)ham_ctas : chunk * blocks;
+  const int per_value = ham_inside ? 1 : ham_split ? 2 * ham_ctas : ham_blocks;
+  const size_t ham_doubles = chunk * (size_t)per_value;
   // gradient partials (tiled: per block; per-gate: [gate][set][block]), then
   // the expectation partials
   const size_t grad_region = tiled ? grad_doubles : (size_t)G * chunk * blocks;
@@ -1938,7 +2243,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
   // The pieces of every parameter's gradient, then those of the expectation.
   // (A gate's partials: [gate][set][CTA] tiled within its block, per gate
   // [gate][set][CTA].)
-  const int per_grad = tiled ? gx : blocks, per_value = ham_split ? 2 * ham_ctas : blocks;
+  const int per_grad = tiled ? gx : blocks;
   std::vector<AdjPiece> pieces;
   std::vector<int32_t> first(nparams + 3, 0);
   {
@@ -1999,9 +2304,17 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     T* ground = ck_direct ? ck_at(0) : psi;
     // (a block that runs on part of the tiles leaves the rest of psi as it is)
     if (ck_direct) KB_CUDA(cudaMemsetAsync(psi, 0, dim * sizeof(T) * nb, st));
-    KB_CUDA(cudaMemsetAsync(ground, 0, dim * sizeof(T) * nb, st));
-    ground_batch<R><<<(unsigned)nb, 1, 0, st>>>(ground, dim);
-    count_launch();
+    if (!resident) {
+      KB_CUDA(cudaMemsetAsync(ground, 0, dim * sizeof(T) * nb, st));
+      ground_batch<R><<<(unsigned)nb, 1, 0, st>>>(ground, dim);
+      count_launch();
+    }
+    auto run_resident = [&](int phases) {
+      adjoint_resident<R><<<(unsigned)nb, res_threads, res_smem, st>>>(
+          psi, lam, ck, n, d_res->as<ResGate>(), (int)G, mats.as<double>(), chunk, hmeta.as<ResTerm>(), T_, phases,
+          part.as<double>(), d_ham_part);
+      count_launch();
+    };
     // checkpoint k = the state at the start of layer k*m
     int next_ck = 0;
     auto store_ck = [&]() {
@@ -2009,7 +2322,9 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
                               cudaMemcpyDeviceToDevice, st));
       ++next_ck;
     };
-    if (ck_direct) {
+    if (resident) {
+      run_resident(ham_inside ? kResForward | kResHam | kResReverse : kResForward);
+    } else if (ck_direct) {
       const int B = (int)tp.blocks.size();
       const T* cur = ground;  // where the state lives now
       next_ck = 1;            // checkpoint 0 is the ground state
@@ -2046,10 +2361,10 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
         count_launch();
       }
     }
-    while (next_ck < n_ckpt) store_ck();
+    while (!resident && next_ck < n_ckpt) store_ck();
     KB_CUDA(cudaGetLastError());
     // lambda = H psi and <H>
-    {
+    if (!ham_inside) {
       if (ham_split) {
         KB_CUDA(cudaMemsetAsync(d_ham_part, 0, sizeof(double) * ham_doubles, st));
         const int g0 = hcls[0].end[3], g1 = hcls[1].end[3];
@@ -2067,7 +2382,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
           }
         }
       } else {
-        dim3 grid((unsigned)blocks, (unsigned)nb);
+        dim3 grid((unsigned)ham_blocks, (unsigned)nb);
         ham_apply<R><<<grid, kAThreads, 0, st>>>(psi, lam, dim, d_flip, d_sign, d_q, d_coef, T_,
                                                  d_ham_part);
         count_launch();
@@ -2075,7 +2390,9 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     }
     // reverse sweep; at the last gate (block) of each segment, walking
     // backwards, psi is reset to the checkpoint of the segment's end
-    if (tiled) {
+    if (resident) {
+      if (!ham_inside) run_resident(kResReverse);
+    } else if (tiled) {
       const int B = (int)tp.blocks.size();
       for (int bi = B; bi-- > 0;) {
         const TBlock& b = tp.blocks[bi];

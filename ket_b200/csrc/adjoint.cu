@@ -849,7 +849,9 @@ __device__ __forceinline__ R pair_grad(int gen, const T& a0, const T& a1, const 
 // (A, B) are register slots known at compile time; RC says whether some
 // control bits are register bits (then each j is tested against cm_r).
 // Forward (REV = false) applies U to p; reverse adds the gradient term and
-// applies U^dag to p and q.
+// applies U^dag to p and q.  What a gate is (its generator, a real matrix, a
+// unit entry) is decided once a gate, not once a pair: with the tests inside
+// the unrolled loops four of five instructions of a block were not arithmetic.
 
 template <typename R, int RB, int S, bool REV, bool RC>
 __device__ __forceinline__ R tile_pair(typename C2T<R>::T* p, typename C2T<R>::T* q, const TGate& g,
@@ -867,21 +869,34 @@ __device__ __forceinline__ R tile_pair(typename C2T<R>::T* p, typename C2T<R>::T
       return part;
     }
     const CM2<R> c = load_cm2<R, REV>(m);
-    const bool real = g.real;
-    const int gen = REV ? g.gen : 0;
+    auto body = [&](auto real, auto generator) {
+      constexpr bool REAL = decltype(real)::value;
+      constexpr int GEN = decltype(generator)::value;
 #pragma unroll
-    for (int j = 0; j < (1 << RB); ++j) {
-      if (j & (1 << S)) continue;
-      const int j1 = j | (1 << S);
-      if (RC && (j & g.cm_r) != g.cm_r) continue;
-      if (REV && gen) part += pair_grad<typename C2T<R>::T, R>(gen, p[j], p[j1], q[j], q[j1]);
-      if (real) {
-        mul2_real(c, p[j], p[j1]);
-        if (REV) mul2_real(c, q[j], q[j1]);
-      } else {
-        mul2(c, p[j], p[j1]);
-        if (REV) mul2(c, q[j], q[j1]);
+      for (int j = 0; j < (1 << RB); ++j) {
+        if (j & (1 << S)) continue;
+        const int j1 = j | (1 << S);
+        if (RC && (j & g.cm_r) != g.cm_r) continue;
+        if (REV && GEN) part += pair_grad<typename C2T<R>::T, R>(GEN, p[j], p[j1], q[j], q[j1]);
+        if constexpr (REAL) {
+          mul2_real(c, p[j], p[j1]);
+          if (REV) mul2_real(c, q[j], q[j1]);
+        } else {
+          mul2(c, p[j], p[j1]);
+          if (REV) mul2(c, q[j], q[j1]);
+        }
       }
+    };
+    using std::integral_constant;
+    const int gen = REV ? g.gen : 0;
+    if (g.real) {
+      if (REV && gen == 2) body(std::true_type{}, integral_constant<int, 2>{});
+      else body(std::true_type{}, integral_constant<int, 0>{});  // (only Y's rotations are real)
+    } else {
+      if (REV && gen == 1) body(std::false_type{}, integral_constant<int, 1>{});
+      else if (REV && gen == 2) body(std::false_type{}, integral_constant<int, 2>{});
+      else if (REV && gen) body(std::false_type{}, integral_constant<int, 3>{});
+      else body(std::false_type{}, integral_constant<int, 0>{});
     }
   }
   return part;
@@ -908,19 +923,32 @@ __device__ __forceinline__ R tile_diag_reg(typename C2T<R>::T* p, typename C2T<R
   R part = 0;
   if constexpr (S < RB) {
     const R m0r = m[0], m0i = REV ? -m[1] : m[1], m3r = m[6], m3i = REV ? -m[7] : m[7];
-    const int gen = REV ? g.gen : 0;
+    auto body = [&](auto unit, auto generator) {
+      constexpr bool UNIT = decltype(unit)::value;  // the entry of target bit 0 is 1
+      constexpr int GEN = decltype(generator)::value;
 #pragma unroll
-    for (int j = 0; j < (1 << RB); ++j) {
-      if (RC && (j & g.cm_r) != g.cm_r) continue;
-      const bool bit = (j >> S) & 1;
-      if (REV && gen) {
-        const R im = q[j].x * p[j].y - q[j].y * p[j].x;  // Im(conj(l) a)
-        if (gen == 3) part += bit ? -im : im;
-        else if (bit) part += im;  // P11
+      for (int j = 0; j < (1 << RB); ++j) {
+        if (RC && (j & g.cm_r) != g.cm_r) continue;
+        const bool bit = (j >> S) & 1;
+        if (REV && (GEN == 3 || (GEN == 4 && bit))) {  // Z, P11: Im(conj(l) a)
+          const R im = q[j].x * p[j].y - q[j].y * p[j].x;
+          part += GEN == 3 && bit ? -im : im;
+        }
+        if (UNIT && !bit) continue;
+        cmul(p[j], bit ? m3r : m0r, bit ? m3i : m0i);
+        if (REV) cmul(q[j], bit ? m3r : m0r, bit ? m3i : m0i);
       }
-      if (!bit && g.real) continue;  // times 1
-      cmul(p[j], bit ? m3r : m0r, bit ? m3i : m0i);
-      if (REV) cmul(q[j], bit ? m3r : m0r, bit ? m3i : m0i);
+    };
+    using std::integral_constant;
+    const int gen = REV ? g.gen : 0;
+    if (g.real) {
+      if (REV && gen == 3) body(std::true_type{}, integral_constant<int, 3>{});
+      else if (REV && gen) body(std::true_type{}, integral_constant<int, 4>{});
+      else body(std::true_type{}, integral_constant<int, 0>{});
+    } else {
+      if (REV && gen == 3) body(std::false_type{}, integral_constant<int, 3>{});
+      else if (REV && gen) body(std::false_type{}, integral_constant<int, 4>{});
+      else body(std::false_type{}, integral_constant<int, 0>{});
     }
   }
   return part;
@@ -935,15 +963,21 @@ __device__ __forceinline__ R tile_diag_grp(typename C2T<R>::T* p, typename C2T<R
   const R pr = bit ? m[6] : m[0];
   const R pi = REV ? -(bit ? m[7] : m[1]) : (bit ? m[7] : m[1]);
   const int gen = REV ? g.gen : 0;
+  if (REV && gen) {
+#pragma unroll
+    for (int j = 0; j < (1 << RB); ++j) {
+      if (RC && (j & g.cm_r) != g.cm_r) continue;
+      part += q[j].x * p[j].y - q[j].y * p[j].x;
+    }
+    part = gen == 3 ? (bit ? -part : part) : (bit ? part : R(0));
+  }
+  if (!bit && g.real) return part;  // times 1
 #pragma unroll
   for (int j = 0; j < (1 << RB); ++j) {
     if (RC && (j & g.cm_r) != g.cm_r) continue;
-    if (REV && gen) part += q[j].x * p[j].y - q[j].y * p[j].x;
-    if (!bit && g.real) continue;  // times 1
     cmul(p[j], pr, pi);
     if (REV) cmul(q[j], pr, pi);
   }
-  if (REV && gen) part = gen == 3 ? (bit ? -part : part) : (bit ? part : R(0));
   return part;
 }
 
@@ -990,39 +1024,50 @@ __device__ __forceinline__ R tile_gate(typename C2T<R>::T* p, typename C2T<R>::T
 
 // Forward (REV = false: psi only, gates in order) or reverse (REV = true:
 // psi and lambda, gates in reverse order, gradient partials) over one block,
-// for every tile of every parameter set of the chunk (gridDim.y = set).  One
-// CTA per SM (the register arrays of both states need ~170 registers); the
-// next tile streams into a second buffer with cp.async while the current one
-// is processed.  Shared memory: two tile buffers (psi, then lambda in the
-// reverse), the block's gate records and this set's matrices, then the
-// per-warp gradient sums (reverse).
+// for every tile of every parameter set of the chunk (gridDim.y = set); the
+// complex128 form.  Two CTAs per SM: forwards the next tile streams into a
+// second buffer with cp.async while the current one is processed; in reverse
+// one buffer holds psi and lambda, and one CTA's copies run under the other's
+// gates.  Shared memory: the tile buffers, the block's gate records and this
+// set's matrices, then the gradient sums (reverse), eight lanes a warp.
+// What bounds it is instruction issue, half busy with two CTAs (a third with
+// one): of a gate's instructions a quarter is FP64 arithmetic, the rest moves of
+// 64 registers between the gate bodies and the bodies' selection.  20 qubits, 8 sets, 4 layers:
+// 8.5 -> 6.0 ms a call against one CTA with two buffers, full warp sums a
+// gradient and a gate's tests inside its loops.
 template <typename R, bool REV>
-__global__ void __launch_bounds__(kTileThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 2)
     tile_sweep(typename C2T<R>::T* __restrict__ psi, typename C2T<R>::T* __restrict__ lam, uint64_t dim,
                TileGeom tg, const TGate* __restrict__ gates, int ngates, const TPhase* __restrict__ phases,
                int nph, const R* __restrict__ mats, uint64_t mat_stride, int ngrad, double* __restrict__ partial) {
   using T = typename C2T<R>::T;
   constexpr int TB = TileCfg<R>::TB, RB = TileCfg<R>::RB, NR = 1 << RB, TILE = 1 << TB;
-  constexpr int BUF = (REV ? 2 : 1) * TILE;  // elements per buffer
   extern __shared__ __align__(16) unsigned char tsm[];
-  T* bufs = reinterpret_cast<T*>(tsm);
-  TGate* sg = reinterpret_cast<TGate*>(tsm + 2 * BUF * sizeof(T));
+  T* bufs = reinterpret_cast<T*>(tsm);  // two of psi, or one of psi and one of lambda
+  TGate* sg = reinterpret_cast<TGate*>(tsm + 2 * TILE * sizeof(T));
   R* smat = reinterpret_cast<R*>(sg + ngates);
-  double* acc = reinterpret_cast<double*>(smat + 8 * (size_t)ngates);  // [warp][ngrad]
-  __shared__ uint64_t off_lo[64], off_hi[64];
+  double* acc = reinterpret_cast<double*>(smat + 8 * (size_t)ngates);  // [gradient][warp][8 lanes]
+  // offset of tile element tid + 256 r: off[tid] + off[256 + r]
+  __shared__ uint64_t off[kTileThreads + NR];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int set = blockIdx.y;
   T* s = psi + (uint64_t)set * dim;
   T* l = REV ? lam + (uint64_t)set * dim : nullptr;
 
-  if (tid < 128) {
-    const int half = tid >> 6, e = tid & 63;
-    uint64_t off = 0;
-    for (int b = 0; b < 6; ++b) {
-      const int tb = 6 * half + b;
-      if (tb < TB && ((e >> b) & 1)) off |= uint64_t{1} << tg.pos[tb];
+  static_assert(kTileThreads << RB == TILE && kTileThreads == 256, "tile elements a thread");
+  {
+    uint64_t o = 0;
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+      if ((tid >> b) & 1) o |= uint64_t{1} << tg.pos[b];
+    off[tid] = o;
+    if (tid < NR) {
+      o = 0;
+#pragma unroll
+      for (int b = 0; b < RB; ++b)
+        if ((tid >> b) & 1) o |= uint64_t{1} << tg.pos[8 + b];
+      off[kTileThreads + tid] = o;
     }
-    (half ? off_hi : off_lo)[e] = off;
   }
   for (int i = tid; i < ngates; i += kTileThreads) {
     const TGate g = gates[i];
@@ -1032,7 +1077,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     for (int k = 0; k < 8; ++k) smat[8 * i + k] = src[k];
   }
   if (REV)
-    for (int i = tid; i < kTileWarps * ngrad; i += kTileThreads) acc[i] = 0.0;
+    for (int i = tid; i < 8 * kTileWarps * ngrad; i += kTileThreads) acc[i] = 0.0;
   __syncthreads();
 
   auto tile_base = [&](uint64_t t) {
@@ -1044,43 +1089,44 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     }
     return base;
   };
-  auto prefetch = [&](uint64_t t, T* buf) {
-    const uint64_t base = tile_base(t);
-#pragma unroll 2
+  const int ptid = tphys<R>(tid);
+  auto prefetch = [&](uint64_t at, T* buf) {
+#pragma unroll
     for (int r = 0; r < NR; ++r) {
-      const int e = tid + r * kTileThreads;
-      const uint64_t o = base + (off_lo[e & 63] | off_hi[e >> 6]);
-      tile_cp_async(buf + tphys<R>(e), s + o);
-      if (REV) tile_cp_async(buf + TILE + tphys<R>(e), l + o);
+      const uint64_t o = at + off[kTileThreads + r];
+      T* d = buf + (ptid ^ tphys<R>(r * kTileThreads));
+      tile_cp_async(d, s + o);
+      if (REV) tile_cp_async(d + TILE, l + o);
     }
   };
 
   int cur = 0;
-  if (blockIdx.x < tg.n_tiles) prefetch(blockIdx.x, bufs);
+  uint64_t at = 0, next_at = 0;  // where this thread's first element of a tile is
+  if (blockIdx.x < tg.n_tiles) {
+    next_at = tile_base(blockIdx.x) + off[tid];
+    if (!REV) prefetch(next_at, bufs);
+  }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   for (uint64_t t = blockIdx.x; t < tg.n_tiles; t += gridDim.x) {
-    T* sp = bufs + cur * BUF;
-    T* sl = sp + TILE;
-    if (t + gridDim.x < tg.n_tiles) prefetch(t + gridDim.x, bufs + (cur ^ 1) * BUF);
+    T* sp = REV ? bufs : bufs + cur * TILE;
+    T* sl = bufs + TILE;  // (reverse)
+    at = next_at;
+    if (t + gridDim.x < tg.n_tiles) next_at = tile_base(t + gridDim.x) + off[tid];
+    if (REV) prefetch(at, bufs);
+    else if (t + gridDim.x < tg.n_tiles) prefetch(next_at, bufs + (cur ^ 1) * TILE);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this tile's copies are done
+    if (REV) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    else asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this tile's copies are done
     __syncthreads();
     for (int k = 0; k < nph; ++k) {
       const TPhase P = phases[REV ? nph - 1 - k : k];
-      // group bits of this thread: the non-register tile bits, ascending
-      int rmask = 0;
-#pragma unroll
-      for (int b = 0; b < RB; ++b) rmask |= 1 << P.r[b];
-      int gbase = 0;
-      {
-        int kk = 0;
-#pragma unroll
-        for (int b = 0; b < TB; ++b)
-          if (!((rmask >> b) & 1)) {
-            gbase |= ((tid >> kk) & 1) << b;
-            ++kk;
-          }
-      }
+      // group bits of this thread: tid with zeros at the register bits, from
+      // the lowest up
+      static_assert(RB == 3, "three register bits");
+      const int r_lo = min(min(P.r[0], P.r[1]), P.r[2]), r_hi = max(max(P.r[0], P.r[1]), P.r[2]);
+      const int r_mid = P.r[0] + P.r[1] + P.r[2] - r_lo - r_hi;
+      auto open = [](int x, int b) { return ((x >> b) << (b + 1)) | (x & ((1 << b) - 1)); };
+      const int gbase = open(open(open(tid, r_lo), r_mid), r_hi);
       // the swizzle is XOR-linear and gbase, rdep(j) have disjoint bits, so
       // the address of element j is tphys(gbase) ^ tphys(rdep(j))
       const int pg = tphys<R>(gbase);
@@ -1104,8 +1150,8 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         if (REV && g.grad >= 0) {
           double v = (double)part;
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) acc[warp * ngrad + g.grad] += v;
+          for (int o = 16; o > 4; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane < 8) acc[(g.grad * kTileWarps + warp) * 8 + lane] += v;
         }
       }
       {
@@ -1130,27 +1176,28 @@ __global__ void __launch_bounds__(kTileThreads, 1)
       __syncthreads();
     }
     {
-      const uint64_t base = tile_base(t);
-      const volatile uint64_t* vlo = off_lo;
-      const volatile uint64_t* vhi = off_hi;
-#pragma unroll 2
+      const volatile uint64_t* voff = off;
+#pragma unroll
       for (int r = 0; r < NR; ++r) {
-        const int e = tid + r * kTileThreads;
-        const uint64_t o = base + (vlo[e & 63] | vhi[e >> 6]);
-        s[o] = sp[tphys<R>(e)];
-        if (REV) l[o] = sl[tphys<R>(e)];
+        const uint64_t o = at + voff[kTileThreads + r];
+        const int e = ptid ^ tphys<R>(r * kTileThreads);
+        s[o] = sp[e];
+        if (REV) l[o] = sl[e];
       }
     }
     __syncthreads();
     cur ^= 1;
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (REV)
-    for (int g = tid; g < ngrad; g += kTileThreads) {
-      double v = 0.0;
-      for (int w = 0; w < kTileWarps; ++w) v += acc[w * ngrad + g];
-      partial[((uint64_t)set * ngrad + g) * gridDim.x + blockIdx.x] = v;
+  if (REV) {
+    __syncthreads();
+    for (int g = warp; g < ngrad; g += kTileWarps) {
+      double v = acc[g * 64 + lane] + acc[g * 64 + 32 + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) partial[((uint64_t)set * ngrad + g) * gridDim.x + blockIdx.x] = v;
     }
+  }
 }
 
 
@@ -1861,9 +1908,11 @@ size_t jit_smem(bool rev, int ngates, int ngrad) {
 template <typename R>
 size_t tile_smem(bool rev, int ngates, int ngrad) {
   using T = typename C2T<R>::T;
-  const size_t tiles = (rev ? 4 : 2) * (size_t{1} << TileCfg<R>::TB) * sizeof(T);
-  const size_t per_gate = sizeof(R) == 4 ? 16 * sizeof(f2) + sizeof(TGate) : sizeof(TGate) + 8 * sizeof(R);
-  return tiles + (size_t)ngates * per_gate + (rev ? (size_t)kTileWarps * ngrad * 8 : 0);
+  const size_t tile = (size_t{1} << TileCfg<R>::TB) * sizeof(T);
+  if (sizeof(R) == 8)
+    return 2 * tile + (size_t)ngates * (sizeof(TGate) + 8 * sizeof(R)) + (rev ? (size_t)kTileWarps * ngrad * 64 : 0);
+  return (rev ? 4 : 2) * tile + (size_t)ngates * (16 * sizeof(f2) + sizeof(TGate)) +
+         (rev ? (size_t)kTileWarps * ngrad * 8 : 0);
 }
 
 std::atomic<uint64_t> g_jit_launches{0};

@@ -31,6 +31,11 @@
 //   TMEM) back to global memory, straight from registers or through shared
 //   memory.  Every mbarrier wait is bounded; on timeout the kernel raises an
 //   error flag, drains its copies, frees its tensor memory and returns.
+//
+// A launch overlaps the pass before it (programmatic dependent launch): its
+// CTAs take the SMs as the other's leave, and set up (barriers, tensor memory,
+// B images: plan tables, which no pass writes) before they wait for its
+// end.  22-qubit brick wall 536 -> 431 us, 26 qubits 5.03 -> 4.88 ms.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_fp16.h>
@@ -92,6 +97,12 @@ struct TcCfg {
   static_assert(SLOTS >= (HALVES ? 2 : 3), "shared memory budget");
   static_assert(!HALVES || HSLOTS >= 4, "shared memory budget");
   static_assert(SMEM <= (size_t)kSmemBudget + 1024, "shared memory budget");
+  // k = 6 staged stores: the output goes through a buffer of half a tile
+  // behind the slots, which the converters can then free (a slot that also
+  // carries its tile's output is one of two: 28 qubits, block 0-5, 845 us a
+  // pass, against 695)
+  static constexpr bool HALF_OUT = KQ == 6;
+  static_assert(!HALF_OUT || (size_t)SLOTS * RAW_BYTES + HALF_BYTES <= STAGE, "shared memory budget");
 };
 
 struct TcGeom {
@@ -129,6 +140,11 @@ struct TcGeom {
   // byte offsets
   uint64_t chunk_g[32];
   uint32_t chunk_s_in[32], chunk_s_out[32];
+  // k = 6 staged stores: the same of a half tile, the tile less the tile bit
+  // top_bit of its highest target (state and staging offsets)
+  int top_bit;
+  uint64_t half_g[16];
+  uint32_t half_s[16];
 };
 
 // Output staging when qubit 0 is a group bit: amplitudes e and e+1 (rows
@@ -180,6 +196,11 @@ __host__ __device__ inline void amp_offsets(const TcGeom& g, int tb, int dim, in
   const int row = q0_group ? ((grp >> 1) | ((grp & 1) << (kGroupBits - 1))) : grp;
   *goff = off;
   *soff = (out_layout && q0_group) ? pair_slot_offset(row, comb, dim) : sw128_offset(row, 2 * comb, 128);
+}
+
+// Tile amplitude of element e of a half tile (top_bit clear).
+__host__ __device__ inline int half_element(const TcGeom& g, int e) {
+  return ((e >> g.top_bit) << (g.top_bit + 1)) | (e & ((1 << g.top_bit) - 1));
 }
 
 // Packed FP32 pairs (sm_100 f32x2 instructions: two FP32 operations each).
@@ -335,7 +356,10 @@ constexpr int kScaleRing = 4;  // row scales in flight (see the converters)
 // NORM: the epilogue also sums |out|^2 into g.norm_out (the plan's last
 // block before its norm restore); a separate instantiation, so the common
 // one carries none of it.
-template <int KQ, bool NORM>
+// DIRECT: the epilogue stores from registers (else through shared memory;
+// staged blocks never take the tensor copy).  One instantiation each: with
+// both in one kernel the direct stores of k = 6 took 194 us a pass at 26 qubits, not 186.
+template <int KQ, bool NORM, bool DIRECT>
 __global__ void __launch_bounds__(kTcThreads, 1)
     fused_tc_kernel(float2* __restrict__ s, TcGeom g, const uint32_t* __restrict__ bimg,
                     const __grid_constant__ CUtensorMap tmap) {
@@ -378,8 +402,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     for (int i = 0; i < SB; ++i) {
-      mbar_init(smem_u32(&bar_full[i]), g.tma_dims ? 1 : kProducers + 1);
-      mbar_init(smem_u32(&bar_free[i]), g.direct ? kConverters : kEpilogue);
+      mbar_init(smem_u32(&bar_full[i]), DIRECT && g.tma_dims ? 1 : kProducers + 1);
+      mbar_init(smem_u32(&bar_free[i]), DIRECT || Cfg::HALF_OUT ? kConverters : kEpilogue);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bar_a_ready[i]), kConverters);
@@ -468,7 +492,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     return b;
   };
 
-  if (warp < 4 && g.tma_dims) {
+  if (DIRECT && warp < 4 && g.tma_dims) {
     // ------------------------------------------ producer, tensor-copy form
     // One thread fetches each tile with one tiled tensor copy (k = 6: two,
     // half q = 2j + h of tile j -- h the highest target's bit -- into slot
@@ -542,7 +566,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // staging row is the rotated one); otherwise lane t carries staging row t.
     const int q = warp & 3;
     const int lane_row = 32 * q + lane;
-    const int row = g.direct ? ((lane_row >> 1) | ((lane_row & 1) << (kGroupBits - 1))) : lane_row;
+    const int row = DIRECT ? ((lane_row >> 1) | ((lane_row & 1) << (kGroupBits - 1))) : lane_row;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
     const int sb = (int)bimg[2 * Cfg::B_BYTES / 4];
     // tensor-copy images: byte offset of this lane's group in the tile (or
@@ -645,7 +669,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           tmem_st16(areg + (uint32_t)(part * 16), hi);
           tmem_st16(areg + (uint32_t)(K / 2 + part * 16), lo);
         }
-        if (g.direct) {  // nothing else reads the images
+        if (DIRECT || Cfg::HALF_OUT) {  // nothing else reads the images
           arrive(&bar_free[slot0]);
           if (slot1 != slot0) arrive(&bar_free[slot1]);
         }
@@ -654,8 +678,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         arrive(&bar_a_ready[j & 1]);
       }
     };
-    if (g.tma_dims) convert_tiles(std::true_type{});
-    else convert_tiles(std::false_type{});
+    if constexpr (DIRECT) {
+      if (g.tma_dims) convert_tiles(std::true_type{});
+      else convert_tiles(std::false_type{});
+    } else {
+      convert_tiles(std::false_type{});
+    }
   } else if (warp < 12) {
     // ------------------------------------------------------------- epilogue
     const int t = tid - 256;
@@ -671,7 +699,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       *unscale = __int_as_float((127 - (int)row_exp[j % kScaleRing][row]) << 23);
       return true;
     };
-    if (g.direct) {
+    if constexpr (DIRECT) {
       // TMEM lane = group `row`; the lanes of a warp vary the five lowest
       // group bits, which include qubits 0 and 1, so each run of lanes
       // fills whole 32-byte sectors.
@@ -703,6 +731,65 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         tc_fence_before();
         arrive(&bar_acc_free[j & 1]);
+      }
+    } else if constexpr (Cfg::HALF_OUT) {
+      // The accumulator half by half (by the highest target) through the half
+      // tile behind the slots.
+      constexpr int HD = DIM / 2;
+      unsigned char* out = raw + S * Cfg::RAW_BYTES;
+      uint64_t g0;
+      uint32_t s0;
+      amp_offsets(g, Cfg::TB, HD, half_element(g, 2 * t), true, &g0, &s0);
+      for (uint64_t j = 0; j < count; ++j) {
+        float us;
+        // the tile before has been read by all; they leave together on a timeout
+        int ok = tile_ready(j, &us);
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.s32 q, %0, 0;\n\t"
+            "bar.red.and.pred p, 1, %1, q;\n\t"
+            "selp.s32 %0, 1, 0, p;\n\t}"
+            : "+r"(ok)
+            : "n"(kEpilogue)
+            : "memory");
+        if (!ok) break;
+        const uint32_t acc = acc_lane + (uint32_t)((j & 1) * N);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h) asm volatile("bar.sync 1, %0;" ::"n"(kEpilogue) : "memory");  // the lower half has been read
+#pragma unroll
+          for (int part = 0; part < N / 32; ++part) {
+            float v[16];
+            tmem_ld<16>(acc + (uint32_t)(h * N / 2 + part * 16), v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              v[i] *= us;
+              if constexpr (NORM) nacc = fma((double)v[i], (double)v[i], nacc);
+            }
+            if (q0_group) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<float2*>(out + pair_slot_offset(row, part * 8 + i, HD)) =
+                    make_float2(v[2 * i], v[2 * i + 1]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(out + sw128_offset(row, part * 16 + 4 * i, 128)) =
+                    make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+          }
+          if (h == 1) {
+            tc_fence_before();
+            arrive(&bar_acc_free[j & 1]);
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(kEpilogue) : "memory");
+          float2* dst = s + base_ring[j % R] + (h ? g.cdep[HD] : 0);
+#pragma unroll
+          for (int i = 0; i < CPT / 2; ++i)
+            *reinterpret_cast<float4*>(dst + (g0 ^ g.half_g[i])) =
+                *reinterpret_cast<const float4*>(out + (s0 ^ g.half_s[i]));
+        }
       }
     } else {
       uint64_t g0;
@@ -973,6 +1060,12 @@ void tile_geometry(int n, const Pass& p, uint64_t active, TcGeom& g) {
     g.chunk_s_in[i] = si;
     g.chunk_s_out[i] = so;
   }
+  if constexpr (Cfg::HALF_OUT) {
+    for (int b = 0; b < Cfg::TB; ++b)
+      if (g.is_target[b]) g.top_bit = b;
+    for (int i = 0; i < CPT / 2; ++i)
+      amp_offsets(g, Cfg::TB, Cfg::DIM / 2, half_element(g, 256 * i), true, &g.half_g[i], &g.half_s[i]);
+  }
 }
 
 // The half tile of a k = 6 block (host only): the tile less its highest
@@ -1078,10 +1171,9 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   }
   static int attr_done[64] = {0};
   if (st.device >= 0 && st.device < 64 && !(attr_done[st.device] & (1 << KQ))) {
-    KB_CUDA(cudaFuncSetAttribute(fused_tc_kernel<KQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Cfg::SMEM));
-    KB_CUDA(cudaFuncSetAttribute(fused_tc_kernel<KQ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Cfg::SMEM));
+    for (auto* f : {fused_tc_kernel<KQ, false, false>, fused_tc_kernel<KQ, false, true>,
+                    fused_tc_kernel<KQ, true, false>, fused_tc_kernel<KQ, true, true>})
+      KB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
     attr_done[st.device] |= 1 << KQ;
   }
   static int sms[64] = {0};
@@ -1099,8 +1191,10 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  KB_CUDA(cudaLaunchKernelEx(&cfg, norm_partials ? fused_tc_kernel<KQ, true> : fused_tc_kernel<KQ, false>,
-                             static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image), tmap));
+  auto* const kernel = norm_partials ? (g.direct ? fused_tc_kernel<KQ, true, true> : fused_tc_kernel<KQ, true, false>)
+                                     : (g.direct ? fused_tc_kernel<KQ, false, true> : fused_tc_kernel<KQ, false, false>);
+  KB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image),
+                             tmap));
   count_launch();
 }
 

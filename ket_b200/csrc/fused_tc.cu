@@ -155,6 +155,13 @@ __host__ __device__ inline uint32_t pair_slot_offset(int row, int comb, int dim)
   return (uint32_t)(((row & 63) * dim + (comb ^ (row & 7))) * 16 + 8 * (row >> 6));
 }
 
+// Byte offset of tile amplitude e in an image in natural tile order, under the
+// 128-byte swizzle (as a tensor copy writes it).  XOR-linear in e.  Directly
+// stored blocks use it with cp.async too: a warp's 16-byte copies fill 128-byte rows (8-byte
+// copies into A rows 233 us a pass at 26 qubits, block 5 9 11 13 17 25; 182
+// now; 16-byte copies scattered over rows of pairs 396).
+__host__ __device__ inline uint32_t natural_offset(int e) { return (uint32_t)(8 * e) ^ (uint32_t)(e & 0x70); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -351,6 +358,8 @@ __host__ __device__ constexpr uint32_t f16_idesc() {
 // stage to stage, so loads of later tiles, the split of tile j+1, the MMAs of
 // tile j and the drain of tile j-1 proceed concurrently.
 constexpr int kProducers = 128, kConverters = 128, kEpilogue = 128;
+// Staging images: A rows (staged stores), the tile in natural order, two halves of it.
+enum { kRows, kTile, kHalves };
 constexpr int kScaleRing = 4;  // row scales in flight (see the converters)
 
 // NORM: the epilogue also sums |out|^2 into g.norm_out (the plan's last
@@ -370,8 +379,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   constexpr int K = Cfg::K;
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   // [B hi][B lo][staging images]; a staging image receives the raw tile (in
-  // the A layout with cp.async, in natural tile order with a tensor copy), is
-  // read by the converters, and with staged stores then carries the
+  // the A layout, or with direct stores in natural tile order), is read by the
+  // converters, and with staged stores then carries the
   // accumulator back out.
   unsigned char* base_ptr = smem_dyn + ((1024 - (smem_u32(smem_dyn) & 1023)) & 1023);
   unsigned char* b_hi = base_ptr;
@@ -529,6 +538,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint64_t g0;
     uint32_t s0;
     amp_offsets(g, Cfg::TB, DIM, 2 * tid, false, &g0, &s0);
+    if (DIRECT) s0 = natural_offset(2 * tid);
     for (uint64_t j = 0; j < count; ++j) {
       const int slot = (int)(j % S);
       if (j >= (uint64_t)S && !wait(&bar_free[slot], (uint32_t)(((j / S) - 1) & 1))) break;
@@ -539,7 +549,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int i = 0; i < CPT; ++i) {
         const uint64_t go = g0 ^ g.chunk_g[i];
         const uint32_t so = s0 ^ g.chunk_s_in[i];
-        if (q0_group) {
+        if (!DIRECT && q0_group) {
           cp_async8(dst + so, src + go);
           cp_async8(dst + so + pair_step, src + go + 1);
         } else {
@@ -562,15 +572,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // fp16 per 32-bit column (re low, im high), into the A region of tile
     // parity j%2 once the MMAs of tile j-2 have released it; s + sb goes to
     // the epilogue through row_exp.
-    // In the direct-store mode TMEM lane t carries group t (its cp.async
-    // staging row is the rotated one); otherwise lane t carries staging row t.
+    // With direct stores TMEM lane t carries group t, else staging row t.
     const int q = warp & 3;
     const int lane_row = 32 * q + lane;
-    const int row = DIRECT ? ((lane_row >> 1) | ((lane_row & 1) << (kGroupBits - 1))) : lane_row;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
     const int sb = (int)bimg[2 * Cfg::B_BYTES / 4];
-    // tensor-copy images: byte offset of this lane's group in the tile (or
-    // in a half tile)
+    // images in natural tile order: byte offset of this lane's group in the
+    // tile (or in a half tile)
     uint32_t gtile = 0;
     if (Cfg::HALVES && g.tma_dims) {
 #pragma unroll
@@ -588,13 +596,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // amplitude's swizzled offset is the swizzled group offset XOR the
     // swizzled combination offset (ctile holds the latter).
     const uint32_t gsw = gtile ^ ((gtile >> 3) & 0x70u);
-    // One loop per producer form, chosen once: with the form a compile-time
+    // One loop per image form, chosen once: with the form a compile-time
     // constant, every staging read of a tile has a constant offset and the
     // reads issue back to back (a per-read branch on the form kept only two
     // in flight, each paying the full shared-memory latency).
     auto convert_tiles = [&](auto form) {
-      constexpr bool TMA = decltype(form)::value;
-      constexpr bool HALF = TMA && Cfg::HALVES;
+      constexpr bool ROWS = decltype(form)::value == kRows;
+      constexpr bool HALF = decltype(form)::value == kHalves;
       for (uint64_t j = 0; j < count; ++j) {
         // the tile's images: one, or (k = 6 tensor copy) its two halves
         int slot0, slot1;
@@ -615,8 +623,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const unsigned char* img1 = raw + slot1 * Cfg::HALF_BYTES;
         // amplitudes 2i and 2i+1 of this row as (re, im, re, im)
         auto amp_pair = [&](int i) -> float4 {
-          if constexpr (!TMA) {
-            return *reinterpret_cast<const float4*>(img0 + sw128_offset(row, 4 * i, 128));
+          if constexpr (ROWS) {
+            return *reinterpret_cast<const float4*>(img0 + sw128_offset(lane_row, 4 * i, 128));
           } else {
             float2 v[2];
 #pragma unroll
@@ -678,11 +686,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         arrive(&bar_a_ready[j & 1]);
       }
     };
-    if constexpr (DIRECT) {
-      if (g.tma_dims) convert_tiles(std::true_type{});
-      else convert_tiles(std::false_type{});
+    using std::integral_constant;
+    if constexpr (!DIRECT) {
+      convert_tiles(integral_constant<int, kRows>{});
+    } else if constexpr (Cfg::HALVES) {
+      if (g.tma_dims) convert_tiles(integral_constant<int, kHalves>{});
+      else convert_tiles(integral_constant<int, kTile>{});
     } else {
-      convert_tiles(std::false_type{});
+      convert_tiles(integral_constant<int, kTile>{});
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------- epilogue
@@ -1157,8 +1168,10 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   } else {
     g.tma_dims = tma_wanted(g, p, Cfg::TB) ? encode_tile_map(st, g, Cfg::TB, &tmap) : 0;
   }
-  if (g.tma_dims && !g.half) {
-    g.direct = 1;
+  if (g.tma_dims) g.direct = 1;
+  if (g.direct && !g.half) {  // images in natural tile order
+    if (!g.tma_dims)
+      for (int i = 0; i < Cfg::TILE / 2 / kProducers; ++i) g.chunk_s_in[i] = natural_offset(256 * i);
     for (int c = 0; c < Cfg::DIM; ++c) {
       uint32_t off = 0;
       for (int b = 0, jb = 0; jb < Cfg::TB; ++jb)

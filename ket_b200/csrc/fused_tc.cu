@@ -112,6 +112,7 @@ struct TcGeom {
   int nh;             // positions above the low run that are zero in a tile
   unsigned char hpos[40];  // base, ascending: tile qubits and inactive ones
   int direct;         // the epilogue stores from registers (see launch_fused_tc)
+  int natural;        // staged: input images in natural tile order (see natural_reads)
   // Tensor-copy producer (tma_dims > 0, see launch_tc): dimension i of the
   // tensor map starts at qubit tma_start[i]; a tile's coordinate in it is
   // (base >> tma_start[i]) & tma_mask[i].  ctile[c] = swizzled byte offset of
@@ -358,8 +359,9 @@ __host__ __device__ constexpr uint32_t f16_idesc() {
 // stage to stage, so loads of later tiles, the split of tile j+1, the MMAs of
 // tile j and the drain of tile j-1 proceed concurrently.
 constexpr int kProducers = 128, kConverters = 128, kEpilogue = 128;
-// Staging images: A rows (staged stores), the tile in natural order, two halves of it.
-enum { kRows, kTile, kHalves };
+// Staging images: A rows, the tile in natural order (read by amplitude, or by
+// pairs when qubit 0 is a target), two halves of it.
+enum { kRows, kTile, kTilePairs, kHalves };
 constexpr int kScaleRing = 4;  // row scales in flight (see the converters)
 
 // NORM: the epilogue also sums |out|^2 into g.norm_out (the plan's last
@@ -379,9 +381,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   constexpr int K = Cfg::K;
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   // [B hi][B lo][staging images]; a staging image receives the raw tile (in
-  // the A layout, or with direct stores in natural tile order), is read by the
-  // converters, and with staged stores then carries the
-  // accumulator back out.
+  // the A layout or in natural tile order), is read by the converters, and
+  // with staged stores of k < 6 then carries the accumulator back out.
   unsigned char* base_ptr = smem_dyn + ((1024 - (smem_u32(smem_dyn) & 1023)) & 1023);
   unsigned char* b_hi = base_ptr;
   unsigned char* b_lo = b_hi + Cfg::B_BYTES;
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint64_t g0;
     uint32_t s0;
     amp_offsets(g, Cfg::TB, DIM, 2 * tid, false, &g0, &s0);
-    if (DIRECT) s0 = natural_offset(2 * tid);
+    if (DIRECT || g.natural) s0 = natural_offset(2 * tid);
     for (uint64_t j = 0; j < count; ++j) {
       const int slot = (int)(j % S);
       if (j >= (uint64_t)S && !wait(&bar_free[slot], (uint32_t)(((j / S) - 1) & 1))) break;
@@ -625,6 +626,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         auto amp_pair = [&](int i) -> float4 {
           if constexpr (ROWS) {
             return *reinterpret_cast<const float4*>(img0 + sw128_offset(lane_row, 4 * i, 128));
+          } else if constexpr (decltype(form)::value == kTilePairs) {
+            return *reinterpret_cast<const float4*>(img0 + (g.ctile[2 * i] ^ gsw));
           } else {
             float2 v[2];
 #pragma unroll
@@ -688,7 +691,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     };
     using std::integral_constant;
     if constexpr (!DIRECT) {
-      convert_tiles(integral_constant<int, kRows>{});
+      if (g.natural) convert_tiles(integral_constant<int, kTilePairs>{});
+      else convert_tiles(integral_constant<int, kRows>{});
     } else if constexpr (Cfg::HALVES) {
       if (g.tma_dims) convert_tiles(integral_constant<int, kHalves>{});
       else convert_tiles(integral_constant<int, kTile>{});
@@ -1003,6 +1007,32 @@ int tma_read_wavefronts(const TcGeom& g, int tb) {
   return 32 >> rank;
 }
 
+// Whether a staged block on qubit 0 takes input images in natural tile order:
+// when the converters read them as fast as A rows (a warp's 32 groups over all
+// eight 16-byte chunks of a 128-byte row).  A warp's copies then fill whole
+// rows; into A rows they scatter: 26 qubits, block 0 4 6 9 11 25 181 us a pass
+// against 236-289, 0 3 4 13 25 216 against 249-325.  Block 0-5, whose lanes are 512
+// bytes apart, keeps A rows.
+bool natural_reads(const TcGeom& g, int tb) {
+  if (!g.is_target[0]) return false;
+  uint32_t lanes[5];
+  int n = 0;
+  for (int j = 0; j < tb && n < 5; ++j)
+    if (!g.is_target[j]) lanes[n++] = (natural_offset(1 << j) >> 4) & 7;
+  int rank = 0;
+  for (int bit = 0; bit < 3; ++bit) {
+    int pivot = -1;
+    for (int i = rank; i < n && pivot < 0; ++i)
+      if ((lanes[i] >> bit) & 1) pivot = i;
+    if (pivot < 0) continue;
+    std::swap(lanes[pivot], lanes[rank]);
+    for (int i = 0; i < n; ++i)
+      if (i != rank && ((lanes[i] >> bit) & 1)) lanes[i] ^= lanes[rank];
+    ++rank;
+  }
+  return rank == 3;
+}
+
 // Whether a block takes the tensor-copy producer (before the tile-run limits).
 bool tma_wanted(const TcGeom& g, const Pass& p, int tb) {
   const int lowest = p.qubits[0];
@@ -1169,7 +1199,8 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
     g.tma_dims = tma_wanted(g, p, Cfg::TB) ? encode_tile_map(st, g, Cfg::TB, &tmap) : 0;
   }
   if (g.tma_dims) g.direct = 1;
-  if (g.direct && !g.half) {  // images in natural tile order
+  g.natural = !g.direct && natural_reads(g, Cfg::TB);
+  if ((g.direct && !g.half) || g.natural) {  // images in natural tile order
     if (!g.tma_dims)
       for (int i = 0; i < Cfg::TILE / 2 / kProducers; ++i) g.chunk_s_in[i] = natural_offset(256 * i);
     for (int c = 0; c < Cfg::DIM; ++c) {

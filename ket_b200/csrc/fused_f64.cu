@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(F64Cfg<KQ>::THREADS, 1)
 }
 
 template <int KQ>
-void launch_k(const State& st, const F64Geom& g, const double2* mat_t) {
+void launch_k(const State& st, const F64Geom& g, const double2* mat_t, bool overlap) {
   using Cfg = F64Cfg<KQ>;
   const size_t smem = sizeof(double2) * Cfg::TEAMS * kStages * ((size_t)1 << g.tb);
   static bool attr[64] = {false};
@@ -269,7 +269,7 @@ void launch_k(const State& st, const F64Geom& g, const double2* mat_t) {
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   KB_CUDA(cudaLaunchKernelEx(&cfg, fused_f64_kernel<KQ>, static_cast<double2*>(st.amps), g, mat_t));
   count_launch();
 }
@@ -279,7 +279,7 @@ void launch_k(const State& st, const F64Geom& g, const double2* mat_t) {
 // A k-qubit complex128 block needs whole 8-group column blocks.
 bool f64_supported(int n, int k) { return k >= 3 && k <= 6 && n >= k + 3; }
 
-void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_t active) {
+void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_t active, bool overlap) {
   F64Geom g{};
   g.k = p.k;
   // 1024-amplitude tiles, fewer amplitudes where that leaves teams without a
@@ -313,10 +313,10 @@ void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_
   g.n_tiles = uint64_t{1} << (__builtin_popcountll(span) - g.tb);
   const double2* m = static_cast<const double2*>(mat_t);
   switch (p.k) {
-    case 3: launch_k<3>(st, g, m); break;
-    case 4: launch_k<4>(st, g, m); break;
-    case 5: launch_k<5>(st, g, m); break;
-    case 6: launch_k<6>(st, g, m); break;
+    case 3: launch_k<3>(st, g, m, overlap); break;
+    case 4: launch_k<4>(st, g, m, overlap); break;
+    case 5: launch_k<5>(st, g, m, overlap); break;
+    case 6: launch_k<6>(st, g, m, overlap); break;
     default: fail(KETGPU_ERR_LOGIC, "launch_fused_f64: unsupported block size");
   }
 }

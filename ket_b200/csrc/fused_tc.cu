@@ -1182,7 +1182,8 @@ int* error_flag() {
 }
 
 template <int KQ>
-void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, uint64_t active) {
+void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+               bool overlap) {
   using Cfg = TcCfg<KQ>;
   TcGeom g;
   tile_geometry<KQ>(st.n, p, active, g);
@@ -1234,7 +1235,7 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   auto* const kernel = norm_partials ? (g.direct ? fused_tc_kernel<KQ, true, true> : fused_tc_kernel<KQ, true, false>)
                                      : (g.direct ? fused_tc_kernel<KQ, false, true> : fused_tc_kernel<KQ, false, false>);
   KB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<float2*>(st.amps), g, static_cast<const uint32_t*>(b_image),
@@ -1329,10 +1330,11 @@ void build_tc_image(const std::vector<cplx>& mat, int k, std::vector<uint32_t>& 
   std::memcpy(lo + img, &sbw, 4);
 }
 
-void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active) {
-  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials, active);
-  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials, active);
-  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials, active);
+void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+                     bool overlap) {
+  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials, active, overlap);
+  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials, active, overlap);
+  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials, active, overlap);
   else fail(KETGPU_ERR_LOGIC, "tensor-core block supports k = 4, 5 or 6");
 }
 

@@ -639,6 +639,11 @@ PassRunner::~PassRunner() {
 void PassRunner::launch(const Pass& p) {
   const State& s = s_;
   const Plan& plan = plan_;
+  // The kernels that build the plan's tables may be the stream's last ones;
+  // their writes are sure to be seen only by a launch that waits for their
+  // end.  Later passes may overlap the one before them: it has waited.
+  const bool overlap = !first_;
+  first_ = false;
   const bool ground = s.version == s.ground_version;
   s.touch();
   const uint64_t dim = uint64_t{1} << active_bits(active_);
@@ -686,10 +691,10 @@ void PassRunner::launch(const Pass& p) {
     return;
   }
   if (s.precision == KETGPU_C128) {
-    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, table, active_);
+    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, table, active_, overlap);
     else launch_fused_simt<double>(s, p, table, active_);
   } else if (p.tensor) {
-    launch_fused_tc(s, p, table, p.norm_out ? plan.d_norm + 2 : nullptr, active_);
+    launch_fused_tc(s, p, table, p.norm_out ? plan.d_norm + 2 : nullptr, active_, overlap);
   } else {
     launch_fused_simt<float>(s, p, table, active_);
   }

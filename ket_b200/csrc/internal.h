@@ -235,6 +235,7 @@ class PassRunner {
   const Plan& plan_;
   uint64_t active_;
   bool keep_;  // what is known outlives the run
+  bool first_ = true;
 };
 // Whether every amplitude but amps[0] is zero and amps[0] is 1 (one read;
 // synchronises).
@@ -244,11 +245,13 @@ void upload_plan_tables(Plan& plan, int device, cudaStream_t stream, bool one_st
 // norm_partials: null, or kNormBlocks doubles that receive the per-CTA sums
 // of |out|^2 (zero beyond the grid).  active (here and below): the index bits
 // that can be set in a nonzero amplitude, the pass's qubits included.
-void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active);
+// overlap (and below): the launch may start under the one before it.
+void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+                     bool overlap);
 // complex128 dense blocks (fused_f64.cu): mat_t = the FP64 matrix,
 // transposed ([c][r], re/im).
 bool f64_supported(int n, int k);
-void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, uint64_t active);
+void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, uint64_t active, bool overlap);
 // Host only: the producer and epilogue forms a tensor-core launch of pass p
 // on an n-qubit state takes (tma_dims = tensor-map dimensions, 0 for the
 // cp.async producers; direct = register-to-HBM stores), given the tensor-map

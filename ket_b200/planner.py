@@ -131,8 +131,16 @@ _states: Dict[int, DeviceState] = {}
 
 
 def _state(n: int) -> DeviceState:
+    """A state to time plans on.  None of its amplitudes is known to be zero, so
+    a pass takes the same time wherever it stands in a plan (from |0...0> the
+    first passes cover only the qubits acted on so far)."""
     if n not in _states:
-        _states[n] = DeviceState(n, "c64")
+        st = DeviceState(n, "c64")
+        c = Circuit(n)
+        for q in range(n):
+            c.h(q)
+        st.apply(c, make_options("c64", "greedy", 5, True))
+        _states[n] = st
     return _states[n]
 
 

@@ -11,9 +11,12 @@
 //   reverse   for i = N..1:  g_i = Im <lambda|G_i|psi_i>  (U_i = exp(-i t G_i / 2))
 //                            psi <- U_i^dag psi, lambda <- U_i^dag lambda
 // For CP(t) = diag(1,1,1,e^{it}) the term is -2 Im <lambda|P11|psi>.
-// One kernel per gate does the inner-product partial sums (FP64) and the two
-// inverse applications in a single pass over psi and lambda; all parameter
-// sets of a chunk share every launch (gridDim.y = set).  Layers are the
+// Three forms: up to 11 qubits one CTA a parameter set holds both states and
+// runs everything in one launch (adjoint_resident); larger states go tile by
+// tile, a block of gates a pass (tile_sweep and its compiled form); and one
+// kernel per gate, on request, does the inner-product partial sums (FP64) and
+// the two inverse applications in a single pass over psi and lambda.  All
+// parameter sets of a chunk share every launch.  Layers are the
 // barrier-delimited runs of ops; with checkpoint_every = m the forward state
 // is stored every m layers and the reverse sweep restarts psi from it, so
 // the uncomputation error does not accumulate across segments.
@@ -770,7 +773,7 @@ __global__ void ground_batch(typename C2T<R>::T* states, uint64_t dim) {
 // diagonal gate needs no register bits at all.  Gradient partial sums are
 // formed per thread over its pairs in the state's precision, reduced across
 // the warp in FP64 and accumulated per warp and gate in shared memory (FP64),
-// then summed in fixed order over warps, CTAs and (on the host) blocks.
+// then summed in fixed order over warps, CTAs and blocks (sum_partials).
 
 // TileCfg, TGate, TPhase, TileGeom, the swizzle, the asynchronous copy and
 // the packed complex64 gate code live in adj_tile.cuh, shared with the
@@ -1691,7 +1694,7 @@ int gen_of(int type) {
 // through a switch, and the register moves at its merge points dominate the
 // instruction count.  Here the block's phases and gates become compile-time
 // constants of a kernel generated from adj_tile.cuh: a swap is a renaming,
-// each gate is straight-line packed arithmetic.  The kernels are compiled
+// each gate is straight-line arithmetic.  The kernels are compiled
 // with NVRTC for sm_100a (loaded with dlopen on first use), loaded with the
 // runtime's library API and cached by their source text, so a layer
 // structure that repeats is compiled once per process.  When NVRTC cannot

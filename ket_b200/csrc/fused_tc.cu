@@ -137,8 +137,8 @@ struct TcGeom {
   // cp.async producers and staged stores: chunk i of thread t covers tile
   // amplitudes e = 2t + 256i and e + 1; its offsets are those of e = 2t
   // XOR those of e = 256i (amp_offsets is XOR-linear in e), and these tables
-  // hold the latter: state offset, A-layout (input) and staging (output)
-  // byte offsets
+  // hold the latter: state offset, input image (A rows, or natural tile
+  // order) and output staging byte offsets
   uint64_t chunk_g[32];
   uint32_t chunk_s_in[32], chunk_s_out[32];
   // k = 6 staged stores: the same of a half tile, the tile less the tile bit

@@ -639,13 +639,17 @@ PassRunner::~PassRunner() {
 void PassRunner::launch(const Pass& p) {
   const State& s = s_;
   const Plan& plan = plan_;
-  // The kernels that build the plan's tables may be the stream's last ones;
-  // their writes are sure to be seen only by a launch that waits for their
-  // end.  Later passes may overlap the one before them: it has waited.
-  const bool overlap = !first_;
-  first_ = false;
   const bool ground = s.version == s.ground_version;
   s.touch();
+  // A phase on zeros only, an exchange of zeros: nothing to launch.
+  if (p.kind == PassKind::Phase && (p.p0 & ~active_)) return;
+  if (p.kind == PassKind::Pair && (p.p0 & ~active_) && (p.p1 & ~active_)) return;
+  // The kernels that build the plan's tables may be the stream's last ones;
+  // their writes are sure to be seen only by a launch that waits for their
+  // end.  Launches after the first may overlap the one before them: it has
+  // waited.
+  const bool overlap = !first_;
+  first_ = false;
   const uint64_t dim = uint64_t{1} << active_bits(active_);
   const void* table = static_cast<const char*>(plan.block.p) + p.table;
   if (p.kind == PassKind::NormCapture) {
@@ -671,14 +675,11 @@ void PassRunner::launch(const Pass& p) {
     return;
   }
   if (p.kind == PassKind::Phase) {
-    if ((p.p0 & ~active_) == 0) {  // else it acts on zeros only
-      if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
-      else launch_pair<double>(s, p, active_);
-    }
+    if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
+    else launch_pair<double>(s, p, active_);
     return;
   }
   if (p.kind == PassKind::Pair) {
-    if ((p.p0 & ~active_) && (p.p1 & ~active_)) return;  // exchanges zeros
     active_ |= p.p0 | p.p1;
     if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
     else launch_pair<double>(s, p, active_);

@@ -614,16 +614,16 @@ constexpr uint64_t kGroundCheckBytes = uint64_t{8} << 20;
 
 PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false) {
   const uint64_t all = s.dim() - 1;
-  if (plan.finite && s.version == s.active_version && s.active != all) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
-    if (cap == cudaStreamCaptureStatusNone) {
-      if (!s.exposed) {
-        active_ = s.active;
-        keep_ = true;
-      } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version && is_ground(s)) {
-        active_ = 0;
-      }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) {
+    s.exposed = true;  // the graph's replays write the amplitudes
+  } else if (plan.finite && s.version == s.active_version && s.active != all) {
+    if (!s.exposed) {
+      active_ = s.active;
+      keep_ = true;
+    } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version && is_ground(s)) {
+      active_ = 0;
     }
   }
   active_ &= all;

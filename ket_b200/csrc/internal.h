@@ -88,8 +88,9 @@ struct State {
   // version equals active_version (see Activity): 0 after set_ground.
   mutable uint64_t active = 0;
   mutable uint64_t active_version = ~uint64_t{0};
-  // The amplitudes' address has been handed out: they may change without a
-  // touch(), so what is known about them is checked on the device before use.
+  // The amplitudes' address has been handed out, or a plan has been captured
+  // into a graph: they may change without a touch(), so what is known about
+  // them is checked on the device before use.
   mutable bool exposed = false;
   uint64_t dim() const { return uint64_t{1} << n; }
   size_t amp_bytes() const { return precision == KETGPU_C64 ? 8 : 16; }
@@ -223,7 +224,8 @@ void learned_predict(const std::vector<float>& rows, std::vector<float>& us);
 // states' worth of blocks instead of 63.
 // Nothing is assumed of a plan with non-finite parameters (0 * inf), under
 // stream capture (a graph may replay on another state), and of a state whose
-// address was handed out unless the device finds it to be |0...0>.
+// address was handed out, or whose stream was captured before (a replay writes
+// it), unless the device finds it to be |0...0>.
 class PassRunner {
  public:
   PassRunner(const State& s, const Plan& plan);

@@ -384,7 +384,7 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
     else
       std::memcpy(static_cast<char*>(out) + at, from, len);
   };
-  if (total < kDirectBytes) {
+  if (total < kDirectBytes && total <= ring * chunk) {
     KB_CUDA(cudaMemcpyAsync(stage, src, total, cudaMemcpyDeviceToHost, stream));
     KB_CUDA(cudaStreamSynchronize(stream));
     emit(stage, 0, total);

@@ -612,7 +612,8 @@ void set_ground(const State& s) {
 // part of it (20 qubits, complex128, 16 MB: 556 -> 510 us with the check).
 constexpr uint64_t kGroundCheckBytes = uint64_t{8} << 20;
 
-PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false) {
+PassRunner::PassRunner(const State& s, const Plan& plan)
+    : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false), ground_(false) {
   const uint64_t all = s.dim() - 1;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
@@ -624,8 +625,10 @@ PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), a
       keep_ = true;
     } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version && is_ground(s)) {
       active_ = 0;
+      ground_ = true;
     }
   }
+  if (!s.exposed) ground_ = s.version == s.ground_version;
   active_ &= all;
 }
 
@@ -639,7 +642,7 @@ PassRunner::~PassRunner() {
 void PassRunner::launch(const Pass& p) {
   const State& s = s_;
   const Plan& plan = plan_;
-  const bool ground = s.version == s.ground_version;
+  const bool ground = ground_ && s.version == s.ground_version;
   s.touch();
   // A phase on zeros only, an exchange of zeros: nothing to launch.
   if (p.kind == PassKind::Phase && (p.p0 & ~active_)) return;

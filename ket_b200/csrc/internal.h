@@ -237,6 +237,7 @@ class PassRunner {
   const Plan& plan_;
   uint64_t active_;
   bool keep_;  // what is known outlives the run
+  bool ground_;  // |0...0> while the version is ground_version
   bool first_ = true;
 };
 // Whether every amplitude but amps[0] is zero and amps[0] is 1 (one read;

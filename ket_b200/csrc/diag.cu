@@ -114,7 +114,7 @@ constexpr int kDiagThreads = 256;
 template <typename R>
 __global__ void __launch_bounds__(kDiagThreads, sizeof(R) == 4 ? 4 : 1)
     diag_kernel(typename CD<R>::T* __restrict__ s, int n, const typename CD<R>::T* __restrict__ table,
-                const double* __restrict__ prm, uint64_t n_chunks) {
+                const double* __restrict__ prm, Extent chunks) {
   using T = typename CD<R>::T;
   const int L = n < kDiagLowBits ? n : kDiagLowBits, H = n - L, CH = 1 << L;
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -123,6 +123,8 @@ __global__ void __launch_bounds__(kDiagThreads, sizeof(R) == 4 ? 4 : 1)
   __shared__ double lin[kDiagLowBits];
   __shared__ double phih;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint64_t n_chunks = chunks.count();
+  if (blockIdx.x >= n_chunks) return;
   for (int i = tid; i < CH; i += kDiagThreads) q[i] = table[i];
   // the coefficients in shared memory too: their sums are chains of loads
   double* sprm = reinterpret_cast<double*>(dsm + ((size_t)CH * sizeof(T) + 15) / 16 * 16);
@@ -204,14 +206,15 @@ __global__ void __launch_bounds__(kDiagThreads, sizeof(R) == 4 ? 4 : 1)
 
 }  // namespace
 
-void launch_diag(const State& s, const Pass& p, const void* data, uint64_t active) {
+void launch_diag(const State& s, const Pass& p, const void* data, const Reach& reach) {
   (void)p;
   const int n = s.n;
   const int L = std::min(n, kDiagLowBits);
-  const uint64_t n_chunks = uint64_t{1} << (std::max(active_bits(active), L) - L);
+  const Extent chunks{uint64_t{1} << (std::max(active_bits(reach.active), L) - L), uint64_t{1} << (n - L),
+                      reach.unknown};
   // complex64: four CTAs an SM in two rounds (the second evens out the SMs at
   // 24 qubits, 51 -> 48 us); complex128: its 64 KB tables leave two
-  const unsigned grid = (unsigned)std::min<uint64_t>(n_chunks, 148ull * (s.precision == KETGPU_C64 ? 8 : 4));
+  const unsigned grid = (unsigned)std::min<uint64_t>(chunks.most(), 148ull * (s.precision == KETGPU_C64 ? 8 : 4));
   const int H = n - L;
   const size_t table = (size_t{1} << L) * s.amp_bytes();
   const size_t smem = (table + 15) / 16 * 16 + sizeof(double) * (size_t)(1 + n + L * H + H * H);
@@ -229,10 +232,10 @@ void launch_diag(const State& s, const Pass& p, const void* data, uint64_t activ
   }
   if (s.precision == KETGPU_C64) {
     diag_kernel<float><<<grid, kDiagThreads, smem, s.stream>>>(static_cast<float2*>(s.amps), n,
-                                                               static_cast<const float2*>(data), prm, n_chunks);
+                                                               static_cast<const float2*>(data), prm, chunks);
   } else {
     diag_kernel<double><<<grid, kDiagThreads, smem, s.stream>>>(static_cast<double2*>(s.amps), n,
-                                                                static_cast<const double2*>(data), prm, n_chunks);
+                                                                static_cast<const double2*>(data), prm, chunks);
   }
   count_launch();
   KB_CUDA(cudaGetLastError());

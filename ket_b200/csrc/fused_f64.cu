@@ -66,9 +66,11 @@ struct F64Geom {
   int tpos[6];          // the block's qubits, ascending
   int is_target[kMaxTileBits];
   int tile_pos[kMaxTileBits];
-  int nins;             // positions that are zero in a tile base, ascending:
-  unsigned char ins[40];   // the tile's qubits and the inactive ones
-  uint64_t n_tiles;
+  // positions that are zero in a tile base, ascending: the tile's qubits and
+  // the inactive ones; [1]: where nothing is known, the tile's alone
+  int nins[2];
+  unsigned char ins[2][40];
+  Extent tiles;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -160,9 +162,12 @@ __global__ void __launch_bounds__(F64Cfg<KQ>::THREADS, 1)
   const uint64_t out_next = uint64_t{1} << g.gpos[0];
   const int o0 = tig ^ slot_swizzle(gid), o1 = (4 + tig) ^ slot_swizzle(gid);
 
+  // Set before the run's first pass, so it can be read ahead of the wait too.
+  const int whole = g.tiles.unknown && *g.tiles.unknown;
+  const uint64_t n_tiles = whole ? g.tiles.all : g.tiles.known;
   auto tile_base = [&](uint64_t t) -> uint64_t {
-    for (int j = 0; j < g.nins; ++j) {
-      const int f = g.ins[j];
+    for (int j = 0; j < g.nins[whole]; ++j) {
+      const int f = g.ins[whole][j];
       t = ((t >> f) << (f + 1)) | (t & ((uint64_t{1} << f) - 1));
     }
     return t;
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(F64Cfg<KQ>::THREADS, 1)
   constexpr unsigned long long kNone = ~0ull;
   auto base_of = [&](unsigned i) -> unsigned long long {
     const uint64_t t = (uint64_t)i * gridDim.x + blockIdx.x;
-    return t < g.n_tiles ? tile_base(t) : kNone;
+    return t < n_tiles ? tile_base(t) : kNone;
   };
   auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(Cfg::TEAM) : "memory"); };
   // kStages - 1 tiles in flight; the barrier that publishes a tile also says
@@ -261,7 +266,7 @@ void launch_k(const State& st, const F64Geom& g, const double2* mat_t, bool over
     if (st.device >= 0 && st.device < 64) attr[st.device] = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)std::min<uint64_t>(g.n_tiles, 148));
+  cfg.gridDim = dim3((unsigned)std::min<uint64_t>(g.tiles.most(), 148));
   cfg.blockDim = dim3(Cfg::THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st.stream;
@@ -279,12 +284,12 @@ void launch_k(const State& st, const F64Geom& g, const double2* mat_t, bool over
 // A k-qubit complex128 block needs whole 8-group column blocks.
 bool f64_supported(int n, int k) { return k >= 3 && k <= 6 && n >= k + 3; }
 
-void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_t active, bool overlap) {
+void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, const Reach& reach, bool overlap) {
   F64Geom g{};
   g.k = p.k;
   // 1024-amplitude tiles, fewer amplitudes where that leaves teams without a
   // tile: 2^11 tiles or more, down to one column block
-  uint64_t span = active;  // index bits of the amplitudes the launch covers
+  uint64_t span = reach.active;  // index bits of the amplitudes the launch covers
   for (int b = 0; b < p.k; ++b) span |= uint64_t{1} << p.qubits[b];
   g.tb = std::clamp(__builtin_popcountll(span) - 11, p.k + 3, kMaxTileBits);
   uint64_t tmask = 0;
@@ -307,10 +312,11 @@ void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, uint64_
       if (!g.is_target[j]) g.gpos[gb++] = q;
       ++j;
     }
-    if (((tile_mask | ~span) >> q) & 1) g.ins[g.nins++] = (unsigned char)q;
+    if (((tile_mask | ~span) >> q) & 1) g.ins[0][g.nins[0]++] = (unsigned char)q;
+    if ((tile_mask >> q) & 1) g.ins[1][g.nins[1]++] = (unsigned char)q;
   }
   g.q0_group = g.gpos[0] == 0;
-  g.n_tiles = uint64_t{1} << (__builtin_popcountll(span) - g.tb);
+  g.tiles = {uint64_t{1} << (__builtin_popcountll(span) - g.tb), st.dim() >> g.tb, reach.unknown};
   const double2* m = static_cast<const double2*>(mat_t);
   switch (p.k) {
     case 3: launch_k<3>(st, g, m, overlap); break;

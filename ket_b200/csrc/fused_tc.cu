@@ -109,8 +109,10 @@ struct TcGeom {
   int tile_pos[16];   // tile qubits, ascending
   int is_target[16];
   int m_low;          // tile qubits 0..m_low-1 form the low run
-  int nh;             // positions above the low run that are zero in a tile
-  unsigned char hpos[40];  // base, ascending: tile qubits and inactive ones
+  // positions above the low run that are zero in a tile base, ascending: tile
+  // qubits and inactive ones; [1]: where nothing is known, tile qubits alone
+  int nh[2];
+  unsigned char hpos[2][40];
   int direct;         // the epilogue stores from registers (see launch_fused_tc)
   int natural;        // staged: input images in natural tile order (see natural_reads)
   // Tensor-copy producer (tma_dims > 0, see launch_tc): dimension i of the
@@ -122,7 +124,7 @@ struct TcGeom {
   uint64_t tma_mask[5];
   uint32_t ctile[64];
   uint64_t cdep[64];  // offset of target combination c from its group's amplitude
-  uint64_t n_tiles;
+  Extent tiles;
   // k = 6 tensor copy in half tiles (half = 1): each tile is two boxes of
   // the tensor map over the tile less its highest target qubit, at the tile
   // base and at base + top_off; ctile[0..31] are the low five targets'
@@ -437,6 +439,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   fence_proxy_async();
+  // Set before the run's first pass, so it can be read ahead of the wait too.
+  const int whole = g.tiles.unknown && *g.tiles.unknown;
+  const uint64_t n_tiles = whole ? g.tiles.all : g.tiles.known;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -445,7 +450,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
   const uint64_t first = blockIdx.x;
   const uint64_t stride = gridDim.x;
-  const uint64_t count = first < g.n_tiles ? (g.n_tiles - first + stride - 1) / stride : 0;
+  const uint64_t count = first < n_tiles ? (n_tiles - first + stride - 1) / stride : 0;
   const bool q0_group = !g.is_target[0];
 
   // Bounded wait; on timeout raise the flags and let every role leave.
@@ -495,8 +500,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto pair_slot = [](int row, int comb) -> uint32_t { return pair_slot_offset(row, comb, DIM); };
   auto tile_base = [&](uint64_t t) -> uint64_t {
     uint64_t b = t << g.m_low;
-    for (int j = 0; j < g.nh; ++j) {
-      const int f = g.hpos[j];
+    for (int j = 0; j < g.nh[whole]; ++j) {
+      const int f = g.hpos[whole][j];
       b = ((b >> f) << (f + 1)) | (b & ((uint64_t{1} << f) - 1));
     }
     return b;
@@ -1044,7 +1049,7 @@ bool tma_wanted(const TcGeom& g, const Pass& p, int tb) {
 // the tile index decomposition, each combination's offset and the
 // cp.async-form direct-store rule.
 template <int KQ>
-void tile_geometry(int n, const Pass& p, uint64_t active, TcGeom& g) {
+void tile_geometry(int n, const Pass& p, const Reach& reach, TcGeom& g) {
   using Cfg = TcCfg<KQ>;
   g = TcGeom{};
   uint64_t tmask = 0;
@@ -1084,12 +1089,13 @@ void tile_geometry(int n, const Pass& p, uint64_t active, TcGeom& g) {
       if ((c >> b) & 1) d |= uint64_t{1} << p.qubits[b];
     g.cdep[c] = d;
   }
-  g.nh = 0;
   // tile bases range over the active qubits outside the tile
-  const uint64_t span = (active & ((uint64_t{1} << n) - 1)) | tiles_mask;
-  for (int q = g.m_low; q < n; ++q)
-    if (((tiles_mask | ~span) >> q) & 1) g.hpos[g.nh++] = (unsigned char)q;
-  g.n_tiles = uint64_t{1} << (__builtin_popcountll(span) - Cfg::TB);
+  const uint64_t span = (reach.active & ((uint64_t{1} << n) - 1)) | tiles_mask;
+  for (int q = g.m_low; q < n; ++q) {
+    if (((tiles_mask | ~span) >> q) & 1) g.hpos[0][g.nh[0]++] = (unsigned char)q;
+    if ((tiles_mask >> q) & 1) g.hpos[1][g.nh[1]++] = (unsigned char)q;
+  }
+  g.tiles = {uint64_t{1} << (__builtin_popcountll(span) - Cfg::TB), (uint64_t{1} << n) >> Cfg::TB, reach.unknown};
   constexpr int CPT = Cfg::TILE / 2 / 128;
   static_assert(CPT <= 32, "chunk tables");
   for (int i = 0; i < CPT; ++i) {
@@ -1182,11 +1188,11 @@ int* error_flag() {
 }
 
 template <int KQ>
-void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm_partials, const Reach& reach,
                bool overlap) {
   using Cfg = TcCfg<KQ>;
   TcGeom g;
-  tile_geometry<KQ>(st.n, p, active, g);
+  tile_geometry<KQ>(st.n, p, reach, g);
   g.error = error_flag();
   g.norm_out = norm_partials;
   if (norm_partials)  // entries past the grid stay zero for the in-order sum
@@ -1224,7 +1230,7 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   static int sms[64] = {0};
   if (!sms[st.device]) sms[st.device] = sm_count_tc(st.device);
   uint64_t grid = (uint64_t)sms[st.device];
-  if (grid > g.n_tiles) grid = g.n_tiles;
+  grid = std::min(grid, g.tiles.most());
   if (norm_partials && grid > (uint64_t)kNormBlocks) fail(KETGPU_ERR_LOGIC, "tensor-core norm partials");
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
@@ -1330,20 +1336,20 @@ void build_tc_image(const std::vector<cplx>& mat, int k, std::vector<uint32_t>& 
   std::memcpy(lo + img, &sbw, 4);
 }
 
-void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, const Reach& reach,
                      bool overlap) {
-  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials, active, overlap);
-  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials, active, overlap);
-  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials, active, overlap);
+  if (p.k == 5) launch_tc<5>(s, p, b_image, norm_partials, reach, overlap);
+  else if (p.k == 4) launch_tc<4>(s, p, b_image, norm_partials, reach, overlap);
+  else if (p.k == 6) launch_tc<6>(s, p, b_image, norm_partials, reach, overlap);
   else fail(KETGPU_ERR_LOGIC, "tensor-core block supports k = 4, 5 or 6");
 }
 
 void tc_form(int n, const Pass& p, int* tma_dims, int* direct) {
   if (p.k < 4 || p.k > 6) fail(KETGPU_ERR_LOGIC, "tensor-core block supports k = 4, 5 or 6");
   TcGeom g;
-  if (p.k == 5) tile_geometry<5>(n, p, ~uint64_t{0}, g);
-  else if (p.k == 6) tile_geometry<6>(n, p, ~uint64_t{0}, g);
-  else tile_geometry<4>(n, p, ~uint64_t{0}, g);
+  if (p.k == 5) tile_geometry<5>(n, p, Reach{~uint64_t{0}}, g);
+  else if (p.k == 6) tile_geometry<6>(n, p, Reach{~uint64_t{0}}, g);
+  else tile_geometry<4>(n, p, Reach{~uint64_t{0}}, g);
   int start[16], tq[16];
   const int nd = p.k == 6 ? encode_half_tiles(nullptr, p, g, nullptr)
                  : tma_wanted(g, p, p.k + kGroupBits) ? tile_runs(g, p.k + kGroupBits, start, tq)

@@ -52,7 +52,7 @@ __device__ __forceinline__ uint64_t spread(uint64_t i, const int* fixed, int nfi
 }
 
 struct PairGeom {
-  uint64_t count;
+  Extent pairs;
   uint64_t p0, p1;
   int fixed[3];
   int nfixed;
@@ -66,13 +66,14 @@ __global__ void __launch_bounds__(kThreads)
     pair_kernel(typename C2<R>::T* __restrict__ s, PairGeom g, Mat2<R> m) {
   using T = typename C2<R>::T;
   const uint64_t start = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
+  const uint64_t count = g.pairs.count();
   T a[kUnroll], b[kUnroll];
   uint64_t k0[kUnroll];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
     const uint64_t i = start + (uint64_t)u * kThreads;
     k0[u] = ~uint64_t{0};
-    if (i < g.count) {
+    if (i < count) {
       const uint64_t base = spread(i, g.fixed, g.nfixed);
       k0[u] = base;
       a[u] = s[base | g.p0];
@@ -107,13 +108,14 @@ __global__ void __launch_bounds__(kThreads)
     phase_kernel(typename C2<R>::T* __restrict__ s, PairGeom g, R pre, R pim) {
   using T = typename C2<R>::T;
   const uint64_t start = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
+  const uint64_t count = g.pairs.count();
   T a[kUnroll];
   uint64_t k[kUnroll];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
     const uint64_t i = start + (uint64_t)u * kThreads;
     k[u] = ~uint64_t{0};
-    if (i < g.count) {
+    if (i < count) {
       k[u] = spread(i, g.fixed, g.nfixed) | g.p0;
       a[u] = s[k[u]];
     }
@@ -155,7 +157,7 @@ __device__ __forceinline__ void pair_update(const Mat2<float>& m, float2 a, floa
 template <int MODE>
 __global__ void __launch_bounds__(kThreads)
     pair_kernel_v2(float2* __restrict__ s, PairGeom g, Mat2<float> m) {
-  const uint64_t count2 = g.count >> 1;
+  const uint64_t count2 = g.pairs.count() >> 1;
   const uint64_t start = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
   float4 a[kUnroll], b[kUnroll];
   uint64_t k0[kUnroll];
@@ -182,7 +184,8 @@ __global__ void __launch_bounds__(kThreads)
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads)
-    pair_kernel_q0(float2* __restrict__ s, uint64_t count, Mat2<float> m) {
+    pair_kernel_q0(float2* __restrict__ s, Extent pairs, Mat2<float> m) {
+  const uint64_t count = pairs.count();
   const uint64_t start = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
   float4 v[kUnroll];
 #pragma unroll
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     phase_kernel_v2(float2* __restrict__ s, PairGeom g, float pre, float pim) {
-  const uint64_t count2 = g.count >> 1;
+  const uint64_t count2 = g.pairs.count() >> 1;
   const uint64_t start = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
   float4 a[kUnroll];
   uint64_t k[kUnroll];
@@ -239,7 +242,7 @@ struct FusedGeom {
   int n, k, tb;           // tb = tile bits = min(kTileBits, n)
   int tile_pos[kTileBits];  // tile bit positions, ascending
   int is_target[kTileBits];
-  uint64_t n_tiles;
+  Extent tiles;
 };
 
 template <typename R>
@@ -250,6 +253,8 @@ __global__ void __launch_bounds__(kThreads)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int dim = 1 << g.k;
   const int tile = 1 << g.tb;
+  const uint64_t n_tiles = g.tiles.count();
+  if (blockIdx.x >= n_tiles) return;
   T* mt = reinterpret_cast<T*>(smem_raw);  // [c][r] : dim*dim
   T* buf = mt + dim * dim;                 // [group][comb] : tile
   __shared__ uint64_t off_lo[64], off_hi[64];
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(kThreads)
   }
   __syncthreads();
 
-  for (uint64_t t = blockIdx.x; t < g.n_tiles; t += gridDim.x) {
+  for (uint64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     // tile base: spread t over the non-tile positions
     uint64_t base = t;
     for (int j = 0; j < g.tb; ++j) {
@@ -342,20 +347,21 @@ int sm_count(int device) {
 }
 
 template <typename R>
-void launch_pair(const State& st, const Pass& p, uint64_t active) {
+void launch_pair(const State& st, const Pass& p, const Reach& reach, bool zeros) {
   using T = typename C2<R>::T;
   PairGeom g{};
   g.nfixed = p.nfixed;
   for (int j = 0; j < 3; ++j) g.fixed[j] = p.fixed[j];
-  g.count = (uint64_t{1} << active_bits(active)) >> p.nfixed;
+  g.pairs = {zeros ? 0 : (uint64_t{1} << active_bits(reach.active)) >> p.nfixed, st.dim() >> p.nfixed, reach.unknown};
+  const uint64_t most = g.pairs.most();
   g.p0 = p.p0;
   g.p1 = p.p1;
   T* s = static_cast<T*>(st.amps);
   // complex64: 16-byte forms when the layout allows them
-  const bool vec2 = sizeof(R) == 4 && p.fixed[0] >= 1 && g.count >= 2;
+  const bool vec2 = sizeof(R) == 4 && p.fixed[0] >= 1 && most >= 2 && g.pairs.known != 1;
   const bool q0 = sizeof(R) == 4 && p.kind == PassKind::Pair && p.nfixed == 1 && p.fixed[0] == 0;
   const uint64_t per_block = (uint64_t)kThreads * kUnroll;
-  const uint64_t blocks = ((vec2 ? g.count / 2 : g.count) + per_block - 1) / per_block;
+  const uint64_t blocks = ((vec2 ? most / 2 : most) + per_block - 1) / per_block;
   Mat2<R> m;
   for (int j = 0; j < 4; ++j) {
     m.re[j] = (R)p.m[j].real();
@@ -385,11 +391,11 @@ void launch_pair(const State& st, const Pass& p, uint64_t active) {
             pair_kernel_v2<kPairGeneral><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g, m);
         } else {
           if (p.mode == kPairSwap)
-            pair_kernel_q0<kPairSwap><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.count, m);
+            pair_kernel_q0<kPairSwap><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.pairs, m);
           else if (p.mode == kPairDiag)
-            pair_kernel_q0<kPairDiag><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.count, m);
+            pair_kernel_q0<kPairDiag><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.pairs, m);
           else
-            pair_kernel_q0<kPairGeneral><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.count, m);
+            pair_kernel_q0<kPairGeneral><<<(unsigned)blocks, kThreads, 0, st.stream>>>(s, g.pairs, m);
         }
         count_launch();
         KB_CUDA(cudaGetLastError());
@@ -408,7 +414,7 @@ void launch_pair(const State& st, const Pass& p, uint64_t active) {
 }
 
 template <typename R>
-void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, uint64_t active) {
+void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, const Reach& reach) {
   using T = typename C2<R>::T;
   FusedGeom g{};
   g.n = st.n;
@@ -432,8 +438,8 @@ void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, uint64
       ++j;
     }
   // the tiles whose base lies below the highest active qubit
-  const uint64_t below = (uint64_t{1} << active_bits(active)) - 1;
-  g.n_tiles = uint64_t{1} << __builtin_popcountll(below & ~tiles_mask);
+  const uint64_t below = (uint64_t{1} << active_bits(reach.active)) - 1;
+  g.tiles = {uint64_t{1} << __builtin_popcountll(below & ~tiles_mask), st.dim() >> g.tb, reach.unknown};
   const int dim = 1 << p.k;
   const size_t smem = sizeof(T) * ((size_t)dim * dim + ((size_t)1 << g.tb));
   static bool attr_set[2] = {false, false};
@@ -444,7 +450,7 @@ void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, uint64
     attr_set[which] = true;
   }
   uint64_t grid = (uint64_t)sm_count(st.device) * 4;
-  if (grid > g.n_tiles) grid = g.n_tiles;
+  grid = std::min(grid, g.tiles.most());
   fused_simt_kernel<R><<<(unsigned)grid, kThreads, smem, st.stream>>>(
       static_cast<T*>(st.amps), g, static_cast<const T*>(mat_t));
   count_launch();
@@ -473,10 +479,12 @@ struct RunGate {
 
 template <typename R>
 __global__ void __launch_bounds__(kThreads)
-    run_kernel(typename C2<R>::T* __restrict__ s, uint64_t n_chunks, int bits,
+    run_kernel(typename C2<R>::T* __restrict__ s, Extent chunks, int bits,
                const RunGate<R>* __restrict__ gates, int ngates) {
   using T = typename C2<R>::T;
   extern __shared__ __align__(16) unsigned char run_smem[];
+  const uint64_t n_chunks = chunks.count();
+  if (blockIdx.x >= n_chunks) return;
   T* sm = reinterpret_cast<T*>(run_smem);
   RunGate<R>* sg = reinterpret_cast<RunGate<R>*>(run_smem + (sizeof(T) << kRunBits));
   for (int i = threadIdx.x; i < ngates; i += kThreads) sg[i] = gates[i];
@@ -554,17 +562,18 @@ void run_device_data(const std::vector<Pass>& gates, int precision, std::vector<
   else append_run_gates<double>(gates, out);
 }
 
-void launch_run(const State& st, const Pass& p, const void* data, uint64_t active) {
+void launch_run(const State& st, const Pass& p, const void* data, const Reach& reach) {
   const int bits = st.n < kRunBits ? st.n : kRunBits;
-  const uint64_t n_chunks = uint64_t{1} << (std::max(active_bits(active), bits) - bits);
+  const Extent chunks{uint64_t{1} << (std::max(active_bits(reach.active), bits) - bits), st.dim() >> bits,
+                      reach.unknown};
   static int sms[64] = {0};
   if (!sms[st.device]) sms[st.device] = sm_count(st.device);
   uint64_t grid = (uint64_t)sms[st.device] * 8;
-  if (grid > n_chunks) grid = n_chunks;
+  grid = std::min(grid, chunks.most());
   if (st.precision == KETGPU_C64) {
     const size_t smem = (sizeof(float2) << kRunBits) + sizeof(RunGate<float>) * (size_t)p.n_gates;
     run_kernel<float><<<(unsigned)grid, kThreads, smem, st.stream>>>(
-        static_cast<float2*>(st.amps), n_chunks, bits, static_cast<const RunGate<float>*>(data), p.n_gates);
+        static_cast<float2*>(st.amps), chunks, bits, static_cast<const RunGate<float>*>(data), p.n_gates);
   } else {
     const size_t smem = (sizeof(double2) << kRunBits) + sizeof(RunGate<double>) * (size_t)p.n_gates;
     static bool attr[64] = {false};
@@ -574,7 +583,7 @@ void launch_run(const State& st, const Pass& p, const void* data, uint64_t activ
       attr[st.device] = true;
     }
     run_kernel<double><<<(unsigned)grid, kThreads, smem, st.stream>>>(
-        static_cast<double2*>(st.amps), n_chunks, bits, static_cast<const RunGate<double>*>(data), p.n_gates);
+        static_cast<double2*>(st.amps), chunks, bits, static_cast<const RunGate<double>*>(data), p.n_gates);
   }
   count_launch();
   KB_CUDA(cudaGetLastError());
@@ -607,13 +616,12 @@ void set_ground(const State& s) {
   KB_CUDA(cudaGetLastError());
 }
 
-// The check of a state whose address was handed out costs a call 12 us and
+// The look at a state whose address was handed out costs a call 12 us and
 // more; below this size a pass on the whole state is no slower than one on
 // part of it (20 qubits, complex128, 16 MB: 556 -> 510 us with the check).
 constexpr uint64_t kGroundCheckBytes = uint64_t{8} << 20;
 
-PassRunner::PassRunner(const State& s, const Plan& plan)
-    : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false), ground_(false) {
+PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), active_(~uint64_t{0}), keep_(false) {
   const uint64_t all = s.dim() - 1;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
@@ -623,12 +631,12 @@ PassRunner::PassRunner(const State& s, const Plan& plan)
     if (!s.exposed) {
       active_ = s.active;
       keep_ = true;
-    } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version && is_ground(s)) {
+    } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version) {
+      word_ = std::make_unique<StreamScratch>(sizeof(unsigned), s.device, s.stream);
+      find_not_ground(s, static_cast<unsigned*>(word_->p));
       active_ = 0;
-      ground_ = true;
     }
   }
-  if (!s.exposed) ground_ = s.version == s.ground_version;
   active_ &= all;
 }
 
@@ -639,21 +647,25 @@ PassRunner::~PassRunner() {
   }
 }
 
+Extent PassRunner::amplitudes() const {
+  return {uint64_t{1} << active_bits(active_), s_.dim(), word_ ? static_cast<const unsigned*>(word_->p) : nullptr};
+}
+
 void PassRunner::launch(const Pass& p) {
   const State& s = s_;
   const Plan& plan = plan_;
-  const bool ground = ground_ && s.version == s.ground_version;
+  const bool ground = !s.exposed && s.version == s.ground_version;
   s.touch();
-  // A phase on zeros only, an exchange of zeros: nothing to launch.
-  if (p.kind == PassKind::Phase && (p.p0 & ~active_)) return;
-  if (p.kind == PassKind::Pair && (p.p0 & ~active_) && (p.p1 & ~active_)) return;
+  // a phase on zeros, an exchange of zeros
+  const bool zeros = (p.kind == PassKind::Phase && (p.p0 & ~active_)) ||
+                     (p.kind == PassKind::Pair && (p.p0 & ~active_) && (p.p1 & ~active_));
+  if (zeros && !word_) return;
   // The kernels that build the plan's tables may be the stream's last ones;
   // their writes are sure to be seen only by a launch that waits for their
   // end.  Launches after the first may overlap the one before them: it has
   // waited.
   const bool overlap = !first_;
   first_ = false;
-  const uint64_t dim = uint64_t{1} << active_bits(active_);
   const void* table = static_cast<const char*>(plan.block.p) + p.table;
   if (p.kind == PassKind::NormCapture) {
     if (ground) {  // |0...0>: the squared norm is 1, no pass over the state
@@ -661,7 +673,7 @@ void PassRunner::launch(const Pass& p) {
       count_launch();
       KB_CUDA(cudaGetLastError());
     } else {
-      norm_to_device(s, dim, plan.d_norm + 2, plan.d_norm);
+      norm_to_device(s, amplitudes(), plan.d_norm + 2, plan.d_norm);
     }
     return;
   }
@@ -669,38 +681,31 @@ void PassRunner::launch(const Pass& p) {
     if (p.norm_out)  // the block before summed |out|^2 per CTA into the partials
       norm_from_partials(s, plan.d_norm + 2, plan.d_norm + 1);
     else
-      norm_to_device(s, dim, plan.d_norm + 2, plan.d_norm + 1);
-    rescale_state(s, dim, plan.d_norm, plan.d_norm + 1);
-    return;
-  }
-  if (p.kind == PassKind::Diagonal) {
-    launch_diag(s, p, table, active_);
-    return;
-  }
-  if (p.kind == PassKind::Phase) {
-    if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
-    else launch_pair<double>(s, p, active_);
+      norm_to_device(s, amplitudes(), plan.d_norm + 2, plan.d_norm + 1);
+    rescale_state(s, amplitudes(), plan.d_norm, plan.d_norm + 1);
     return;
   }
   if (p.kind == PassKind::Pair) {
-    active_ |= p.p0 | p.p1;
-    if (s.precision == KETGPU_C64) launch_pair<float>(s, p, active_);
-    else launch_pair<double>(s, p, active_);
-    return;
+    if (!zeros) active_ |= p.p0 | p.p1;
+  } else if (p.kind == PassKind::Fused || p.kind == PassKind::SharedRun) {
+    for (int gi : p.gates)
+      for (int j = 0; j < gate_arity(plan.ops[gi].type); ++j) active_ |= uint64_t{1} << plan.ops[gi].q[j];
   }
-  for (int gi : p.gates)
-    for (int j = 0; j < gate_arity(plan.ops[gi].type); ++j) active_ |= uint64_t{1} << plan.ops[gi].q[j];
-  if (p.kind == PassKind::SharedRun) {
-    launch_run(s, p, table, active_);
-    return;
-  }
-  if (s.precision == KETGPU_C128) {
-    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, table, active_, overlap);
-    else launch_fused_simt<double>(s, p, table, active_);
+  const Reach reach{active_, amplitudes().unknown};
+  if (p.kind == PassKind::Diagonal) {
+    launch_diag(s, p, table, reach);
+  } else if (p.kind == PassKind::Phase || p.kind == PassKind::Pair) {
+    if (s.precision == KETGPU_C64) launch_pair<float>(s, p, reach, zeros);
+    else launch_pair<double>(s, p, reach, zeros);
+  } else if (p.kind == PassKind::SharedRun) {
+    launch_run(s, p, table, reach);
+  } else if (s.precision == KETGPU_C128) {
+    if (f64_supported(s.n, p.k)) launch_fused_f64(s, p, table, reach, overlap);
+    else launch_fused_simt<double>(s, p, table, reach);
   } else if (p.tensor) {
-    launch_fused_tc(s, p, table, p.norm_out ? plan.d_norm + 2 : nullptr, active_, overlap);
+    launch_fused_tc(s, p, table, p.norm_out ? plan.d_norm + 2 : nullptr, reach, overlap);
   } else {
-    launch_fused_simt<float>(s, p, table, active_);
+    launch_fused_simt<float>(s, p, table, reach);
   }
 }
 

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <complex>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -213,6 +214,22 @@ bool learned_model_attached();
 void learned_predict(const std::vector<float>& rows, std::vector<float>& us);
 
 // ---- kernel launchers (gates.cu / fused_*.cu / reduce.cu) ------------------
+// The part of a state that a pass works on: the amplitudes whose set index
+// bits all lie within `active`.  unknown (null: that is certain) points to a
+// device word; where it holds nonzero, the pass works on the whole state.
+struct Reach {
+  uint64_t active;
+  const unsigned* unknown = nullptr;
+};
+// How many of something (tiles, chunks, pairs, amplitudes) a launch works on.
+struct Extent {
+  uint64_t known, all;
+  const unsigned* unknown;
+  uint64_t most() const { return unknown ? all : known; }
+#ifdef __CUDACC__
+  __device__ __forceinline__ uint64_t count() const { return unknown && *unknown ? all : known; }
+#endif
+};
 // Runs a plan's passes in order on the part of the state that can be nonzero.
 //
 // From |0...0> only amplitudes whose set index bits lie within the qubits
@@ -222,10 +239,12 @@ void learned_predict(const std::vector<float>& rows, std::vector<float>& us);
 // amplitudes are zeros and stay so.  Planned in an order that activates
 // qubits late (order_passes), the 30-qubit depth-40 brick wall moves 47.1
 // states' worth of blocks instead of 63.
-// Nothing is assumed of a plan with non-finite parameters (0 * inf), under
-// stream capture (a graph may replay on another state), and of a state whose
-// address was handed out, or whose stream was captured before (a replay writes
-// it), unless the device finds it to be |0...0>.
+// Nothing is assumed of a plan with non-finite parameters (0 * inf) and under
+// stream capture (a graph may replay on another state).  A state whose address
+// was handed out, or whose stream was captured before (a replay writes it), is
+// looked at on the device after a reset: a kernel sets a word if it is not
+// |0...0>, and each pass takes the part of the state that it works on by that
+// word, so the host waits for nothing.
 class PassRunner {
  public:
   PassRunner(const State& s, const Plan& plan);
@@ -233,28 +252,29 @@ class PassRunner {
   void launch(const Pass& p);
 
  private:
+  Extent amplitudes() const;  // the lowest indices that hold all active ones
+
   const State& s_;
   const Plan& plan_;
   uint64_t active_;
   bool keep_;  // what is known outlives the run
-  bool ground_;  // |0...0> while the version is ground_version
+  std::unique_ptr<StreamScratch> word_;  // set by the device: not |0...0> at the start
   bool first_ = true;
 };
-// Whether every amplitude but amps[0] is zero and amps[0] is 1 (one read;
-// synchronises).
-bool is_ground(const State& s);
+// Enqueues: *word = whether the state differs from |0...0> (one read of it).
+void find_not_ground(const State& s, unsigned* word);
 // one_stream: the plan runs on `stream` only (the tables are not waited for).
 void upload_plan_tables(Plan& plan, int device, cudaStream_t stream, bool one_stream);
 // norm_partials: null, or kNormBlocks doubles that receive the per-CTA sums
-// of |out|^2 (zero beyond the grid).  active (here and below): the index bits
-// that can be set in a nonzero amplitude, the pass's qubits included.
+// of |out|^2 (zero beyond the grid).  reach (here and below): the index bits
+// that can be set in a nonzero amplitude, the pass's gates' qubits included.
 // overlap (and below): the launch may start under the one before it.
-void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, uint64_t active,
+void launch_fused_tc(const State& s, const Pass& p, const void* b_image, double* norm_partials, const Reach& reach,
                      bool overlap);
 // complex128 dense blocks (fused_f64.cu): mat_t = the FP64 matrix,
 // transposed ([c][r], re/im).
 bool f64_supported(int n, int k);
-void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, uint64_t active, bool overlap);
+void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, const Reach& reach, bool overlap);
 // Host only: the producer and epilogue forms a tensor-core launch of pass p
 // on an n-qubit state takes (tma_dims = tensor-map dimensions, 0 for the
 // cp.async producers; direct = register-to-HBM stores), given the tensor-map
@@ -262,9 +282,9 @@ void launch_fused_f64(const State& s, const Pass& p, const void* mat_t, uint64_t
 void tc_form(int n, const Pass& p, int* tma_dims, int* direct);
 // Diagonal pass: device data = table (2^L complex, state precision) then FP64
 // coefficients.
-void launch_diag(const State& s, const Pass& p, const void* data, uint64_t active);
+void launch_diag(const State& s, const Pass& p, const void* data, const Reach& reach);
 // SharedRun pass: device gate records laid out by run_device_data (gates.cu).
-void launch_run(const State& s, const Pass& p, const void* data, uint64_t active);
+void launch_run(const State& s, const Pass& p, const void* data, const Reach& reach);
 void run_device_data(const std::vector<Pass>& gates, int precision, std::vector<unsigned char>& out);
 // The coefficients the diagonal kernel reads after its table (diag.cu).
 void diag_coefficients(const DiagPoly& poly, int n, std::vector<double>& out);
@@ -277,9 +297,9 @@ void build_tc_image(const std::vector<cplx>& mat, int k, std::vector<uint32_t>& 
 bool tc_supported(int k);
 
 void set_ground(const State& s);
-// Squared norm of the first dim amplitudes into a device scalar (partials:
+// Squared norm of the first amplitudes into a device scalar (partials:
 // kNormBlocks doubles).
-void norm_to_device(const State& s, uint64_t dim, double* partials, double* out);
+void norm_to_device(const State& s, const Extent& dim, double* partials, double* out);
 // The same from partials a tensor-core block already wrote (in index order).
 void norm_from_partials(const State& s, const double* partials, double* out);
 // Look up (and so load) the no-allocation entry point's scratch array and
@@ -315,9 +335,9 @@ struct StreamLease {
   StreamLease(const StreamLease&) = delete;
   StreamLease& operator=(const StreamLease&) = delete;
 };
-// The first dim amplitudes *= sqrt(target[0] / current[0]), factor read on the
+// The first amplitudes *= sqrt(target[0] / current[0]), factor read on the
 // device.
-void rescale_state(const State& s, uint64_t dim, const double* target, const double* current);
+void rescale_state(const State& s, const Extent& dim, const double* target, const double* current);
 double reduce_norm(const State& s);
 cplx reduce_inner(const State& a, const State& b);
 void compare_states(const State& a, const State& b, double out[5]);

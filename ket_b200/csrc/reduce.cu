@@ -58,8 +58,9 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 }
 
 template <typename T>
-__global__ void norm_partial(const T* __restrict__ s, uint64_t dim, double* __restrict__ part) {
+__global__ void norm_partial(const T* __restrict__ s, Extent extent, double* __restrict__ part) {
   __shared__ double sh[32];
+  const uint64_t dim = extent.count();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   // 16-byte loads, eight in flight, a sum each (one 8-byte load at a time:
@@ -416,8 +417,9 @@ int grid_for(uint64_t work, int per_block) {
 }
 
 template <typename T>
-__global__ void rescale_kernel(T* __restrict__ s, uint64_t dim, const double* __restrict__ target,
+__global__ void rescale_kernel(T* __restrict__ s, Extent extent, const double* __restrict__ target,
                                const double* __restrict__ current) {
+  const uint64_t dim = extent.count();
   const double c = current[0];
   const double f = c > 0.0 ? sqrt(target[0] / c) : 1.0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -457,7 +459,7 @@ __global__ void rescale_kernel(T* __restrict__ s, uint64_t dim, const double* __
 
 }  // namespace
 
-void norm_to_device(const State& st, uint64_t dim, double* partials, double* out) {
+void norm_to_device(const State& st, const Extent& dim, double* partials, double* out) {
   if (st.precision == KETGPU_C64)
     norm_partial<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), dim,
                                                                    partials);
@@ -475,7 +477,7 @@ void norm_from_partials(const State& st, const double* partials, double* out) {
   KB_CUDA(cudaGetLastError());
 }
 
-void rescale_state(const State& st, uint64_t dim, const double* target, const double* current) {
+void rescale_state(const State& st, const Extent& dim, const double* target, const double* current) {
   if (st.precision == KETGPU_C64)
     rescale_kernel<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<float2*>(st.amps), dim,
                                                                      target, current);
@@ -501,9 +503,7 @@ __global__ void not_ground(const uint64_t* __restrict__ w, uint64_t words, uint6
 }
 }  // namespace
 
-bool is_ground(const State& st) {
-  StreamScratch sc(sizeof(unsigned), st.device, st.stream);
-  unsigned* d = static_cast<unsigned*>(sc.p);
+void find_not_ground(const State& st, unsigned* d) {
   KB_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned), st.stream));
   const bool c64 = st.precision == KETGPU_C64;
   const uint64_t words = st.dim() * (c64 ? 1 : 2);
@@ -511,20 +511,17 @@ bool is_ground(const State& st) {
       static_cast<const uint64_t*>(st.amps), words, c64 ? 0x3f800000ull : 0x3ff0000000000000ull, d);
   count_launch();
   KB_CUDA(cudaGetLastError());
-  unsigned h = 1;
-  KB_CUDA(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st.stream));
-  KB_CUDA(cudaStreamSynchronize(st.stream));
-  return h == 0;
 }
 
 double reduce_norm(const State& st) {
   const int blocks = grid_for(st.dim(), kRThreads * 8);
   StreamScratch part(sizeof(double) * (blocks + 1), st.device, st.stream);
   double* d = static_cast<double*>(part.p);
+  const Extent all{st.dim(), st.dim(), nullptr};
   if (st.precision == KETGPU_C64)
-    norm_partial<float2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), st.dim(), d);
+    norm_partial<float2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), all, d);
   else
-    norm_partial<double2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), st.dim(), d);
+    norm_partial<double2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), all, d);
   finish_partials<<<1, kRThreads, 0, st.stream>>>(d, blocks, 1, d + blocks);
   count_launch(2);
   KB_CUDA(cudaGetLastError());

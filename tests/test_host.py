@@ -481,3 +481,31 @@ def test_plan_block_matrices_match_the_oracle(oracle, golden):
                     want = oracle.block_matrix(np.ascontiguousarray(ops[gates]), qs)
                     assert np.abs(got - want).max() < 1e-12, (rep, n, prec, k, i)
                 p.close()
+
+
+@pytest.mark.parametrize("last_qubit", [False, True])
+def test_planning_time_grows_with_the_passes(last_qubit):
+    """A circuit of lone gates between barriers, a qubit idle or used only at
+    the end: four times the passes take about four times as long to plan (10
+    times when every pass was searched for among all that are left)."""
+    import time
+    import ket_b200 as ket
+    from ket_b200.api import Plan
+
+    def seconds(passes):
+        c = ket.Circuit(21)
+        for i in range(passes):
+            c.u(i % 20, 0.1, 0.2, 0.3)
+            c.barrier()
+        if last_qubit:
+            c.h(20)
+        ops = c.to_ops()
+        t0 = time.process_time()
+        p = Plan(21, ops, ket.make_options("c64"))
+        t = time.process_time() - t0
+        assert int(p.stats()["n_passes"]) == passes + last_qubit
+        p.close()
+        return t
+
+    small = min(seconds(25000) for _ in range(2))
+    assert seconds(100000) < 6.5 * small

@@ -97,8 +97,10 @@ def test_execute_waits_for_nothing(precision):
     st.reset()
     with torch.cuda.stream(stream):
         torch.cuda._sleep(10**9)  # about half a second
+        slept = torch.cuda.Event()
+        slept.record(stream)
     plan.execute(st, sync=False)
-    assert not stream.query()
+    assert not slept.query()
     assert np.array_equal(st.to_numpy(), want)
 
 

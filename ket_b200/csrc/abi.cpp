@@ -39,8 +39,16 @@ void set_last_error(const char* msg) { t_err = msg; }
 
 void check_cuda(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return;
+  cudaGetLastError();  // the next launch's check is not to find this error
   const int code = (e == cudaErrorMemoryAllocation) ? KETGPU_ERR_OOM : KETGPU_ERR_CUDA;
   throw Error(code, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+void release_kept() {
+  release_run_state();
+  release_idle_states();
+  release_workspaces();
+  release_pools();
 }
 
 DeviceGuard::DeviceGuard(int dev) {
@@ -77,11 +85,20 @@ cudaMemPool_t scratch_pool(int device) {
 }
 }  // namespace
 
-StreamScratch::StreamScratch(size_t bytes, int device, cudaStream_t stream) : st(stream) {
+namespace {
+void* pool_alloc(size_t bytes, int device, cudaStream_t stream) {
+  void* p = nullptr;
   cudaMemPool_t pool = scratch_pool(device);
-  if (pool) KB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream));
-  else KB_CUDA(cudaMallocAsync(&p, bytes ? bytes : 8, stream));
+  allocate("device scratch", [&] {
+    return pool ? cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream)
+                : cudaMallocAsync(&p, bytes ? bytes : 8, stream);
+  });
+  return p;
 }
+}  // namespace
+
+StreamScratch::StreamScratch(size_t bytes, int device, cudaStream_t stream)
+    : p(pool_alloc(bytes, device, stream)), st(stream) {}
 
 StreamScratch::~StreamScratch() {
   if (p) cudaFreeAsync(p, st);
@@ -163,7 +180,7 @@ Workspace::Workspace(size_t b, int dev) : bytes(b), device(dev) {
     return;
   }
   free_on(w.device, w.p);
-  KB_CUDA(cudaMalloc(&p, bytes ? bytes : 8));
+  allocate("cudaMalloc(workspace)", [&] { return cudaMalloc(&p, bytes ? bytes : 8); });
 }
 
 Workspace::~Workspace() {
@@ -178,11 +195,7 @@ Workspace::~Workspace() {
   free_on(device, p);
 }
 
-DeviceBlock::DeviceBlock(size_t bytes, int device, cudaStream_t stream) {
-  cudaMemPool_t pool = scratch_pool(device);
-  if (pool) KB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 8, pool, stream));
-  else KB_CUDA(cudaMallocAsync(&p, bytes ? bytes : 8, stream));
-}
+DeviceBlock::DeviceBlock(size_t bytes, int device, cudaStream_t stream) : p(pool_alloc(bytes, device, stream)) {}
 
 DeviceBlock& DeviceBlock::operator=(DeviceBlock&& o) noexcept {
   std::swap(p, o.p);
@@ -613,20 +626,18 @@ State* create_state(int n, int precision) {
   size_t free_b = 0, total_b = 0;
   KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   if (bytes > free_b) {  // give back what is kept between calls first
-    release_run_state();
-    release_idle_states();
-    release_workspaces();
-    release_pools();
+    release_kept();
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   }
   if (bytes > free_b)
     fail(KETGPU_ERR_OOM, "state of " + std::to_string(bytes) + " bytes exceeds free device memory (" +
                              std::to_string(free_b) + ")");
   KB_CUDA(cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking));
-  const cudaError_t e = cudaMalloc(&st->amps, bytes);
-  if (e != cudaSuccess) {
+  try {
+    allocate("cudaMalloc(state)", [&] { return cudaMalloc(&st->amps, bytes); });
+  } catch (...) {
     cudaStreamDestroy(st->stream);
-    check_cuda(e, "cudaMalloc(state)");
+    throw;
   }
   std::unique_ptr<State, void (*)(State*)> guard_st(st.release(), destroy_state);
   noalloc_prepare(guard_st->device);
@@ -868,12 +879,7 @@ KB_API int ketgpu_run_last_profile(double* out6) {
 }
 
 KB_API int ketgpu_release_cache(void) {
-  return guard([&] {
-    release_run_state();
-    release_idle_states();
-    release_workspaces();
-    release_pools();
-  });
+  return guard([&] { release_kept(); });
 }
 
 KB_API int ketgpu_norm(const ketgpu_state* s, double* out) {

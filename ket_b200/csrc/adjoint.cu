@@ -2012,10 +2012,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     size_t free_b = 0, total_b = 0;
     KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     if ((uint64_t)((free_b * 0.6) / per_set) < batch) {  // first take back what is kept between calls
-      release_run_state();
-      release_idle_states();
-      release_workspaces();
-      release_pools();
+      release_kept();
       KB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     }
     chunk = std::max<uint64_t>(1, (uint64_t)((free_b * 0.6) / per_set));

@@ -40,6 +40,22 @@ struct DeviceGuard {
   ~DeviceGuard();
 };
 
+// Gives back what the library keeps between calls: idle states, workspaces,
+// scratch.
+void release_kept();
+// Device memory: `alloc` (returning a cudaError_t), once more after what is
+// kept between calls has been given back if there is no room.
+template <class F>
+void allocate(const char* what, F&& alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    release_kept();
+    e = alloc();
+  }
+  check_cuda(e, what);
+}
+
 // Device scratch of one call, stream-ordered, from the library's own pool on
 // the device.  The pool keeps up to kPoolKeep bytes between calls (taking them
 // back from the driver at each synchronisation cost 0.1 ms and more a call);

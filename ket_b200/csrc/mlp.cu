@@ -208,11 +208,11 @@ void ensure(Mlp& M, size_t batch, size_t samples) {
   cudaFree(M.idx);
   M.xbuf = M.ybuf = M.act = M.out = nullptr;
   M.idx = nullptr;
-  KB_CUDA(cudaMalloc(&M.xbuf, need * IN * sizeof(float)));
-  KB_CUDA(cudaMalloc(&M.ybuf, need * sizeof(float)));
-  KB_CUDA(cudaMalloc(&M.act, need * 2 * HID * sizeof(float)));
-  KB_CUDA(cudaMalloc(&M.out, need * sizeof(float)));
-  KB_CUDA(cudaMalloc(&M.idx, need * sizeof(int)));
+  allocate("cudaMalloc(planner rows)", [&] { return cudaMalloc(&M.xbuf, need * IN * sizeof(float)); });
+  allocate("cudaMalloc(planner rows)", [&] { return cudaMalloc(&M.ybuf, need * sizeof(float)); });
+  allocate("cudaMalloc(planner rows)", [&] { return cudaMalloc(&M.act, need * 2 * HID * sizeof(float)); });
+  allocate("cudaMalloc(planner rows)", [&] { return cudaMalloc(&M.out, need * sizeof(float)); });
+  allocate("cudaMalloc(planner rows)", [&] { return cudaMalloc(&M.idx, need * sizeof(int)); });
   M.cap = need;
 }
 

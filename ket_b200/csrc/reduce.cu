@@ -607,7 +607,7 @@ Levels build_tree(const State& st) {
   // The tree lives with the state (1/31 of a complex128 state's size, 1/15
   // of a complex64 one) and is rebuilt only after the amplitudes changed.
   if (total && !st.tree) {
-    KB_CUDA(cudaMalloc(&st.tree, sizeof(double) * total));
+    allocate("cudaMalloc(sampling tree)", [&] { return cudaMalloc(&st.tree, sizeof(double) * total); });
     st.tree_doubles = total;
   }
   if (!total || st.tree_version == st.version) return lv;

@@ -240,7 +240,7 @@ void pauli_masks(int n, const char* pauli, uint64_t& flip, uint64_t& sign, int& 
   q = num_y % 4;
 }
 
-int tc_error_flag(bool reset);
+int tc_error_flag(int device, bool reset);
 
 namespace {
 
@@ -528,8 +528,8 @@ void execute(const Plan& plan, State& s, bool one_stream = false) {
   for (const Pass& p : plan.passes) run.launch(p);
 }
 
-void check_tc_flag() {
-  if (tc_error_flag(true))
+void check_tc_flag(const State& s) {
+  if (tc_error_flag(s.device, true))
     fail(KETGPU_ERR_TIMEOUT, "tensor-core block kernel timed out waiting on its MMA barrier");
 }
 
@@ -769,7 +769,7 @@ KB_API int ketgpu_state_synchronize(ketgpu_state* s) {
     need(s != nullptr, "state is null");
     DeviceGuard g(as_state(s)->device);
     KB_CUDA(cudaStreamSynchronize(as_state(s)->stream));
-    check_tc_flag();
+    check_tc_flag(*as_state(s));
   });
 }
 
@@ -820,7 +820,7 @@ KB_API int ketgpu_apply(ketgpu_state* s, const ketgpu_op* ops, uint64_t n_ops, c
     execute(plan, st, true);
     KB_CUDA(cudaStreamSynchronize(st.stream));
     plan.idle = true;
-    check_tc_flag();
+    check_tc_flag(st);
   });
 }
 
@@ -863,7 +863,7 @@ KB_API int ketgpu_run(int32_t n, const ketgpu_op* ops, uint64_t n_ops, const ket
     DownloadTimes dt;
     download(*st, 0, st->dim(), out_c128, o.precision == KETGPU_C64, &dt);
     const double down_ms = ms_since(t3);
-    check_tc_flag();
+    check_tc_flag(*st);
     const double prof[6] = {plan_ms, state_ms, exec_ms, down_ms, dt.copy_wait_ms, dt.widen_ms};
     std::copy(prof, prof + 6, t_run_profile);
     std::lock_guard<std::mutex> lk(g_run_mu);  // keep it for the next call
@@ -1005,7 +1005,7 @@ KB_API int ketgpu_plan_execute_timed(const ketgpu_plan* p, ketgpu_state* s, floa
     KB_CUDA(cudaEventSynchronize(ev[np]));
     for (size_t i = 0; i < np; ++i) KB_CUDA(cudaEventElapsedTime(&pass_ms[i], ev[i], ev[i + 1]));
     for (auto& e : ev) cudaEventDestroy(e);
-    check_tc_flag();
+    check_tc_flag(st);
   });
 }
 

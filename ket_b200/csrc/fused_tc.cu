@@ -1168,21 +1168,23 @@ int encode_half_tiles(const State* st, const Pass& p, TcGeom& g, CUtensorMap* ma
   return nd;
 }
 
-// The timeout flag: mapped host memory, so that the host reads it after a
-// synchronisation without a device call (a copy from a device symbol took
-// 15 us a call).  Null until the first tensor-core launch.
-std::atomic<int*> g_error_flag{nullptr};
+// The timeout flags, one a device: mapped host memory, so that the host reads
+// them after a synchronisation without a device call (a copy from a device
+// symbol took 15 us a call).  Null until a device's first tensor-core launch.
+constexpr int kFlagDevices = 64;
+std::atomic<int*> g_error_flags[kFlagDevices];
 std::mutex g_error_mu;
 
-int* error_flag() {
-  int* p = g_error_flag.load(std::memory_order_acquire);
+int* error_flag(int device) {
+  if (device < 0 || device >= kFlagDevices) fail(KETGPU_ERR_LOGIC, "tensor-core timeout flag");
+  int* p = g_error_flags[device].load(std::memory_order_acquire);
   if (p) return p;
   std::lock_guard<std::mutex> lk(g_error_mu);
-  p = g_error_flag.load(std::memory_order_relaxed);
+  p = g_error_flags[device].load(std::memory_order_relaxed);
   if (!p) {
     KB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
     *p = 0;
-    g_error_flag.store(p, std::memory_order_release);
+    g_error_flags[device].store(p, std::memory_order_release);
   }
   return p;
 }
@@ -1193,7 +1195,7 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
   using Cfg = TcCfg<KQ>;
   TcGeom g;
   tile_geometry<KQ>(st.n, p, reach, g);
-  g.error = error_flag();
+  g.error = error_flag(st.device);
   g.norm_out = norm_partials;
   if (norm_partials)  // entries past the grid stay zero for the in-order sum
     KB_CUDA(cudaMemsetAsync(norm_partials, 0, sizeof(double) * kNormBlocks, st.stream));
@@ -1358,8 +1360,9 @@ void tc_form(int n, const Pass& p, int* tma_dims, int* direct) {
   *direct = nd ? 1 : g.direct;
 }
 
-int tc_error_flag(bool reset) {
-  int* p = g_error_flag.load(std::memory_order_acquire);
+int tc_error_flag(int device, bool reset) {
+  if (device < 0 || device >= kFlagDevices) return 0;
+  int* p = g_error_flags[device].load(std::memory_order_acquire);
   if (!p) return 0;
   const int v = *reinterpret_cast<volatile int*>(p);
   if (reset && v) *reinterpret_cast<volatile int*>(p) = 0;

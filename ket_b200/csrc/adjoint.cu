@@ -2081,12 +2081,11 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     }
     d_ham = std::make_unique<DevBuf>(sizeof(HamTerm) * std::max(T_, 1), dev, st);
     KB_CUDA(cudaMemcpyAsync(d_ham->p, ht.data(), sizeof(HamTerm) * T_, cudaMemcpyHostToDevice, st));
-    static bool ham_attr[2] = {false, false};
-    if (!ham_attr[sizeof(R) == 8]) {
+    static OncePerDevice ham_attr;  // one for each R
+    ham_attr(dev, [] {
       KB_CUDA(cudaFuncSetAttribute(ham_half<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)ham_smem(kHamSmemTerms)));
-      ham_attr[sizeof(R) == 8] = true;
-    }
+    });
   }
   // ham_half grid: about one set's worth of resident CTAs per half
   const uint64_t ham_words = dim / 2 / kHamPer;
@@ -2267,8 +2266,8 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
       b.part_off = grad_doubles;
       grad_doubles += b.grad_gate.size() * chunk * (size_t)gx;
     }
-    static bool attr_set[2] = {false, false};
-    if (!attr_set[sizeof(R) == 8]) {
+    static OncePerDevice tile_attr;  // one for each R
+    tile_attr(dev, [] {
       const int smem_rev = (int)tile_smem<R>(true, kMaxBlockGates, kMaxBlockGrads);
       const int smem_fwd = (int)tile_smem<R>(false, kMaxBlockGates, 0);
       if constexpr (sizeof(R) == 4) {
@@ -2278,8 +2277,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
         KB_CUDA(cudaFuncSetAttribute(tile_sweep<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_rev));
         KB_CUDA(cudaFuncSetAttribute(tile_sweep<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_fwd));
       }
-      attr_set[sizeof(R) == 8] = true;
-    }
+    });
   }
   const int per_value = ham_inside ? 1 : ham_split ? 2 * ham_ctas : ham_blocks;
   const size_t ham_doubles = chunk * (size_t)per_value;

@@ -220,16 +220,13 @@ void launch_diag(const State& s, const Pass& p, const void* data, const Reach& r
   const size_t smem = (table + 15) / 16 * 16 + sizeof(double) * (size_t)(1 + n + L * H + H * H);
   const double* prm = reinterpret_cast<const double*>(static_cast<const unsigned char*>(data) + table);
   // at 40 qubits: the table and 9.3 KB of coefficients
-  static bool attr[2][64] = {};
-  const int which = s.precision == KETGPU_C64 ? 0 : 1;
-  if (s.device < 0 || s.device >= 64 || !attr[which][s.device]) {
-    const int most = (int)(((size_t)s.amp_bytes() << kDiagLowBits) + 10240);
-    if (which == 0)
-      KB_CUDA(cudaFuncSetAttribute(diag_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    else
-      KB_CUDA(cudaFuncSetAttribute(diag_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    if (s.device >= 0 && s.device < 64) attr[which][s.device] = true;
-  }
+  static OncePerDevice attr;
+  attr(s.device, [] {
+    KB_CUDA(cudaFuncSetAttribute(diag_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)((sizeof(float2) << kDiagLowBits) + 10240)));
+    KB_CUDA(cudaFuncSetAttribute(diag_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)((sizeof(double2) << kDiagLowBits) + 10240)));
+  });
   if (s.precision == KETGPU_C64) {
     diag_kernel<float><<<grid, kDiagThreads, smem, s.stream>>>(static_cast<float2*>(s.amps), n,
                                                                static_cast<const float2*>(data), prm, chunks);

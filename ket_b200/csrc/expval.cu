@@ -294,11 +294,11 @@ void launch_flips_r(dim3 grid, int device, cudaStream_t st, const T* s, int n, c
                     uint64_t stride) {
   constexpr int smem = (int)sizeof(T) * kFlipThreads << R;
   if constexpr (smem > 16 * 1024) {
-    static bool attr[64] = {false};
-    if (device < 0 || device >= 64 || !attr[device]) {
-      KB_CUDA(cudaFuncSetAttribute(expval_flips<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      if (device >= 0 && device < 64) attr[device] = true;
-    }
+    static OncePerDevice attr;
+    attr(device, [] {
+      KB_CUDA(cudaFuncSetAttribute(expval_flips<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(T) * kFlipThreads << R));
+    });
   }
   expval_flips<T, R><<<grid, kFlipThreads, smem, st>>>(s, n, g, part, stride);
 }

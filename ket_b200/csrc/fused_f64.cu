@@ -259,12 +259,11 @@ template <int KQ>
 void launch_k(const State& st, const F64Geom& g, const double2* mat_t, bool overlap) {
   using Cfg = F64Cfg<KQ>;
   const size_t smem = sizeof(double2) * Cfg::TEAMS * kStages * ((size_t)1 << g.tb);
-  static bool attr[64] = {false};
-  if (st.device < 0 || st.device >= 64 || !attr[st.device]) {
+  static OncePerDevice attr;  // one for each KQ
+  attr(st.device, [] {
     KB_CUDA(cudaFuncSetAttribute(fused_f64_kernel<KQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double2) * Cfg::TEAMS * kStages << kMaxTileBits)));
-    if (st.device >= 0 && st.device < 64) attr[st.device] = true;
-  }
+  });
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)std::min<uint64_t>(g.tiles.most(), 148));
   cfg.blockDim = dim3(Cfg::THREADS);

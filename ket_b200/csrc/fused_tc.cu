@@ -1222,13 +1222,12 @@ void launch_tc(const State& st, const Pass& p, const void* b_image, double* norm
       g.ctile[c] = off ^ ((off >> 3) & 0x70u);  // swizzled (see the converters)
     }
   }
-  static int attr_done[64] = {0};
-  if (st.device >= 0 && st.device < 64 && !(attr_done[st.device] & (1 << KQ))) {
+  static OncePerDevice attr;  // one for each KQ
+  attr(st.device, [] {
     for (auto* f : {fused_tc_kernel<KQ, false, false>, fused_tc_kernel<KQ, false, true>,
                     fused_tc_kernel<KQ, true, false>, fused_tc_kernel<KQ, true, true>})
       KB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
-    attr_done[st.device] |= 1 << KQ;
-  }
+  });
   static int sms[64] = {0};
   if (!sms[st.device]) sms[st.device] = sm_count_tc(st.device);
   uint64_t grid = (uint64_t)sms[st.device];

@@ -442,13 +442,11 @@ void launch_fused_simt(const State& st, const Pass& p, const void* mat_t, const 
   g.tiles = {uint64_t{1} << __builtin_popcountll(below & ~tiles_mask), st.dim() >> g.tb, reach.unknown};
   const int dim = 1 << p.k;
   const size_t smem = sizeof(T) * ((size_t)dim * dim + ((size_t)1 << g.tb));
-  static bool attr_set[2] = {false, false};
-  const int which = sizeof(R) == 8 ? 1 : 0;
-  if (!attr_set[which]) {
+  static OncePerDevice attr;  // one for each R
+  attr(st.device, [] {
     KB_CUDA(cudaFuncSetAttribute(fused_simt_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  200 * 1024));
-    attr_set[which] = true;
-  }
+  });
   uint64_t grid = (uint64_t)sm_count(st.device) * 4;
   grid = std::min(grid, g.tiles.most());
   fused_simt_kernel<R><<<(unsigned)grid, kThreads, smem, st.stream>>>(
@@ -576,12 +574,11 @@ void launch_run(const State& st, const Pass& p, const void* data, const Reach& r
         static_cast<float2*>(st.amps), chunks, bits, static_cast<const RunGate<float>*>(data), p.n_gates);
   } else {
     const size_t smem = (sizeof(double2) << kRunBits) + sizeof(RunGate<double>) * (size_t)p.n_gates;
-    static bool attr[64] = {false};
-    if (!attr[st.device]) {
+    static OncePerDevice attr;
+    attr(st.device, [] {
       KB_CUDA(cudaFuncSetAttribute(run_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)((sizeof(double2) << kRunBits) + sizeof(RunGate<double>) * kRunMaxGates)));
-      attr[st.device] = true;
-    }
+    });
     run_kernel<double><<<(unsigned)grid, kThreads, smem, st.stream>>>(
         static_cast<double2*>(st.amps), chunks, bits, static_cast<const RunGate<double>*>(data), p.n_gates);
   }

@@ -43,6 +43,22 @@ struct DeviceGuard {
 // Gives back what the library keeps between calls: idle states, workspaces,
 // scratch.
 void release_kept();
+// Kernel attributes are a device's: `set` on the first call for each device.
+// One object for each set of attributes.
+class OncePerDevice {
+ public:
+  template <class F>
+  void operator()(int device, F&& set) {
+    const bool noted = device >= 0 && device < 64;
+    if (noted && done_[device].load(std::memory_order_acquire)) return;
+    set();
+    if (noted) done_[device].store(true, std::memory_order_release);
+  }
+
+ private:
+  std::atomic<bool> done_[64] = {};
+};
+
 // Device memory: `alloc` (returning a cudaError_t), once more after what is
 // kept between calls has been given back if there is no room.
 template <class F>

@@ -274,12 +274,11 @@ void upload_plan_tables(Plan& plan, int device, cudaStream_t stream, bool one_st
                               stream));
     if (!jobs.empty()) {
       const size_t smem = max_k ? sizeof(double2) << (2 * max_k) : 0;
-      static bool attr[64] = {false};
-      if (device < 0 || device >= 64 || !attr[device]) {
+      static OncePerDevice attr;
+      attr(device, [] {
         KB_CUDA(cudaFuncSetAttribute(build_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)(sizeof(double2) << 12)));
-        if (device >= 0 && device < 64) attr[device] = true;
-      }
+      });
       build_tables<<<(unsigned)jobs.size(), kTableThreads, smem, stream>>>(static_cast<unsigned char*>(block.p),
                                                                             jobs_at);
       count_launch();

@@ -17,6 +17,7 @@
 #include <exception>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <random>
 #include <string>
 #include <thread>
@@ -370,10 +371,46 @@ constexpr uint64_t kDirectBytes = uint64_t{4} << 20;
 // Piece of a download that fits the staging buffers as a whole.
 constexpr uint64_t kPieceBytes = uint64_t{1} << 19;
 
+// Events without times.
+struct Events {
+  std::vector<cudaEvent_t> ev;
+  explicit Events(size_t count) : ev(count, nullptr) {
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < count && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+    if (e != cudaSuccess) destroy();
+    KB_CUDA(e);
+  }
+  ~Events() { destroy(); }
+  void destroy() {
+    for (cudaEvent_t& x : ev)
+      if (x) cudaEventDestroy(x), x = nullptr;
+  }
+  cudaEvent_t operator[](size_t i) const { return ev[i]; }
+};
+
+// Helper threads, up to `most` of them: fewer, or none, where the system has
+// no more to give.
+struct Helpers {
+  std::vector<std::thread> th;
+  template <class F>
+  Helpers(size_t most, F&& work) {
+    th.reserve(most);
+    try {
+      for (size_t t = 0; t < most; ++t) th.emplace_back(work, t);
+    } catch (...) {
+    }
+  }
+  ~Helpers() {
+    for (auto& x : th) x.join();
+  }
+};
+
 // `total` bytes of device memory into a host buffer, as they are or (widen)
-// floats as doubles.  Large buffers go through pinned staging and are written
-// by several threads: most of the time of a copy into fresh pageable memory
-// is its page faults (32 MB: 7.4 ms in one call, 1.7 ms this way).
+// floats as doubles.  Large buffers go through pinned staging and are
+// written by several threads: most of the time of a copy into fresh pageable
+// memory is its page faults (32 MB: 7.4 ms in one call, 1.7 ms this way).  The
+// staging is one download's at a time: two threads that read 64 MB each take
+// 5.8 ms in turn, 16.3 ms when one of them copies directly.
 void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream_t stream, DownloadTimes* times) {
   if (!total) return;
   if (!widen && total < kDirectBytes) {
@@ -404,18 +441,26 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
     return;
   }
   const unsigned hw = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-  cudaError_t err = cudaSuccess;  // no throw while the workers run
-  std::vector<std::thread> th;
+  cudaError_t err = cudaSuccess;  // no throw while copies are in flight
+  auto finish = [&] {
+    if (err != cudaSuccess) cudaStreamSynchronize(stream);  // copies still on their way into the staging
+    check_cuda(err, "download");
+  };
   if (total <= ring * chunk) {
-    // every piece in flight at once, each handed to whichever worker is next
+    // every piece in flight at once, each handed to whichever thread is next
     // when it has landed
     const uint64_t pieces = (total + kPieceBytes - 1) / kPieceBytes;
-    std::vector<cudaEvent_t> ev(pieces);
-    for (auto& e : ev) KB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const Events ev(pieces);
     std::atomic<uint64_t> landed{0}, taken{0};
-    auto work = [&] {
+    const auto start = std::chrono::steady_clock::now();
+    auto work = [&](size_t) {
       for (uint64_t c; (c = taken.fetch_add(1)) < pieces;) {
-        while (landed.load(std::memory_order_acquire) <= c) _mm_pause();
+        // spins for 5 ms (a thread that wakes up costs a call of 10^6 draws
+        // 0.8 ms), then looks from time to time: the stream may have long work
+        // ahead of the copies
+        for (unsigned spins = 1; landed.load(std::memory_order_acquire) <= c;)
+          if (spins % 256 || ms_since(start) < 5.0) _mm_pause(), ++spins;
+          else std::this_thread::sleep_for(std::chrono::microseconds(200));
         emit(stage + c * kPieceBytes, c * kPieceBytes, std::min(kPieceBytes, total - c * kPieceBytes));
       }
     };
@@ -425,7 +470,7 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
       if (err == cudaSuccess) err = cudaEventRecord(ev[c], stream);
     }
     if (err == cudaSuccess) {
-      for (unsigned t = 1; t < std::min<uint64_t>(hw, pieces); ++t) th.emplace_back(work);
+      const Helpers helpers(std::min<uint64_t>(hw, pieces) - 1, work);
       const auto w0 = std::chrono::steady_clock::now();
       for (uint64_t c = 0; c < pieces; ++c) {
         if (err == cudaSuccess) err = cudaEventSynchronize(ev[c]);
@@ -433,16 +478,13 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
       }
       if (times) times->copy_wait_ms += ms_since(w0);
       const auto s0 = std::chrono::steady_clock::now();
-      work();
-      for (auto& x : th) x.join();
+      work(0);
       if (times) times->widen_ms += ms_since(s0);
     }
-    for (auto& e : ev) cudaEventDestroy(e);
-    check_cuda(err, "download");
+    finish();
     return;
   }
-  std::vector<cudaEvent_t> ev(ring);
-  for (auto& e : ev) KB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  const Events ev(ring);
   const uint64_t nchunks = (total + chunk - 1) / chunk;
   auto issue = [&](uint64_t c) {
     const uint64_t lo = c * chunk, len = std::min(chunk, total - lo);
@@ -450,11 +492,13 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
     if (e == cudaSuccess) e = cudaEventRecord(ev[c % ring], stream);
     if (e != cudaSuccess && err == cudaSuccess) err = e;
   };
-  // Chunk c is written out by every worker while chunks c+1 .. c+ring-1 are
-  // in flight.  The workers start once per download and step through the
-  // chunks between two barriers; the calling thread is worker 0 and also
-  // issues the copies.
-  const unsigned nt = hw;
+  // Chunk c is written out by every thread while chunks c+1 .. c+ring-1 are
+  // in flight.  The helpers start once per download and step through the
+  // chunks between two barriers; the calling thread works too and also issues
+  // the copies.
+  unsigned nt = 1;
+  std::optional<std::barrier<>> sync;  // once it is known how many threads there are
+  std::atomic<bool> go{false};
   auto slice = [&](unsigned t, uint64_t c) {
     const uint64_t lo = c * chunk, len = std::min(chunk, total - lo);
     // rounded to 64 bytes per worker
@@ -462,33 +506,37 @@ void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream
     const uint64_t a = std::min(len, t * per), b = std::min(len, a + per);
     if (b > a) emit(stage + (c % ring) * chunk + a, lo + a, b - a);
   };
-  std::barrier sync(nt);
-  auto work = [&](unsigned t) {
+  auto work = [&](size_t t) {
+    go.wait(false);
     for (uint64_t c = 0; c < nchunks; ++c) {
-      sync.arrive_and_wait();  // chunk c has landed
-      slice(t, c);
-      sync.arrive_and_wait();  // chunk c is consumed
+      sync->arrive_and_wait();  // chunk c has landed
+      slice((unsigned)t + 1, c);
+      sync->arrive_and_wait();  // chunk c is consumed
     }
   };
-  for (unsigned t = 1; t < nt; ++t) th.emplace_back(work, t);
   for (uint64_t c = 0; c < std::min<uint64_t>(ring - 1, nchunks); ++c) issue(c);
-  for (uint64_t c = 0; c < nchunks; ++c) {
-    const auto w0 = std::chrono::steady_clock::now();
-    if (err == cudaSuccess) {
-      const cudaError_t e = cudaEventSynchronize(ev[c % ring]);
-      if (e != cudaSuccess) err = e;
+  {
+    const Helpers helpers(hw - 1, work);
+    nt = 1 + (unsigned)helpers.th.size();
+    sync.emplace(nt);
+    go.store(true);
+    go.notify_all();
+    for (uint64_t c = 0; c < nchunks; ++c) {
+      const auto w0 = std::chrono::steady_clock::now();
+      if (err == cudaSuccess) {
+        const cudaError_t e = cudaEventSynchronize(ev[c % ring]);
+        if (e != cudaSuccess) err = e;
+      }
+      if (times) times->copy_wait_ms += ms_since(w0);
+      if (c + ring - 1 < nchunks && err == cudaSuccess) issue(c + ring - 1);
+      sync->arrive_and_wait();
+      const auto s0 = std::chrono::steady_clock::now();
+      slice(0, c);
+      if (times) times->widen_ms += ms_since(s0);
+      sync->arrive_and_wait();
     }
-    if (times) times->copy_wait_ms += ms_since(w0);
-    if (c + ring - 1 < nchunks && err == cudaSuccess) issue(c + ring - 1);
-    sync.arrive_and_wait();
-    const auto s0 = std::chrono::steady_clock::now();
-    slice(0, c);
-    if (times) times->widen_ms += ms_since(s0);
-    sync.arrive_and_wait();
   }
-  for (auto& x : th) x.join();
-  for (auto& e : ev) cudaEventDestroy(e);
-  check_cuda(err, "download");
+  finish();
 }
 
 // Amplitudes [first, first + count) into a host buffer, in the state's format

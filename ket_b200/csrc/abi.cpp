@@ -405,15 +405,22 @@ struct Helpers {
   }
 };
 
+bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
 // `total` bytes of device memory into a host buffer, as they are or (widen)
-// floats as doubles.  Large buffers go through pinned staging and are
+// floats as doubles.  Large pageable buffers go through pinned staging and are
 // written by several threads: most of the time of a copy into fresh pageable
 // memory is its page faults (32 MB: 7.4 ms in one call, 1.7 ms this way).  The
 // staging is one download's at a time: two threads that read 64 MB each take
 // 5.8 ms in turn, 16.3 ms when one of them copies directly.
 void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream_t stream, DownloadTimes* times) {
   if (!total) return;
-  if (!widen && total < kDirectBytes) {
+  if (!widen && (total < kDirectBytes || page_locked(out))) {
     KB_CUDA(cudaMemcpyAsync(out, src, total, cudaMemcpyDeviceToHost, stream));
     KB_CUDA(cudaStreamSynchronize(stream));
     return;

@@ -1,5 +1,5 @@
 """Downloads and their helper threads: none to be had, a stream with other work
-ahead and several downloads at once."""
+ahead, several downloads at once, page-locked buffers."""
 import os
 import subprocess
 import sys
@@ -102,3 +102,18 @@ def test_downloads_at_once():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("n", [17, 21, 23])
+def test_page_locked_buffers(n):
+    import torch
+
+    import ket_b200 as kb
+    from ket_b200 import _lib
+    st = kb.DeviceState(n, "c128")
+    v = torch.view_as_real(st.torch_view())
+    v.copy_(torch.arange(v.numel(), device="cuda").reshape(v.shape))
+    torch.cuda.synchronize()
+    out = torch.zeros((1 << n, 2), dtype=torch.float64).pin_memory()
+    _lib.check(_lib.lib.ketgpu_state_download(st.handle, 0, 1 << n, out.data_ptr()))
+    assert torch.equal(out, v.cpu())

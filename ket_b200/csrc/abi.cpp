@@ -716,9 +716,20 @@ void free_state(State* s) {
   delete s;
 }
 
+// Waits until nothing reads or writes the state any more.  Where its address
+// was handed out that may be work on any stream (cudaFree would wait for it).
+bool quiet(const State& s) {
+  if (!s.exposed) return cudaStreamSynchronize(s.stream) == cudaSuccess;
+  int prev = -1;
+  if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(s.device) != cudaSuccess) return false;
+  const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+  cudaSetDevice(prev);
+  return ok;
+}
+
 void destroy_state(State* s) {
   if (!s) return;
-  if (s->amps && s->stream && state_bytes(*s) <= kIdleBytes && cudaStreamSynchronize(s->stream) == cudaSuccess) {
+  if (s->amps && s->stream && state_bytes(*s) <= kIdleBytes && quiet(*s)) {
     for (State* x : keep_idle_state(s)) free_state(x);
     return;
   }

@@ -358,6 +358,8 @@ void expval_terms(const State& st, const std::vector<uint64_t>& flip, const std:
   for (int t = 0; t < T; ++t) order[t] = t;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return flip[a] < flip[b]; });
   size_t open = 0;  // groups before it are full
+  uint64_t last_flip = 0;  // the flip placed last, and its group
+  size_t last = 0;
   for (int i = 0; i < T;) {
     const uint64_t f = flip[order[i]];
     if (!f) {
@@ -369,7 +371,8 @@ void expval_terms(const State& st, const std::vector<uint64_t>& flip, const std:
     int cnt = 1;
     while (cnt < kPerFlip && i + cnt < T && flip[order[i + cnt]] == f) ++cnt;
     while (open < groups.size() && gens[open] == r) ++open;
-    size_t gi = open;
+    // the groups up to the last one of this flip hold it, span it or are full
+    size_t gi = f == last_flip ? std::max(open, last + 1) : open;
     for (; gi < groups.size(); ++gi)
       if (gens[gi] < r && bases[gi].reduce(f)) break;
     if (gi == groups.size()) {
@@ -379,6 +382,8 @@ void expval_terms(const State& st, const std::vector<uint64_t>& flip, const std:
       bases.emplace_back();
       gens.push_back(0);
     }
+    last_flip = f;
+    last = gi;
     bases[gi].add(f);
     FlipGroup& g = groups[gi];
     const int c = gens[gi]++;

@@ -134,7 +134,8 @@ int ketgpu_plan_create(int32_t n_qubits, const ketgpu_op* ops, uint64_t n_ops,
                        const ketgpu_options* opt, ketgpu_plan** out);
 int ketgpu_plan_destroy(ketgpu_plan* p);
 int ketgpu_plan_stats_get(const ketgpu_plan* p, ketgpu_plan_stats* out);
-/* Enqueue every pass of the plan on the state's stream (no host sync). */
+/* Enqueue every pass of the plan on the state's stream (no host sync; the
+ * plan's first execution builds its tables and waits for them). */
 int ketgpu_plan_execute(const ketgpu_plan* p, ketgpu_state* s);
 /* Execute and time every pass with CUDA events on the state's stream;
  * pass_ms receives n_passes durations (milliseconds).  Synchronises. */
@@ -208,9 +209,9 @@ int ketgpu_run(int32_t n_qubits, const ketgpu_op* ops, uint64_t n_ops,
 int ketgpu_run_last_profile(double* out6);
 /* Free what the library keeps between calls on the device: the state of
  * ketgpu_run, destroyed states for reuse (at most 256 MB), the states of
- * ketgpu_adjoint (at most 4 GB) and scratch
- * memory (at most 64 MB a device) (no-op when
- * there is none).  No counterpart in ket, whose run holds no device memory. */
+ * ketgpu_adjoint (at most 4 GB) and scratch memory (at most 64 MB a device);
+ * a no-op when there is none.  The library does so itself before an allocation
+ * of its own fails.  No counterpart in ket, whose run holds no device memory. */
 int ketgpu_release_cache(void);
 
 /* ---- reductions (FP64 accumulation) --------------------------------- */
@@ -290,11 +291,14 @@ int ketgpu_adjoint(int32_t n_qubits, const ketgpu_op* ops, uint64_t n_ops,
                    const char* const* paulis, uint64_t n_terms,
                    int32_t precision, int32_t checkpoint_every, double* values,
                    double* grads);
-/* Sweep methods: AUTO = TILED when n_qubits >= the tile size (12 qubits
- * for KETGPU_C64, 11 for KETGPU_C128), else PER_GATE.  PER_GATE streams the
- * states through HBM once per gate; TILED runs each block of consecutive
- * gates that fits one tile in shared memory and registers, one HBM pass per
- * block.  Both give the same values and gradients up to rounding. */
+/* Sweep methods.  AUTO: up to 11 qubits one launch runs the whole circuit and
+ * its reverse sweep, a thread block a parameter set, with the states in shared
+ * memory; above that TILED (complex64 from 16 qubits: TILED_JIT).  PER_GATE
+ * streams the states through HBM once per gate; TILED runs each block of
+ * consecutive gates that fits one tile in shared memory and registers, one HBM
+ * pass per block, and needs n_qubits >= the tile size (12 qubits for
+ * KETGPU_C64, 11 for KETGPU_C128).  All give the same values and gradients up
+ * to rounding. */
 #define KETGPU_ADJOINT_AUTO 0
 #define KETGPU_ADJOINT_PER_GATE 1
 #define KETGPU_ADJOINT_TILED 2

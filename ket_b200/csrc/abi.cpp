@@ -594,7 +594,6 @@ void fetch_bytes(const void* src, uint64_t bytes, void* out, cudaStream_t stream
   copy_out(static_cast<const char*>(src), bytes, out, false, stream, nullptr);
 }
 
-// Create a state on the current device (used by adjoint.cu too).
 // The device state of the last ketgpu_run call, kept for the next call of
 // the same size and device.  Freeing a 30-qubit state (8 GiB) costs
 // 150-700 ms in cudaFree, more than downloading it.  Guarded by g_run_mu;
@@ -661,6 +660,7 @@ void release_idle_states() {
   for (State* s : all) free_state(s);
 }
 
+// Create a state on the current device.
 State* create_state(int n, int precision) {
   if (n < 0 || n > 40) fail(KETGPU_ERR_INVALID, "n_qubits must be in [0, 40]");
   if (precision != KETGPU_C64 && precision != KETGPU_C128)

@@ -465,8 +465,8 @@ __device__ __forceinline__ float nk_diag(NatState& a, NatState& l, const TGate& 
 // Pieces of a complex64 tiled sweep, used by the per-block kernels that are
 // generated with their phases and gates as compile-time constants.
 
-// Per-CTA set-up: tile offset tables and this set's packed coefficients (U forward, U^dag reverse), and `acc_words`
-// zeroed 4-byte words of gradient sums.
+// Per-CTA set-up: tile offset tables and this set's packed coefficients (U
+// forward, U^dag reverse), and `acc_words` zeroed 4-byte words of gradient sums.
 template <bool REV>
 __device__ __forceinline__ void c64_setup(const TileGeom& tg, const TGate* __restrict__ gates, int ngates,
                                           const float* __restrict__ mats, uint64_t mat_stride, int set,

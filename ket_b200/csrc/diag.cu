@@ -12,8 +12,8 @@
 //
 // The kernel splits x into L = min(n, 12) low bits and n - L high bits.  The
 // pair terms inside the low bits are one table of 2^L phases, formed in FP64
-// with the plan's other tables (tables.cu).  A CTA handles 2^L consecutive amplitudes, whose high bits h
-// are fixed.  For that chunk, the linear coefficients of the low bits
+// with the plan's other tables (tables.cu).  A CTA handles 2^L consecutive
+// amplitudes, whose high bits h are fixed.  For that chunk, the linear coefficients of the low bits
 // (a_i + sum_j b_ij h_j) and the constant phi(h) fold into two 64-entry tables,
 // built in FP64 with sincos.  Each amplitude then costs three complex products
 // and one read and one write.  All phases are formed in FP64 and rounded to

@@ -278,11 +278,6 @@ bool block_on_tensor_cores(int n, int k, const PlanOptions& opt) {
   return opt.precision == KETGPU_C64 && opt.tensor && tc_supported(k) && n >= k + 7;
 }
 
-// Greedy DAG-aware block growth over the gates `order` of `ops`.  With
-// diag_runs, whenever the next gate to place is diagonal, every diagonal gate
-// that can be moved to the front of what is left (no earlier non-diagonal
-// gate shares a qubit with it) is collected; if that run spans more qubits
-// than one block holds, it becomes a single Diagonal pass.
 // A partition in flat arrays: the planner grows many and keeps one.
 struct Partition {
   std::vector<int> gates;        // op indices, block after block
@@ -296,6 +291,11 @@ struct Partition {
   }
 };
 
+// Greedy DAG-aware block growth over the gates `order` of `ops`.  With
+// diag_runs, whenever the next gate to place is diagonal, every diagonal gate
+// that can be moved to the front of what is left (no earlier non-diagonal
+// gate shares a qubit with it) is collected; if that run spans more qubits
+// than one block holds, it becomes a single Diagonal pass.
 Partition grow_blocks(int n, const ketgpu_op* ops, const std::vector<int>& order, int max_k, bool diag_runs) {
   const size_t G = order.size();
   Partition part;
@@ -362,13 +362,6 @@ Partition grow_blocks(int n, const ketgpu_op* ops, const std::vector<int>& order
   return part;
 }
 
-// Topological orders of a segment's gates for the greedy block growth.  The
-// program order is one; a "band" order of width w sorts the gates by
-// ((ASAP depth + offset) / w, lowest qubit, depth), subject to every dependency, so
-// growth from the first gate follows a few neighbouring qubits through w
-// levels of the circuit before moving on: light-cone-shaped blocks.  On the
-// 30-qubit, 40-layer brick wall at k = 5 the best band order needs 119
-// passes against 154 in program order.  Returns op indices.
 struct Dependencies {  // of a segment's gates
   std::vector<int> depth, lowest, indegree;  // ASAP depth, lowest qubit, direct predecessors
   std::vector<int> succ_at, succ;            // successors of gate i: succ[succ_at[i] .. succ_at[i + 1])
@@ -407,6 +400,13 @@ Dependencies dependencies(const ketgpu_op* ops, const std::vector<int>& seg, int
   return d;
 }
 
+// Topological orders of a segment's gates for the greedy block growth.  The
+// program order is one; a "band" order of width w sorts the gates by
+// ((ASAP depth + offset) / w, lowest qubit, depth), subject to every dependency, so
+// growth from the first gate follows a few neighbouring qubits through w
+// levels of the circuit before moving on: light-cone-shaped blocks.  On the
+// 30-qubit, 40-layer brick wall at k = 5 the best band order needs 119
+// passes against 154 in program order.  Returns op indices.
 std::vector<int> band_order(const std::vector<int>& seg, const Dependencies& d, int w, int off) {
   const size_t G = seg.size();
   // (band, lowest qubit, depth, gate), smallest first

@@ -2192,7 +2192,13 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     }
     d_res = std::make_unique<DevBuf>(sizeof(ResGate) * std::max<size_t>(G, 1), dev, st);
     if (G) KB_CUDA(cudaMemcpyAsync(d_res->p, rg.data(), sizeof(ResGate) * G, cudaMemcpyHostToDevice, st));
-    KB_CUDA(cudaFuncSetAttribute(adjoint_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_smem));
+    // the most that any size takes: calls of other sizes may be between here
+    // and their launch on other threads
+    static OncePerDevice res_attr;  // one for each R
+    res_attr(dev, [] {
+      KB_CUDA(cudaFuncSetAttribute(adjoint_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)resident_smem(sizeof(T) << kResMaxQubits, kResThreads, sizeof(R))));
+    });
   }
 
   // tiled plan

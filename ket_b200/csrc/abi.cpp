@@ -405,9 +405,11 @@ struct Helpers {
   }
 };
 
-bool page_locked(const void* p) {
+// Memory that this process cannot or need not write itself: page-locked,
+// managed, a device's.
+bool known_to_cuda(const void* p) {
   cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
   cudaGetLastError();
   return false;
 }
@@ -420,7 +422,7 @@ bool page_locked(const void* p) {
 // 5.8 ms in turn, 16.3 ms when one of them copies directly.
 void copy_out(const char* src, uint64_t total, void* out, bool widen, cudaStream_t stream, DownloadTimes* times) {
   if (!total) return;
-  if (!widen && (total < kDirectBytes || page_locked(out))) {
+  if (!widen && (total < kDirectBytes || known_to_cuda(out))) {
     KB_CUDA(cudaMemcpyAsync(out, src, total, cudaMemcpyDeviceToHost, stream));
     KB_CUDA(cudaStreamSynchronize(stream));
     return;

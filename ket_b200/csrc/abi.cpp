@@ -671,7 +671,7 @@ State* create_state(int n, int precision) {
   KB_CUDA(cudaGetDevice(&device));
   if (State* idle = take_idle_state(n, precision, device)) {
     std::unique_ptr<State, void (*)(State*)> guard_idle(idle, destroy_state);
-    idle->exposed = false;
+    idle->exposed = idle->captured = false;
     set_ground(*idle);
     return guard_idle.release();
   }

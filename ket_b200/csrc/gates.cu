@@ -623,7 +623,7 @@ PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), a
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   KB_CUDA(cudaStreamIsCapturing(s.stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) {
-    s.exposed = true;  // the graph's replays write the amplitudes
+    s.exposed = s.captured = true;  // the graph's replays write the amplitudes
   } else if (plan.finite && s.version == s.active_version && s.active != all) {
     if (!s.exposed) {
       active_ = s.active;

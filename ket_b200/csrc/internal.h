@@ -125,6 +125,8 @@ struct State {
   // into a graph: they may change without a touch(), so what is known about
   // them is checked on the device before use.
   mutable bool exposed = false;
+  // A plan has been captured into a graph: the tree is built for each call.
+  mutable bool captured = false;
   uint64_t dim() const { return uint64_t{1} << n; }
   size_t amp_bytes() const { return precision == KETGPU_C64 ? 8 : 16; }
   void touch() const { ++version; }

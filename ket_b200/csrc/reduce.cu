@@ -600,7 +600,8 @@ Levels tree_levels(const State& st, uint64_t* total) {
   return lv;
 }
 
-// The state's tree, built on its stream if the amplitudes changed.
+// The state's tree, built on its stream if the amplitudes changed, or may have:
+// a graph's replays are not seen.
 Levels build_tree(const State& st) {
   uint64_t total = 0;
   const Levels lv = tree_levels(st, &total);
@@ -610,7 +611,7 @@ Levels build_tree(const State& st) {
     allocate("cudaMalloc(sampling tree)", [&] { return cudaMalloc(&st.tree, sizeof(double) * total); });
     st.tree_doubles = total;
   }
-  if (!total || st.tree_version == st.version) return lv;
+  if (!total || (st.tree_version == st.version && !st.captured)) return lv;
   double* buf = st.tree;
   g_tree_builds.fetch_add(1);
   for (int l = 1; l <= lv.L; ++l) {

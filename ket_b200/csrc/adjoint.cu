@@ -2113,6 +2113,7 @@ void run_adjoint(int n, const ketgpu_op* ops, uint64_t nops, const int32_t* pidx
     if (pi >= 0 && g.gen == 0) fail(KETGPU_ERR_INVALID, "adjoint: parameterised op must be Rx/Ry/Rz/CRx/CRy/CRz/CP");
     if (pi >= (int32_t)nparams) fail(KETGPU_ERR_OUT_OF_RANGE, "adjoint: parameter index out of range");
   }
+  if (!batch) return;  // no sets: the arguments have been checked
 
   // the gates as gate_matrices takes them: 2x2 U, row-major, FP64
   // interleaved; the tiled sweep stores a phase gate as diag(1, phase)

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <random>
 #include <type_traits>
 #include <cstring>
@@ -600,11 +601,16 @@ Levels tree_levels(const State& st, uint64_t* total) {
   return lv;
 }
 
+// What draws make on demand in a state, its tree and its second stream, is made
+// by one thread: several may draw from a state at once.
+std::mutex g_draw_mu;
+
 // The state's tree, built on its stream if the amplitudes changed, or may have:
 // a graph's replays are not seen.
 Levels build_tree(const State& st) {
   uint64_t total = 0;
   const Levels lv = tree_levels(st, &total);
+  std::lock_guard<std::mutex> lk(g_draw_mu);
   // The tree lives with the state (1/31 of a complex128 state's size, 1/15
   // of a complex64 one) and is rebuilt only after the amplitudes changed.
   if (total && !st.tree) {
@@ -657,6 +663,16 @@ void draw(const State& st, const Levels& lv, const U* d_u, uint64_t count, uint6
   fetch_bytes(d_out, sizeof(uint64_t) * count, out, st.stream);
 }
 
+cudaStream_t side_stream(const State& st) {
+  std::lock_guard<std::mutex> lk(g_draw_mu);
+  if (!st.side) {
+    int least = 0, greatest = 0;
+    KB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    KB_CUDA(cudaStreamCreateWithPriority(&st.side, cudaStreamNonBlocking, greatest));
+  }
+  return st.side;
+}
+
 // Draws from which the uniforms are made on the device.  A call of 8192 draws
 // at 12 qubits takes 79 us with them made on the device and 120 on the host;
 // one of 1000 takes 61 us on the host.
@@ -686,24 +702,20 @@ void sample_tree_seeded(const State& st, uint32_t seed, uint64_t count, uint64_t
     sample_tree(st, u.data(), count, out);
     return;
   }
-  if (!st.side) {
-    int least = 0, greatest = 0;
-    KB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    KB_CUDA(cudaStreamCreateWithPriority(&st.side, cudaStreamNonBlocking, greatest));
-  }
   // the words on the second stream, beside whatever the first one still does
   // to the amplitudes and the tree's building
-  StreamScratch words(sizeof(uint2) * count, st.device, st.side);
+  const cudaStream_t side = side_stream(st);
+  StreamScratch words(sizeof(uint2) * count, st.device, side);
   MtState mt;
   mt.x[0] = seed;
   for (uint32_t i = 1; i < 624; ++i) mt.x[i] = 1812433253u * (mt.x[i - 1] ^ (mt.x[i - 1] >> 30)) + i;
-  mt19937_words<<<1, kMtThreads, 0, st.side>>>(mt, (uint32_t)(2 * count), static_cast<uint32_t*>(words.p));
+  mt19937_words<<<1, kMtThreads, 0, side>>>(mt, (uint32_t)(2 * count), static_cast<uint32_t*>(words.p));
   count_launch();
   KB_CUDA(cudaGetLastError());
   const Levels lv = build_tree(st);
   cudaEvent_t made;
   KB_CUDA(cudaEventCreateWithFlags(&made, cudaEventDisableTiming));
-  cudaError_t e = cudaEventRecord(made, st.side);
+  cudaError_t e = cudaEventRecord(made, side);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(st.stream, made, 0);
   cudaEventDestroy(made);
   check_cuda(e, "sample_tree_seeded");

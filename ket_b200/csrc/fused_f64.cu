@@ -66,10 +66,15 @@ struct F64Geom {
   int tpos[6];          // the block's qubits, ascending
   int is_target[kMaxTileBits];
   int tile_pos[kMaxTileBits];
-  // positions that are zero in a tile base, ascending: the tile's qubits and
-  // the inactive ones; [1]: where nothing is known, the tile's alone
-  int nins[2];
-  unsigned char ins[2][40];
+  // A tile's base is its index spread over the active qubits outside the tile:
+  // run by run of adjacent ones, the index shifted and masked ([1]: where
+  // nothing is known, over all qubits outside the tile).  One thread of a team
+  // forms it while the others wait (inserting a zero bit at a time, positions
+  // picked by what is known: 27 qubits, depth 20, 38.1 ms a circuit, now 37.0;
+  // 20 qubits 501 us, now 475).  At most 20 runs in 40 qubits.
+  int nruns[2];
+  unsigned char shift[2][20];
+  uint64_t run[2][20];
   Extent tiles;
 };
 
@@ -166,11 +171,9 @@ __global__ void __launch_bounds__(F64Cfg<KQ>::THREADS, 1)
   const int whole = g.tiles.unknown && *g.tiles.unknown;
   const uint64_t n_tiles = whole ? g.tiles.all : g.tiles.known;
   auto tile_base = [&](uint64_t t) -> uint64_t {
-    for (int j = 0; j < g.nins[whole]; ++j) {
-      const int f = g.ins[whole][j];
-      t = ((t >> f) << (f + 1)) | (t & ((uint64_t{1} << f) - 1));
-    }
-    return t;
+    uint64_t b = 0;
+    for (int j = 0; j < g.nruns[whole]; ++j) b |= (t << g.shift[whole][j]) & g.run[whole][j];
+    return b;
   };
   const int mine = tid < tile ? per : 0;
   auto stage_at = [&](int stage) { return f64_tile + ((size_t)(team * kStages + stage) << g.tb); };
@@ -311,8 +314,14 @@ void launch_fused_f64(const State& st, const Pass& p, const void* mat_t, const R
       if (!g.is_target[j]) g.gpos[gb++] = q;
       ++j;
     }
-    if (((tile_mask | ~span) >> q) & 1) g.ins[0][g.nins[0]++] = (unsigned char)q;
-    if ((tile_mask >> q) & 1) g.ins[1][g.nins[1]++] = (unsigned char)q;
+    for (int w = 0; w < 2; ++w) {
+      const uint64_t zero = w ? tile_mask : tile_mask | ~span;
+      if ((zero >> q) & 1) continue;
+      const int below = q - __builtin_popcountll(~zero & ((uint64_t{1} << q) - 1));
+      int& r = g.nruns[w];
+      if (!r || g.shift[w][r - 1] != below) g.shift[w][r++] = (unsigned char)below;
+      g.run[w][r - 1] |= uint64_t{1} << q;
+    }
   }
   g.q0_group = g.gpos[0] == 0;
   g.tiles = {uint64_t{1} << (__builtin_popcountll(span) - g.tb), st.dim() >> g.tb, reach.unknown};

@@ -44,10 +44,10 @@ METRIC = "time per 30q circuit"
 
 # DRAM bytes (read + write) of one fused_tc_kernel<k> launch on a 2^26
 # complex64 state, from ncu (dram__bytes_read.sum + dram__bytes_write.sum,
-# one dense block of the 26-qubit workload `--workload kernels26`; see
+# one dense block that stores directly; see
 # profiles/fused_tc_kernel6_26q.md).  A launch streams the state once, so the
 # figure scales with 2^n.
-TC_TRAFFIC_BYTES_26Q = {5: 536.966400e6 + 477.739776e6, 6: 537.047552e6 + 477.192448e6}
+TC_TRAFFIC_BYTES_26Q = {5: 536.966400e6 + 477.739776e6, 6: 537.020672e6 + 478.800896e6}
 
 
 def peaks():

@@ -261,7 +261,8 @@ int ketgpu_uniforms_mt19937(uint32_t seed, uint64_t count, double* out);
  * each draw the first index whose running sum exceeds u.  The tree is kept
  * with the state and rebuilt only after the amplitudes changed (any
  * execute, apply, reset, upload, copy into the state, or
- * ketgpu_state_device_ptr), so repeated draws from one state -- ket's
+ * ketgpu_state_device_ptr; once a plan has been captured into a graph on the
+ * state, for every call), so repeated draws from one state -- ket's
  * StateVectorSimulation::sample, statevector.cpp:33-42, called once per
  * shot -- cost one descent each. */
 int ketgpu_sample(const ketgpu_state* s, const double* uniforms, uint64_t count,

@@ -712,6 +712,7 @@ void free_state(State* s) {
     cudaStreamDestroy(s->side);
   }
   if (s->tree) cudaFree(s->tree);
+  s->word = DeviceBlock();
   if (s->amps) cudaFree(s->amps);
   if (s->stream) cudaStreamDestroy(s->stream);
   if (prev >= 0) cudaSetDevice(prev);

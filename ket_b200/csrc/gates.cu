@@ -629,8 +629,7 @@ PassRunner::PassRunner(const State& s, const Plan& plan) : s_(s), plan_(plan), a
       active_ = s.active;
       keep_ = true;
     } else if (s.dim() * s.amp_bytes() >= kGroundCheckBytes && s.version == s.ground_version) {
-      word_ = std::make_unique<StreamScratch>(sizeof(unsigned), s.device, s.stream);
-      find_not_ground(s, static_cast<unsigned*>(word_->p));
+      word_ = find_not_ground(s);
       active_ = 0;
     }
   }
@@ -645,7 +644,7 @@ PassRunner::~PassRunner() {
 }
 
 Extent PassRunner::amplitudes() const {
-  return {uint64_t{1} << active_bits(active_), s_.dim(), word_ ? static_cast<const unsigned*>(word_->p) : nullptr};
+  return {uint64_t{1} << active_bits(active_), s_.dim(), word_};
 }
 
 void PassRunner::launch(const Pass& p) {

@@ -504,7 +504,9 @@ __global__ void not_ground(const uint64_t* __restrict__ w, uint64_t words, uint6
 }
 }  // namespace
 
-void find_not_ground(const State& st, unsigned* d) {
+const unsigned* find_not_ground(const State& st) {
+  if (!st.word.p) st.word = DeviceBlock(sizeof(unsigned), st.device, st.stream);
+  unsigned* d = static_cast<unsigned*>(st.word.p);
   KB_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned), st.stream));
   const bool c64 = st.precision == KETGPU_C64;
   const uint64_t words = st.dim() * (c64 ? 1 : 2);
@@ -512,6 +514,7 @@ void find_not_ground(const State& st, unsigned* d) {
       static_cast<const uint64_t*>(st.amps), words, c64 ? 0x3f800000ull : 0x3ff0000000000000ull, d);
   count_launch();
   KB_CUDA(cudaGetLastError());
+  return d;
 }
 
 double reduce_norm(const State& st) {

@@ -253,8 +253,10 @@ __global__ void __launch_bounds__(kThreads)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int dim = 1 << g.k;
   const int tile = 1 << g.tb;
-  const uint64_t n_tiles = g.tiles.count();
-  if (blockIdx.x >= n_tiles) return;
+  // in shared memory: with it in registers, or an early return, the products'
+  // loop is compiled for fewer in flight (k = 6, one tile: 25.6 us, now 21.5)
+  __shared__ uint64_t n_tiles;
+  if (threadIdx.x == 0) n_tiles = g.tiles.count();
   T* mt = reinterpret_cast<T*>(smem_raw);  // [c][r] : dim*dim
   T* buf = mt + dim * dim;                 // [group][comb] : tile
   __shared__ uint64_t off_lo[64], off_hi[64];
@@ -650,7 +652,7 @@ Extent PassRunner::amplitudes() const {
 void PassRunner::launch(const Pass& p) {
   const State& s = s_;
   const Plan& plan = plan_;
-  const bool ground = !s.exposed && s.version == s.ground_version;
+  const bool reset = s.version == s.ground_version, ground = reset && !s.exposed;
   s.touch();
   // a phase on zeros, an exchange of zeros
   const bool zeros = (p.kind == PassKind::Phase && (p.p0 & ~active_)) ||
@@ -669,7 +671,10 @@ void PassRunner::launch(const Pass& p) {
       count_launch();
       KB_CUDA(cudaGetLastError());
     } else {
-      norm_to_device(s, amplitudes(), plan.d_norm + 2, plan.d_norm);
+      // most likely |0...0> all the same: of up to 128 KB by one CTA, without a
+      // second launch
+      const int blocks = reset && s.dim() <= (uint64_t{1} << 14) ? 1 : kNormBlocks;
+      norm_to_device(s, amplitudes(), plan.d_norm + 2, plan.d_norm, blocks);
     }
     return;
   }

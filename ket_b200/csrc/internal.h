@@ -338,8 +338,8 @@ bool tc_supported(int k);
 
 void set_ground(const State& s);
 // Squared norm of the first amplitudes into a device scalar (partials:
-// kNormBlocks doubles).
-void norm_to_device(const State& s, const Extent& dim, double* partials, double* out);
+// kNormBlocks doubles), by `blocks` CTAs.
+void norm_to_device(const State& s, const Extent& dim, double* partials, double* out, int blocks = kNormBlocks);
 // The same from partials a tensor-core block already wrote (in index order).
 void norm_from_partials(const State& s, const double* partials, double* out);
 // Look up (and so load) the no-allocation entry point's scratch array and

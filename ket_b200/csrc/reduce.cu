@@ -460,15 +460,17 @@ __global__ void rescale_kernel(T* __restrict__ s, Extent extent, const double* _
 
 }  // namespace
 
-void norm_to_device(const State& st, const Extent& dim, double* partials, double* out) {
+void norm_to_device(const State& st, const Extent& dim, double* partials, double* out, int blocks) {
+  double* part = blocks == 1 ? out : partials;
   if (st.precision == KETGPU_C64)
-    norm_partial<float2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), dim,
-                                                                   partials);
+    norm_partial<float2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const float2*>(st.amps), dim, part);
   else
-    norm_partial<double2><<<kNormBlocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), dim,
-                                                                    partials);
-  finish_partials<<<1, kRThreads, 0, st.stream>>>(partials, kNormBlocks, 1, out);
-  count_launch(2);
+    norm_partial<double2><<<blocks, kRThreads, 0, st.stream>>>(static_cast<const double2*>(st.amps), dim, part);
+  count_launch();
+  if (blocks > 1) {
+    finish_partials<<<1, kRThreads, 0, st.stream>>>(partials, blocks, 1, out);
+    count_launch();
+  }
   KB_CUDA(cudaGetLastError());
 }
 
